@@ -1,49 +1,62 @@
 // Window search, primary-surface selection, K-sample emission and per-sample
-// point selection, fused into one kernel.
+// point selection.
 //
 // Replaces _C.quick_sampling (epcq/csrc/epcq_render_topk.cu:341-417), which
 // zero-fills all four outputs, runs quick_sampling_kernel (:82-220, one warp
 // per ray, one lane per window cell, a 128-bin shared-memory histogram built
 // with float atomics and a serial walk on lane 0) and then
 // quick_search_nearby_pc (:10-81, one thread per (ray, sample slot) re-walking
-// the window).  Here a CTA owns an 8x32 pixel tile: it stages the points of
-// the tile's window halo (clamped to the image) into shared memory once as
-// float4 (x, y, z, id) with coalesced gathers, then one thread owns one ray
-// end to end and writes every output element of that ray exactly once:
+// the window).  Here a launch is two kernels:
 //
-//   pass A  kept candidates (ray distance < radius, at most 48 per window cell,
-//           cells row-major and clamped, bucket order) -> tmin, tmax
-//   pass B  the same candidates binned by int((t - tmin) / t_intvl); instead of
-//           a 128-bin histogram the thread keeps the 4 smallest distinct bins
-//           (count, distance sum) in registers -- exactly the bins the walk
-//           reaches first -- and re-collects further bins only if the walk
-//           goes past them
+//   k_ray_list        one block per 256-pixel tile: each ray's window candidate
+//                count from the hash table; rays without any get their default
+//                outputs (coalesced runs), the others go into a list with
+//                their directions, a tile's rays ordered by count
+//   k_quick_sampling  persistent warps take rays from the list.  A ray with few
+//                candidates is served by 8 lanes (four rays a warp), a heavy
+//                one by the whole warp; lanes stand for candidates:
+//
+//   pass A  every candidate of the window (rows of cells are runs of the
+//           sorted ids) is tested against the ray once; those within the
+//           radius -- at most 48 per window cell -- are "kept" and give tmin.
+//           The kept ones, and the few just outside the radius or beyond a
+//           cell's 48, are listed (indices, in window order) in shared memory:
+//           no later pass looks at any other candidate
+//   bins    int((t - tmin) / t_intvl) of the kept entries: a histogram in
+//           shared memory of counts and quantised distance sums
 //   walk    bins with >= 2 points in ascending order: alpha = gamma *
 //           exp(-mean_dist / alpha_g), emit when alpha * T > 1e-3, T -= alpha,
 //           stop when T < 1e-3 or S samples are out
-//   ball    per emitted sample, the reference's 8-entry id buffer over the
-//           whole window (including its quirk that, while the buffer fills, the
-//           tracked "farthest" entry is the nearest one), all samples of a ray
-//           in one walk.  Candidates whose position along the ray is further
-//           than radius (+ a rounding margin orders of magnitude above float
-//           error) from a sample are skipped for it before the distance is
-//           computed: they cannot be within the radius, so each buffer sees
-//           exactly the same sequence.
+//   ball    per sample, the reference's 8-entry id buffer over the listed
+//           candidates, with its quirk that, while the buffer fills, the
+//           tracked "farthest" entry is the nearest one.  The hits go to shared
+//           memory in order; 8 lanes hold the buffer in ascending distance, so
+//           a replacement is one ballot and one shift
 //
-// Each pass walks the ray's window as one flat candidate sequence, and the
-// tile's rays are ranked by window size before they are handed to threads, so
-// the lanes of a warp run loops of similar length instead of diverging on
-// every cell's bucket size.  The radius test decides on the squared distance
-// when it is clear of the threshold and calls norm3df only near it (see
-// RadiusTest); the mean distance of a bin is computed only for bins the walk
-// can reach.  Tiles
-// whose halo holds more points than the stage read candidates straight from
-// global memory through the same code.
+// The candidates the ball query can take are within the radius of a point of
+// the ray, so they are within the radius of the ray up to float error, and the
+// list's margin (see near_limit) is orders of magnitude above that: each
+// buffer sees exactly the sequence of the full window walk.
+//
+// What bounds it is instruction issue, then the latency of the candidates'
+// first touch.  One thread per ray (tiles staged in shared memory, 32 rays of a
+// window-size class a warp) left half the lanes idle -- every window row and
+// buffer replacement waited for the longest lane -- and its blocks idle at
+// each tile's end; with lanes as candidates 27 of 32 lanes are active and there
+// is no barrier.  1M points, 800 x 800, radius 0.008: 1000 us -> 471 us (446 M
+// -> 366 M warp instructions, 54% -> 74% of the issue slots); 4M points at
+// 512 x 512: 4470 -> 1280 us; 100k points, 3 x 3 window: 193 -> 55 us.  Measured
+// and not kept: the listed candidates themselves in shared memory (20 bytes an
+// entry leave too little L1: 780-1010 us on the first view), re-walking the
+// window in every pass instead of a list (760-850 us), copies of the code per
+// lane count (instruction-cache misses: 560-620 us), two samples a ball pass
+// (registers: 662-730 us).
 //
 // Bin sums are accumulated in window-cell then bucket order; the reference
 // adds them with shared-memory atomics in an unspecified order, so a bin's
 // mean distance can differ from the reference's in the last bit -- which moves
 // an output only if alpha * T or T sits within that bit of 1e-3.
+#include <cmath>
 #include <cstdio>
 #include <mutex>
 
@@ -51,17 +64,38 @@
 
 namespace hp {
 
-#ifndef HP_BIN_LIST
-#define HP_BIN_LIST 6
-#endif
-constexpr int kBinList = HP_BIN_LIST;  // distinct t-bins collected per candidate pass
-constexpr int kTeReg = 4;        // emitted sample depths kept in registers
+constexpr int kTeReg = 4;        // emitted sample depths kept in registers (sample_ray_warp)
 constexpr int kBallPass = 2;     // samples served by one ball-query walk
 constexpr int kHeavyWindow = 320;  // default: rays with more window candidates get a whole warp
 constexpr int kMaxHeavyWindow = 4096;  // largest tunable threshold
-constexpr int kMaskWords = (kHeavyWindow + 31) / 32;  // kept-candidate mask of a thread-served ray (larger windows run unmasked)
-constexpr int kClasses = 64;     // window-size classes used to group a tile's rays
-constexpr int kWalkBatch = 4;    // bins whose sums one walk pass of a warp-served ray gathers
+constexpr int kWalkBatch = 4;    // bins whose sums one walk pass of sample_ray_warp gathers
+constexpr int kClasses = 64;     // window-size classes a tile's rays are ordered by
+constexpr int kThreads = 256;    // pixels of a tile, threads per block of the list kernels
+constexpr int kWarps = kThreads / 32;
+constexpr int kServeThreads = 128;  // threads per block of the serving kernels
+constexpr int kServeWarps = kServeThreads / 32;
+constexpr int64_t kMaxTilesPerView = 1 << 21;
+constexpr int kHistWords = 512;  // per warp: the rays' bin histograms, then their ball hits
+
+// The reference keeps a candidate when norm3df(e) < radius (e = point minus its
+// projection on the ray).  The squared length e2 (three roundings) decides it
+// without the square root whenever e2 is outside a band of relative width
+// 2^-16 around radius^2 -- far wider than the few-ulp errors of e2 and
+// norm3df -- and norm3df decides inside the band, so the result is identical.
+struct RadiusTest {
+  float r, lo2, hi2;
+  bool fast;  // else the band is everything
+};
+
+// t-bin index int((t - tmin) / t_intvl) of a kept candidate (x = t - tmin >= 0).
+// y = x * RN(1 / t_intvl) is within 3.1 * 2^-24 * q of the quotient q and of
+// its rounding RN(q), so when y widened by 2^-21 relative on both sides
+// truncates to one integer, that integer is int(RN(q)); otherwise (a bin
+// edge within a few ulps) the division is done exactly.
+struct BinDiv {
+  float intvl, inv;
+  bool fast;
+};
 
 struct SampleArgs {
   const float* __restrict__ xyz;
@@ -76,68 +110,52 @@ struct SampleArgs {
   int* __restrict__ pc_idx;
   float* __restrict__ sp_t;
   uint8_t* __restrict__ mask;
-  int heavy;  // rays with more window candidates than this are served by a whole warp
+  // derived from the options once per launch (derive_args)
+  RadiusTest rt;
+  BinDiv bins;
+  float near0;   // near_limit's constant part
+  float quanta;  // 1 / radius
+  float eps;     // relative error of alpha from a mean distance off by one part of the radius (serve_rays)
 };
 
-// Stage configurations: kCap staged points per tile, kBlocks resident blocks
-// per SM, and the tile: kTileH rows x kTileW pixels, one thread per pixel
-// (kThreads = 256 or 128 threads per block).  Shared memory per SM bounds
-// stage and blocks together, and registers per thread follow from the
-// resident threads: 64 at 4 x 256 or 8 x 128, 80 at 3 x 256 or 6 x 128, 128 at
-// 2 x 256.  A larger stage splits fewer dense tiles into row bands (less
-// re-staging of shared halo rows) but keeps fewer warps resident; a square
-// tile stages a smaller window halo per ray (20 x 20 cells for 256 rays
-// against 12 x 36 at k = 5).  Which wins depends on how the cloud's points
-// spread over the image, so the launch picks one (hp_tuning.stage_config) and
-// hashpoint.batch.Autotuner searches them.  (128-thread blocks on 8 x 16 tiles
-// -- 4 warps waiting at a tile's end instead of 8, for a 12 x 20 halo per 128
-// rays -- measured 3-5% slower on the shapes views and 12-17% on the clustered
-// ones, with 1216 points x 8 blocks and 1856 x 6, so none is offered.)
-template <int kCap_, int kBlocks_, int kTileH_, int kTileW_>
+// The rays to serve, each as (ray, direction bits): those of 8 lanes in units
+// of four from the front (a tile's last unit is filled up with ray -1), those
+// of a whole warp from the back.
+struct RayList {
+  int4* rays;
+  long long cap;
+  unsigned* counts;  // [4]: front entries, back entries, next front unit, next back entry to serve
+  int* front_view;   // batched launches: view of each front unit
+  int* back_view;    // and of each back entry
+  int light;         // rays with more window candidates than this are served by a whole warp
+};
+
+// Stage configurations: a block's warps hold kStage listed candidates on chip
+// (a quarter of a warp's per ray served by 8 lanes) at kBlocks blocks of
+// kServeThreads per SM, and the ray list is built over kTileH x kTileW pixel
+// tiles.  Registers per thread follow from the resident threads (64, 80, 96):
+// fewer warps spill less but hide less of the candidates' latency.  960 entries
+// a warp: with 640, 4M-point views at 512 x 512 lose 22% to rays whose list
+// overflows; shapes and sphere views are level, the 3M-point clustered view
+// gains 5% (less shared memory leaves more L1).
+template <int kStage_, int kBlocks_, int kTileH_, int kTileW_>
 struct StageCfg {
-  static constexpr int kCap = kCap_;
+  static constexpr int kStage = kStage_;
   static constexpr int kBlocks = kBlocks_;
   static constexpr int kTileH = kTileH_;
   static constexpr int kTileW = kTileW_;
-  static constexpr int kThreads = kTileH * kTileW;
-  static constexpr int kHaloMax = (kTileH + kMaxKernel - 1) * (kTileW + kMaxKernel - 1);
-  static constexpr int kItemsPerTile = kTileH * 4;  // rows, each in up to four column quarters
-  static_assert((kThreads == 256 || kThreads == 128) && kTileW >= 4 && kTileW <= 32 && kTileH <= 16, "tile shape");
+  static constexpr int kEntries = kStage / kServeWarps;  // per warp
+  static constexpr int kWarpBytes = kEntries * 4 + kHistWords * 4;
+  static constexpr int kSmem = kServeWarps * kWarpBytes;
+  static_assert(kTileH * kTileW == kThreads && kEntries % 32 == 0 && kEntries <= 1024 && kBlocks * (kSmem + 1024) <= 227 * 1024, "stage");
 };
-using Cfg2560x4 = StageCfg<2560, 4, 8, 32>;     // 40 KB stage, 4 blocks per SM, 8 x 32 tiles
-using Cfg3712x3 = StageCfg<3712, 3, 8, 32>;     // 58 KB stage, 3 blocks per SM
-using Cfg5888x2 = StageCfg<5888, 2, 8, 32>;     // 92 KB stage, 2 blocks per SM
-using Cfg2560x4Sq = StageCfg<2560, 4, 16, 16>;  // 16 x 16 tiles
-using Cfg3712x3Sq = StageCfg<3712, 3, 16, 16>;
-constexpr int kStageConfigs = 5;      // hp_tuning.stage_config 1..5 (0 = the default)
-// The default: 16 x 16 tiles with 2560 staged points x 4 blocks, measured
-// fastest or level on the shapes, clustered and multi-view workloads (the
-// small sphere view prefers 5888 x 2, which a tuner finds).
+using Cfg1 = StageCfg<3840, 8, 8, 32>;
+using Cfg2 = StageCfg<3968, 6, 8, 32>;
+using Cfg3 = StageCfg<4096, 5, 8, 32>;
+using Cfg4 = StageCfg<3840, 8, 16, 16>;
+using Cfg5 = StageCfg<3968, 6, 16, 16>;
+constexpr int kStageConfigs = 5;  // hp_tuning.stage_config 1..5 (0 = the default)
 constexpr int kDefaultStageConfig = 4;
-constexpr int kMaxItemsPerTile = 64;  // over the configurations (16 rows, four column ranges each)
-constexpr int kCellsPerThread = 2;    // halo cells per thread (<= 432 = the largest halo)
-
-template <class Cfg>
-struct Stage {
-  float4 cand[Cfg::kCap];   // x, y, z, id (as int bits; -1 = invalid id)
-  int cls[kClasses];        // rays per window-size class
-  int cls_base[kClasses];   // first rank of each class
-  int order[Cfg::kThreads];  // pixel of each rank, heaviest class first
-  int off[Cfg::kHaloMax + 1];  // staged offset of each halo cell, exclusive prefix
-  int start[Cfg::kHaloMax];    // the cell's first index in sorted_point_idx
-  int warp_tot[Cfg::kThreads / 32];
-  int next_unit;            // next work unit of the tile (see process_tile)
-  unsigned kept[kMaskWords][Cfg::kThreads];  // per thread: window positions pass A accepted
-};
-// kBlocks CTAs per SM (228 KB of shared memory, 1 KB reserved per CTA)
-template <class Cfg>
-constexpr bool fits_sm() {
-  return Cfg::kBlocks * (sizeof(Stage<Cfg>) + 16 + 1024) <= 228 * 1024 && Cfg::kItemsPerTile <= kMaxItemsPerTile &&
-         Cfg::kHaloMax <= kCellsPerThread * Cfg::kThreads;
-}
-static_assert(fits_sm<Cfg2560x4>() && fits_sm<Cfg3712x3>() && fits_sm<Cfg5888x2>() && fits_sm<Cfg2560x4Sq>() &&
-                  fits_sm<Cfg3712x3Sq>(),
-              "a stage configuration exceeds the shared memory of its blocks per SM");
 
 // Clipped bucket range of a hash entry: [x, x + count) within [0, n_sorted).
 __device__ __forceinline__ int2 bucket_range(int2 h, int n_sorted) {
@@ -145,31 +163,9 @@ __device__ __forceinline__ int2 bucket_range(int2 h, int n_sorted) {
   return make_int2(h.x, h.x + min(h.y, n_sorted - h.x));
 }
 
-// Candidates from the tile's shared-memory stage.
-template <class Cfg>
-struct SrcStaged {
-  static constexpr bool kStaged = true;
-  static constexpr int kKeptStride = Cfg::kThreads;  // the kept masks' word stride (one column per thread)
-  const Stage<Cfg>* st;
-  int rv0, ru0, nu;
-  __device__ __forceinline__ int cell(int vv, int uu) const { return (vv - rv0) * nu + (uu - ru0); }
-  __device__ __forceinline__ int2 range(const SampleArgs&, int vv, int uu) const {
-    const int c = cell(vv, uu);
-    return make_int2(st->off[c], st->off[c + 1]);
-  }
-  __device__ __forceinline__ float4 fetch(const SampleArgs&, int i) const { return st->cand[i]; }
-};
-
-// Candidates straight from global memory (tiles whose halo overflows the stage).
-struct SrcGlobal {
-  static constexpr bool kStaged = false;
-  static constexpr int kKeptStride = 1;  // no kept masks
-  __device__ __forceinline__ int cell(int, int) const { return 0; }
-  __device__ __forceinline__ int2 range(const SampleArgs& a, int vv, int uu) const {
-    return bucket_range(__ldg(a.hash + (size_t)vv * a.cam.width + uu), a.n_sorted);
-  }
-  __device__ __forceinline__ float4 fetch(const SampleArgs& a, int j) const { return __ldg(a.pts + j); }
-};
+__device__ __forceinline__ int2 cell_range(const SampleArgs& a, int vv, int uu) {
+  return bucket_range(__ldg(a.hash + (size_t)vv * a.cam.width + uu), a.n_sorted);
+}
 
 // Pack the candidates once per launch: pts[j] = (xyz of sorted_point_idx[j],
 // its id), or id -1 when the id is outside [0, n_points).  Every later fetch
@@ -201,177 +197,46 @@ __device__ __forceinline__ void pack_range(const int* __restrict__ sidx, int j0,
   }
 }
 
-// Visit a ray's window candidates in the reference's order -- window rows
-// top to bottom, cells left to right (coordinates clamped into the image, so
-// border windows repeat cells), entries in bucket order -- calling
-// body(point) for each; body returns true when it accepts the candidate, and
-// a cell is left once `cap` of its candidates were accepted.
-//
-// Staged tiles: a window row whose columns need no clamping is a run of
-// consecutive halo cells, i.e. one contiguous range of the stage, so the loop
-// only watches for cell boundaries (for the cap).  Other rows, and tiles read
-// from global memory, go cell by cell.  No integer division per cell.
-template <class Src, class Body>
-__device__ __forceinline__ void walk_window(const SampleArgs& a, const Src& src, int v, int u, int cap, Body&& body) {
-  const int H = a.cam.height, W = a.cam.width, k = a.opt.k;
-  const int koff = (k + 1) >> 1, lo = koff - 1, hi = k - koff;
-  const bool cols_clamped = (u - lo < 0) || (u + hi > W - 1);
-  for (int dv = -lo; dv <= hi; dv++) {
-    const int vv = min(max(v + dv, 0), H - 1);
-    bool done_row = false;
-    if constexpr (Src::kStaged) {
-      if (!cols_clamped) {
-        const int c0 = src.cell(vv, u - lo);
-        const int* off = src.st->off;
-        int j = off[c0];
-        const int jend = off[c0 + k];
-        int c = c0, cell_end = off[c0 + 1], nk = 0;
-        while (j < jend) {
-          while (j >= cell_end) {  // entered the next non-empty cell
-            c++;
-            cell_end = off[c + 1];
-            nk = 0;
-          }
-          if (nk >= cap) {
-            j = cell_end;
-            continue;
-          }
-          if (body(src.fetch(a, j))) nk++;
-          j++;
-        }
-        done_row = true;
-      }
-    }
-    if (!done_row) {
-      for (int du = -lo; du <= hi; du++) {
-        const int uu = min(max(u + du, 0), W - 1);
-        const int2 rg = src.range(a, vv, uu);
-        int nk = 0;
-        for (int j = rg.x; j < rg.y && nk < cap; j++)
-          if (body(src.fetch(a, j))) nk++;
-      }
-    }
-  }
-}
-
-// Staged tiles, unclamped window columns: the same visit as walk_window's
-// fast path, also passing each candidate's position f in the window's
-// candidate sequence (window rows concatenated, entries in stage order).
-template <class Src, class Body>
-__device__ __forceinline__ void walk_rows(const SampleArgs& a, const Src& src, int v, int u, int cap, Body&& body) {
-  const int H = a.cam.height, k = a.opt.k;
-  const int lo = ((k + 1) >> 1) - 1;
-  const int* off = src.st->off;
-  int f0 = 0;
-  for (int r = 0; r < k; r++) {
-    const int c0 = src.cell(min(max(v - lo + r, 0), H - 1), u - lo);
-    const int jb = off[c0], jend = off[c0 + k];
-    int j = jb, c = c0, cell_end = off[c0 + 1], nk = 0;
-    while (j < jend) {
-      while (j >= cell_end) {
-        c++;
-        cell_end = off[c + 1];
-        nk = 0;
-      }
-      if (nk >= cap) {
-        j = cell_end;
-        continue;
-      }
-      if (body(src.fetch(a, j), f0 + (j - jb))) nk++;
-      j++;
-    }
-    f0 += jend - jb;
-  }
-}
-
-// Visit the candidates whose window positions are set in a kept mask (nw
-// words, stride Src::kKeptStride), in order; the position is mapped back to the stage
-// row by row.
-template <class Src, class Body>
-__device__ __forceinline__ void walk_kept(const SampleArgs& a, const Src& src, int v, int u, const unsigned* mask,
-                                          int nw, Body&& body) {
-  const int H = a.cam.height, k = a.opt.k;
-  const int lo = ((k + 1) >> 1) - 1;
-  const int* off = src.st->off;
-  int r = -1, rf0 = 0, rf1 = 0, jb = 0;
-  for (int w = 0; w < nw; w++) {
-    unsigned m = mask[w * Src::kKeptStride];
-    while (m) {
-      const int f = (w << 5) + __ffs(m) - 1;
-      m &= m - 1;
-      while (f >= rf1) {
-        r++;
-        const int c0 = src.cell(min(max(v - lo + r, 0), H - 1), u - lo);
-        jb = off[c0];
-        rf0 = rf1;
-        rf1 += off[c0 + k] - jb;
-      }
-      body(src.fetch(a, jb + (f - rf0)));
-    }
-  }
-}
-
-// Fill n elements from p with v using 16-byte stores where aligned.
-template <typename T>
-__device__ __forceinline__ void fill_run(T* p, int n, T v) {
-  constexpr int kVec = 16 / sizeof(T);
-  int i = 0;
-  while (i < n && (((uintptr_t)(p + i)) & 15) != 0) p[i++] = v;
-  if (i + kVec <= n) {
-    T vv[kVec];
-#pragma unroll
-    for (int q = 0; q < kVec; q++) vv[q] = v;
-    const int4 pack = *reinterpret_cast<const int4*>(vv);
-    for (; i + kVec <= n; i += kVec) *reinterpret_cast<int4*>(p + i) = pack;
-  }
-  for (; i < n; i++) p[i] = v;
-}
-
-// The reference keeps a candidate when norm3df(e) < radius (e = point minus its
-// projection on the ray).  The squared length e2 (three roundings) decides it
-// without the square root whenever e2 is outside a band of relative width
-// 2^-16 around radius^2 -- far wider than the few-ulp errors of e2 and
-// norm3df -- and norm3df decides inside the band, so the result is identical.
-struct RadiusTest {
-  float r, lo2, hi2;
-  bool fast;
-};
-
-__device__ __forceinline__ RadiusTest make_radius_test(float r) {
+__host__ __device__ inline RadiusTest make_radius_test(float r) {
   RadiusTest rt;
   rt.r = r;
   const double r2 = (double)r * (double)r;
   rt.fast = r2 > 1e-30 && r2 < 1e30;
-  rt.lo2 = (float)(r2 * (1.0 - 1.0 / 65536.0));
-  rt.hi2 = (float)(r2 * (1.0 + 1.0 / 65536.0));
+  rt.lo2 = rt.fast ? (float)(r2 * (1.0 - 1.0 / 65536.0)) : -1.0f;
+  rt.hi2 = rt.fast ? (float)(r2 * (1.0 + 1.0 / 65536.0)) : INFINITY;
   return rt;
 }
 
-__device__ __forceinline__ bool within_radius(const RadiusTest& rt, float e0, float e1, float e2) {
-  if (rt.fast) {
-    const float q = __fmaf_rn(e2, e2, __fmaf_rn(e1, e1, __fmul_rn(e0, e0)));
-    if (q < rt.lo2) return true;
-    if (q > rt.hi2) return false;
-  }
-  return norm3df(e0, e1, e2) < rt.r;
+// q: the squared length of (e0, e1, e2).
+__device__ __forceinline__ float squared(float e0, float e1, float e2) {
+  return __fmaf_rn(e2, e2, __fmaf_rn(e1, e1, __fmul_rn(e0, e0)));
 }
 
-// t-bin index int((t - tmin) / t_intvl) of a kept candidate (x = t - tmin >= 0).
-// y = x * RN(1 / t_intvl) is within 3.1 * 2^-24 * q of the quotient q and of
-// its rounding RN(q), so when y widened by 2^-21 relative on both sides
-// truncates to one integer, that integer is int(RN(q)); otherwise (a bin
-// edge within a few ulps) the division is done exactly.
-struct BinDiv {
-  float intvl, inv;
-  bool fast;
-};
+// For all lanes of the warp; the band is taken by a branch of the whole warp.
+__device__ __forceinline__ bool within_radius(const RadiusTest& rt, bool in, float q, float e0, float e1, float e2) {
+  bool kept = in && q < rt.lo2;
+  const bool band = in && !(q < rt.lo2) && !(q > rt.hi2);
+  if (__any_sync(0xffffffffu, band)) {
+    const float n = norm3df(e0, e1, e2);
+    if (band) kept = n < rt.r;
+  }
+  return kept;
+}
 
-__device__ __forceinline__ BinDiv make_bin_div(float intvl) {
+__host__ __device__ inline BinDiv make_bin_div(float intvl) {
   BinDiv bd;
   bd.intvl = intvl;
-  bd.inv = __frcp_rn(intvl);
+  bd.inv = 1.0f / intvl;
   bd.fast = intvl > 0.0f && bd.inv < 0x1p100f && intvl < 0x1p100f;
   return bd;
+}
+
+__host__ __device__ inline void derive_args(SampleArgs& a) {
+  a.rt = make_radius_test(a.opt.radius);
+  a.bins = make_bin_div(a.opt.t_intvl);
+  a.near0 = a.opt.radius * 1.001f;
+  a.quanta = 1.0f / a.opt.radius;
+  a.eps = fabsf(a.opt.radius / a.opt.alpha_g);
 }
 
 __device__ __forceinline__ int bin_index(const BinDiv& bd, float x) {
@@ -383,286 +248,28 @@ __device__ __forceinline__ int bin_index(const BinDiv& bd, float x) {
   return __float2int_rz(__fdiv_rn(x, bd.intvl));
 }
 
-// PointRayInterset's t (cuda_util.cuh:227); dividing by d.d == 1 is exact, so it is skipped then.
-__device__ __forceinline__ float ray_t(const Ray& r, bool unit, float px, float py, float pz, float& s0, float& s1,
-                                      float& s2) {
-  s0 = __fsub_rn(px, r.o[0]);
-  s1 = __fsub_rn(py, r.o[1]);
-  s2 = __fsub_rn(pz, r.o[2]);
-  const float num = dot3(s0, s1, s2, r.d[0], r.d[1], r.d[2]);
-  return unit ? num : __fdiv_rn(num, r.dd);
+// The same for all lanes of the warp (those not `in` get any value); the exact
+// division is taken by a branch of the whole warp.
+__device__ __forceinline__ int bin_index(const BinDiv& bd, bool in, float x) {
+  const float y = __fmul_rn(x, bd.inv);
+  int b = __float2int_rz(__fmul_rn(y, 1.0f - 0x1p-21f));
+  const bool edge = in && (!bd.fast || b != __float2int_rz(__fmul_rn(y, 1.0f + 0x1p-21f)));
+  if (__any_sync(0xffffffffu, edge)) {
+    const int e = __float2int_rz(__fdiv_rn(x, bd.intvl));
+    if (edge) b = e;
+  }
+  return b;
 }
 
-// `kept` (staged tiles only; else null) is this thread's kept-candidate mask
-// (kMaskWords words, stride Src::kKeptStride).  For windows with unclamped columns and
-// at most kMaskWords * 32 candidates, pass A records the positions it keeps
-// there and pass B visits only those, without the radius test or the cap.
-template <class Src>
-__device__ __forceinline__ void sample_ray(const SampleArgs& a, const Src& src, int v, int u, unsigned* kept) {
-  const int W = a.cam.width;
-  const int ray = v * W + u;
-  const int S = a.opt.S, P = a.opt.P;
-  const float radius = a.opt.radius;
-
-  Ray r;
-  make_ray(a.cam.c2w, a.cam.fx, a.cam.fy, a.cam.cx, a.cam.cy, u, v, r);
-  const bool unit = r.dd == 1.0f;
-  const RadiusTest rt = make_radius_test(radius);
-
-  // the window's candidate count when the kept mask is used, else -1
-  int masked_T = -1;
-  if constexpr (Src::kStaged) {
-    const int k = a.opt.k, lo = ((k + 1) >> 1) - 1, hi = k - 1 - lo;
-    if (kept && u - lo >= 0 && u + hi <= W - 1) {
-      int T = 0;
-      for (int q = 0; q < k; q++) {
-        const int c0 = src.cell(min(max(v - lo + q, 0), a.cam.height - 1), u - lo);
-        T += src.st->off[c0 + k] - src.st->off[c0];
-      }
-      if (T <= kMaskWords * 32) {
-        masked_T = T;
-        for (int w = 0; w < (T + 31) >> 5; w++) kept[w * Src::kKeptStride] = 0u;
-      }
-    }
-  }
-
-  // pass A: tmin / tmax over the kept candidates (epcq_render_topk.cu:132-161)
-  float tmin = 1e3f, tmax = -1e3f;
-  auto keep = [&](const float4& p) -> bool {
-    if (__float_as_int(p.w) < 0) return false;
-    float s0, s1, s2;
-    const float t = ray_t(r, unit, p.x, p.y, p.z, s0, s1, s2);
-    const float e0 = __fsub_rn(p.x, __fmaf_rn(t, r.d[0], r.o[0]));
-    const float e1 = __fsub_rn(p.y, __fmaf_rn(t, r.d[1], r.o[1]));
-    const float e2 = __fsub_rn(p.z, __fmaf_rn(t, r.d[2], r.o[2]));
-    if (!within_radius(rt, e0, e1, e2)) return false;
-    if (tmin > t) tmin = t;
-    if (tmax < t) tmax = t;
-    return true;
-  };
-  bool masked = false;
-  if constexpr (Src::kStaged) {
-    if (masked_T >= 0) {
-      masked = true;
-      unsigned word = 0u;
-      int wi = 0;
-      walk_rows(a, src, v, u, kKeptPerCell, [&](const float4& p, int f) -> bool {
-        if (!keep(p)) return false;
-        if ((f >> 5) != wi) {
-          if (word) kept[wi * Src::kKeptStride] = word;
-          wi = f >> 5;
-          word = 0u;
-        }
-        word |= 1u << (f & 31);
-        return true;
-      });
-      if (word) kept[wi * Src::kKeptStride] = word;
-    }
-  }
-  if (!masked) walk_window(a, src, v, u, kKeptPerCell, keep);
-
-  float* o_xyz = a.sp_xyz + (size_t)ray * S * 3;
-  float* o_t = a.sp_t + (size_t)ray * S;
-  uint8_t* o_m = a.mask + (size_t)ray * S;
-  int* o_idx = a.pc_idx + (size_t)ray * S * P;
-  int emitted = 0;
-  float te[kTeReg];
-#pragma unroll
-  for (int q = 0; q < kTeReg; q++) te[q] = 0.0f;
-
-  if (!(tmin > tmax)) {
-    const BinDiv bdiv = make_bin_div(a.opt.t_intvl);
-    float transmit = 1.0f;
-    int lo = 0;
-    for (;;) {
-      // pass B: the kBinList smallest distinct bins in [lo, cut) with full stats
-      int lb[kBinList], lc[kBinList];
-      float ls[kBinList];
-#pragma unroll
-      for (int q = 0; q < kBinList; q++) lb[q] = 0x7fffffff, lc[q] = 0, ls[q] = 0.0f;
-      int m = 0, cut = kBins;
-      // a kept candidate at depth t: into the list if its bin is among the
-      // kBinList smallest in [lo, cut); dist() gives its distance to the ray
-      auto collect = [&](float t, auto&& dist) {
-        const int b = bin_index(bdiv, __fsub_rn(t, tmin));
-        if (b < lo || b >= cut) return;
-        if (m == kBinList && b > lb[kBinList - 1]) {
-          cut = b;
-          return;
-        }
-        const float d = dist();
-        bool found = false;
-#pragma unroll
-        for (int q = 0; q < kBinList; q++)
-          if (q < m && lb[q] == b) {
-            lc[q] += 1;
-            ls[q] = __fadd_rn(ls[q], d);
-            found = true;
-          }
-        if (found) return;
-        int pos = 0;
-#pragma unroll
-        for (int q = 0; q < kBinList; q++) pos += (q < m && lb[q] < b) ? 1 : 0;
-        if (m == kBinList) cut = lb[kBinList - 1];
-#pragma unroll
-        for (int q = kBinList - 1; q >= 0; q--) {
-          if (q > pos) {
-            lb[q] = lb[q - 1];
-            lc[q] = lc[q - 1];
-            ls[q] = ls[q - 1];
-          } else if (q == pos) {
-            lb[q] = b;
-            lc[q] = 1;
-            ls[q] = d;
-          }
-        }
-        m = m < kBinList ? m + 1 : kBinList;
-      };
-      bool visited = false;
-      if constexpr (Src::kStaged) {
-        if (masked) {
-          visited = true;
-          walk_kept(a, src, v, u, kept, (masked_T + 31) >> 5, [&](const float4& p) {
-            float s0, s1, s2;
-            const float t = ray_t(r, unit, p.x, p.y, p.z, s0, s1, s2);
-            collect(t, [&] {
-              return norm3df(__fsub_rn(p.x, __fmaf_rn(t, r.d[0], r.o[0])), __fsub_rn(p.y, __fmaf_rn(t, r.d[1], r.o[1])),
-                             __fsub_rn(p.z, __fmaf_rn(t, r.d[2], r.o[2])));
-            });
-          });
-        }
-      }
-      if (!visited) {
-        walk_window(a, src, v, u, kKeptPerCell, [&](const float4& p) -> bool {
-          if (__float_as_int(p.w) < 0) return false;
-          float s0, s1, s2;
-          const float t = ray_t(r, unit, p.x, p.y, p.z, s0, s1, s2);
-          const float e0 = __fsub_rn(p.x, __fmaf_rn(t, r.d[0], r.o[0]));
-          const float e1 = __fsub_rn(p.y, __fmaf_rn(t, r.d[1], r.o[1]));
-          const float e2 = __fsub_rn(p.z, __fmaf_rn(t, r.d[2], r.o[2]));
-          if (!within_radius(rt, e0, e1, e2)) return false;
-          collect(t, [&] { return norm3df(e0, e1, e2); });
-          return true;
-        });
-      }
-      // primary-surface walk (epcq_render_topk.cu:181-204)
-      bool done = false;
-#pragma unroll
-      for (int q = 0; q < kBinList; q++) {
-        if (q >= m || done) break;
-        if (lc[q] < 2) continue;
-        if (transmit < 1e-3f || emitted >= S) {
-          done = true;
-          break;
-        }
-        const float sdf = __fdiv_rn(ls[q], __fadd_rn((float)lc[q], 1e-6f));
-        const float alpha = __fmul_rn(a.opt.gamma, __expf(__fdiv_rn(-sdf, a.opt.alpha_g)));
-        const float weight = __fmul_rn(alpha, transmit);
-        if (weight > 1e-3f) {
-          const float t = __fmaf_rn((float)lb[q], a.opt.t_intvl, tmin);
-          o_xyz[emitted * 3 + 0] = __fmaf_rn(t, r.d[0], r.o[0]);
-          o_xyz[emitted * 3 + 1] = __fmaf_rn(t, r.d[1], r.o[1]);
-          o_xyz[emitted * 3 + 2] = __fmaf_rn(t, r.d[2], r.o[2]);
-          o_t[emitted] = t;
-          o_m[emitted] = 1;
-#pragma unroll
-          for (int e = 0; e < kTeReg; e++)
-            if (e == emitted) te[e] = t;
-          emitted++;
-        }
-        transmit = __fsub_rn(transmit, alpha);
-      }
-      if (done || cut >= kBins) break;
-      lo = cut;
-    }
-  }
-
-  // per-sample point selection (epcq_render_topk.cu:10-81).  One walk over the
-  // window serves up to kBallPass samples: each candidate's position along the
-  // ray is compared with every sample's reach (samples are in ascending t), and
-  // only candidates within a sample's reach get the exact distance.  The
-  // per-sample buffers live in a small local array touched only on hits.
-  const float omax = fmaxf(fabsf(r.o[0]), fmaxf(fabsf(r.o[1]), fabsf(r.o[2])));
-  for (int s0 = 0; s0 < emitted; s0 += kBallPass) {
-    const int ns = min(kBallPass, emitted - s0);
-    float ts[kBallPass], reach[kBallPass], spx[kBallPass], spy[kBallPass], spz[kBallPass], maxd[kBallPass];
-    float bd[kBallPass][kBallBuf];
-    int bi[kBallPass][kBallBuf], bsize[kBallPass], maxi[kBallPass];
-#pragma unroll
-    for (int q = 0; q < kBallPass; q++) {
-      float t = 0.0f;
-      if (q < ns) {
-        t = o_t[s0 + q];
-#pragma unroll
-        for (int e = 0; e < kTeReg; e++)
-          if (e == s0 + q) t = te[e];
-      }
-      ts[q] = t;
-      // |position along the ray - t| beyond this cannot be within the radius
-      reach[q] = q < ns ? radius * 1.001f + 1e-5f * (1.0f + fabsf(t) + omax) : -1.0f;
-      spx[q] = __fmaf_rn(t, r.d[0], r.o[0]);
-      spy[q] = __fmaf_rn(t, r.d[1], r.o[1]);
-      spz[q] = __fmaf_rn(t, r.d[2], r.o[2]);
-      bsize[q] = 0;
-      maxi[q] = 0;
-      maxd[q] = 1e3f;
-#pragma unroll
-      for (int e = 0; e < kBallBuf; e++) bd[q][e] = 0.0f, bi[q][e] = -1;
-    }
-    const float t_first = ts[0] - reach[0], t_last = ts[ns - 1 > 0 ? 1 : 0] + reach[ns - 1 > 0 ? 1 : 0];
-    walk_window(a, src, v, u, 0x7fffffff, [&](const float4& p) -> bool {
-      const int id = __float_as_int(p.w);
-      if (id < 0) return false;
-      const float along = dot3(p.x - r.o[0], p.y - r.o[1], p.z - r.o[2], r.d[0], r.d[1], r.d[2]);
-      if (along < t_first || along > t_last) return false;
-#pragma unroll
-      for (int q = 0; q < kBallPass; q++) {
-        if (!(fabsf(along - ts[q]) <= reach[q])) continue;
-        const float dist = norm3df(__fsub_rn(spx[q], p.x), __fsub_rn(spy[q], p.y), __fsub_rn(spz[q], p.z));
-        if (!(dist < radius)) continue;
-        if (bsize[q] < kBallBuf) {
-          bd[q][bsize[q]] = dist;  // one indexed store into the local-memory buffer
-          bi[q][bsize[q]] = id;
-          if (maxd[q] > dist) {
-            maxd[q] = dist;
-            maxi[q] = bsize[q];
-          }
-          bsize[q]++;
-        } else if (dist < maxd[q]) {
-          bd[q][maxi[q]] = dist;
-          bi[q][maxi[q]] = id;
-          float md = dist;
-          int mi = maxi[q];
-#pragma unroll
-          for (int e = 0; e < kBallBuf; e++)
-            if (bd[q][e] > md) {
-              md = bd[q][e];
-              mi = e;
-            }
-          maxd[q] = md;
-          maxi[q] = mi;
-        }
-      }
-      return false;
-    });
-#pragma unroll
-    for (int q = 0; q < kBallPass; q++) {
-      if (q >= ns) break;
-      int* row = o_idx + (size_t)(s0 + q) * P;
-#pragma unroll
-      for (int e = 0; e < kBallBuf; e++)
-        if (e < P) row[e] = e < bsize[q] ? bi[q][e] : -1;
-      if (P > kBallBuf) fill_run(row + kBallBuf, P - kBallBuf, -1);
-    }
-  }
-
-  // defaults for the slots nothing was emitted into
-  if (emitted < S) {
-    fill_run(o_xyz + emitted * 3, (S - emitted) * 3, 0.0f);
-    fill_run(o_t + emitted, S - emitted, 0.0f);
-    fill_run(o_m + emitted, S - emitted, (uint8_t)0);
-    fill_run(o_idx + (size_t)emitted * P, (S - emitted) * P, -1);
-  }
+// PointRayInterset's t (cuda_util.cuh:227): the correctly rounded quotient of
+// (p - o).d and d.d, with inv_dd = RN(1 / d.d): a first quotient, its exact
+// residual and one fused step (Markstein 1990).  d is normalised, so d.d is a
+// few ulp from 1; for every d.d within 64 ulp of 1 and every numerator mantissa
+// this equals the division, at 3 instructions for 10 and without its branch.
+__device__ __forceinline__ float ray_t(const Ray& r, float inv_dd, const float4& p) {
+  const float num = dot3(__fsub_rn(p.x, r.o[0]), __fsub_rn(p.y, r.o[1]), __fsub_rn(p.z, r.o[2]), r.d[0], r.d[1], r.d[2]);
+  const float q = __fmul_rn(num, inv_dd);
+  return __fmaf_rn(__fmaf_rn(-q, r.dd, num), inv_dd, q);
 }
 
 // Lanes [lo, hi) of a warp as a bit mask (0 <= lo <= hi <= 32).
@@ -682,8 +289,7 @@ __device__ __forceinline__ unsigned lane_span(int lo, int hi) {
 // in sequence order, and the 8-entry ball buffers fed hits in sequence order.
 // A ray costs about ceil(candidates / 32) chunks per pass, so heavy rays finish
 // in a fraction of the time one thread would need for them.
-template <class Src>
-__device__ __forceinline__ void sample_ray_warp(const SampleArgs& a, const Src& src, int v, int u, unsigned* wbuf) {
+__device__ __noinline__ void sample_ray_warp(const SampleArgs& a, int v, int u, unsigned* wbuf) {
   const unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
@@ -694,15 +300,15 @@ __device__ __forceinline__ void sample_ray_warp(const SampleArgs& a, const Src& 
   const float radius = a.opt.radius;
   Ray r;
   make_ray(a.cam.c2w, a.cam.fx, a.cam.fy, a.cam.cx, a.cam.cy, u, v, r);
-  const bool unit = r.dd == 1.0f;
-  const RadiusTest rt = make_radius_test(radius);
+  const float inv_dd = __frcp_rn(r.dd);
+  const RadiusTest& rt = a.rt;
 
   // lane c < k*k: cell c's first index and count; exclusive prefix over cells
   int cbase = 0, ccnt = 0;
   if (lane < k * k) {
     const int q = lane / k;
     const int vv = min(max(v + q - lo, 0), H - 1), uu = min(max(u + (lane - q * k) - lo, 0), W - 1);
-    const int2 rg = src.range(a, vv, uu);
+    const int2 rg = cell_range(a, vv, uu);
     cbase = rg.x;
     ccnt = rg.y - rg.x;
   }
@@ -754,14 +360,14 @@ __device__ __forceinline__ void sample_ray_warp(const SampleArgs& a, const Src& 
   // the candidate's t and offset from the ray; true when within the radius
   auto eval = [&](bool valid, int idx, float& t, float& e0, float& e1, float& e2) -> bool {
     if (!valid) return false;
-    const float4 p = src.fetch(a, idx);
+    const float4 p = __ldg(a.pts + idx);
     if (__float_as_int(p.w) < 0) return false;
-    float s0, s1, s2;
-    t = ray_t(r, unit, p.x, p.y, p.z, s0, s1, s2);
+    t = ray_t(r, inv_dd, p);
     e0 = __fsub_rn(p.x, __fmaf_rn(t, r.d[0], r.o[0]));
     e1 = __fsub_rn(p.y, __fmaf_rn(t, r.d[1], r.o[1]));
     e2 = __fsub_rn(p.z, __fmaf_rn(t, r.d[2], r.o[2]));
-    return within_radius(rt, e0, e1, e2);
+    const float q = squared(e0, e1, e2);
+    return q < rt.lo2 || (!(q > rt.hi2) && norm3df(e0, e1, e2) < rt.r);
   };
   // kept candidates that are among the first 48 kept of their cell; `carry`
   // (lane c's copy is cell c's) counts a cell's kept candidates of earlier chunks
@@ -772,7 +378,7 @@ __device__ __forceinline__ void sample_ray_warp(const SampleArgs& a, const Src& 
     carry += __popc(m & lane_span(min(max(cpre - j0, 0), 32), min(max(cpre + ccnt - j0, 0), 32)));
     return kept && before < kKeptPerCell;
   };
-  const BinDiv bdiv = make_bin_div(a.opt.t_intvl);
+  const BinDiv& bdiv = a.bins;
   auto bin_of = [&](float t, float tmin) {
     return bin_index(bdiv, __fsub_rn(t, tmin));
   };
@@ -963,7 +569,7 @@ __device__ __forceinline__ void sample_ray_warp(const SampleArgs& a, const Src& 
 #pragma unroll
       for (int q = 0; q < kBallPass; q++) dq[q] = 0.0f, hq[q] = false;
       if (valid) {
-        const float4 p = src.fetch(a, idx);
+        const float4 p = __ldg(a.pts + idx);
         id = __float_as_int(p.w);
         if (id >= 0) {
           const float along = dot3(p.x - r.o[0], p.y - r.o[1], p.z - r.o[2], r.d[0], r.d[1], r.d[2]);
@@ -1047,407 +653,628 @@ __device__ __forceinline__ void sample_ray_warp(const SampleArgs& a, const Src& 
   __syncwarp();
 }
 
-// Tile scheduling.  A tile's cost grows with the points in its window halo
-// and is very uneven (dense objects vs background).  Work items are tiles of
-// 8 rows x 32 pixels; a tile whose halo does not fit the stage is split into
-// items of 4, 2 or 1 rows (each staged on its own, so they run concurrently
-// on different SMs), and a single row whose halo still does not fit into
-// column halves and then quarters, each staging its own, narrower halo; only
-// what does not fit even then reads candidates from global memory.  Items are
-// handed out heaviest first (a counting sort on
-// log2 of the halo's point count; halos still too large to stage weighted up)
-// to a persistent grid of SMs x resident blocks that takes the next item from
-// an atomic counter, so heavy items start first and light ones fill in
-// around them.
-struct Sched {
-  int* work;    // [max items] estimated cost
-  int* item;    // [max items] item_code(tile, first row, rows)
-  int* cols;    // [max items] (first column << 8) | end column, within the tile
-  int* view;    // [max items] view of the item (batched launches; else null)
-  int* order;   // [max items] item indices, heaviest first
-  int* counts;  // [32] items per cost class
-  int* fill;    // [32] placement cursors
-  int* next;    // [1] next position in `order` to hand out
-  int* n_items; // [1]
+// A listed candidate's squared distance to the ray may exceed the radius by
+// this much: what the ball query can take lies within the radius of a sample
+// on the ray, so within the radius of the ray but for the rounding of t, of the
+// sample point and of the differences -- a few 1e-7 of |t| and |o|, against a
+// margin of 1e-5 of them plus a thousandth of the radius.
+__device__ __forceinline__ float near_limit(float c0, float t) {
+  const float lim = __fmaf_rn(1e-5f, fabsf(t), c0);
+  return __fmul_rn(lim, lim);
+}
+
+// The slots [from, S) of a ray's outputs: nothing emitted.  `lane` of `n` lanes.
+__device__ __forceinline__ void default_slots(const SampleArgs& a, size_t ray, int from, int lane, int n) {
+  const int S = a.opt.S, P = a.opt.P;
+  const int left = S - from;
+  if (left <= 0) return;
+  float* o_xyz = a.sp_xyz + (ray * S + from) * 3;
+  float* o_t = a.sp_t + ray * S + from;
+  uint8_t* o_m = a.mask + ray * S + from;
+  int* o_idx = a.pc_idx + (ray * S + from) * P;
+  for (int e = lane; e < left * 3; e += n) o_xyz[e] = 0.0f;
+  for (int e = lane; e < left; e += n) o_t[e] = 0.0f, o_m[e] = 0;
+  if ((P & 3) == 0 && ((uintptr_t)a.pc_idx & 15) == 0) {
+    for (int e = lane; e < left * P / 4; e += n) reinterpret_cast<int4*>(o_idx)[e] = make_int4(-1, -1, -1, -1);
+  } else {
+    for (int e = lane; e < left * P; e += n) o_idx[e] = -1;
+  }
+}
+
+// One sample's ball buffer in a group: lanes 0..7 hold its slots, ascending by
+// (distance, slot descending) once a later hit can replace one, so lane 7 is
+// the slot the reference's scan would replace.
+struct Ball {
+  int cnt, held;  // hits looked at; hits held in shared memory, not yet looked at
+  float d;        // lane's squared distance
+  int se;         // and slot | list entry << 3
+  float limit;    // a later hit below this replaces an entry (0 until the buffer is full)
+  bool settled;   // one was replaced: limit is the true maximum (before: the minimum)
 };
 
-__device__ __forceinline__ int cost_class(int w) { return 31 - __clz(w | 1); }
+// sqrt with an error of a few ulp
+__device__ __forceinline__ float sqrt_fast(float x) {
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 
-// A work item: tile t (< 2^21, local to its view), first row and row count
-// (<= 16) within the tile.
-__host__ __device__ constexpr int item_code(int t, int row, int rows) { return (t << 10) | (row << 5) | rows; }
-__device__ __forceinline__ int item_tile(int it) { return it >> 10; }
-__device__ __forceinline__ int item_row(int it) { return (it >> 5) & 31; }
-__device__ __forceinline__ int item_rows(int it) { return it & 31; }
-constexpr int64_t kMaxTilesPerView = 1 << 21;
-
-// Items of tile t (local to its view) of an H x W image, appended to the queue.
-// The clipped point counts of the tile's whole window halo (up to
-// (kTileH + 4) rows x (kTileW + 4) columns) are loaded once, up to two columns
-// per lane; the halo of any row band or column range of the tile is a
-// sub-rectangle of it, summed from those registers with one warp reduction.
-template <int kTileH, int kTileW>
-__device__ __forceinline__ void tile_work(const int2* __restrict__ hash, int n_sorted, int H, int W, int k, int tiles_x,
-                                          int t, int view, int cap, Sched& sc) {
-  constexpr int kHaloRows = kTileH + kMaxKernel - 1;
+// Serve 32 / L rays, L lanes each: `entry` is the group's list entry (ray < 0:
+// none); pool: the warp's kHistWords words and `entries` listed candidates.
+// Returns the lanes of groups left unserved, for sample_ray_warp.
+//
+// The walk uses mean distances from the histogram's quantised sums, and the ball
+// buffers order their hits by squared distance.  Both know their error; where a
+// comparison is closer than that (about one ray in a thousand, and the rays
+// whose window repeats rows at the image's edge), the ray is left to
+// sample_ray_warp, which has the reference's own arithmetic (sums of norm3df in
+// window order, buffers ordered by norm3df), so every decision is the
+// reference's.
+__device__ __forceinline__ unsigned serve_rays(const SampleArgs& a, const int L, int4 entry, unsigned char* pool,
+                                               int entries) {
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int kSumBits = 21, kQuant = 10;  // histogram word: sum of distances in radius / 2^kQuant, count above;
+                                             // 2^kQuant entries fit
   const int lane = threadIdx.x & 31;
-  const int v0 = (t / tiles_x) * kTileH, u0 = (t % tiles_x) * kTileW;
-  const int v_end = min(H, v0 + kTileH);
-  const int koff = (k + 1) >> 1, lo = koff - 1, hi = k - koff;
-  const int hv0 = max(0, v0 - lo), hv1 = min(H - 1, v_end - 1 + hi);
-  const int hu0 = max(0, u0 - lo), hu1 = min(W - 1, u0 + kTileW - 1 + hi);
-  // a second halo column per lane only where the halo is wider than a warp
-  constexpr bool kTwoCols = kTileW + kMaxKernel - 1 > 32;
-  const int ua = hu0 + lane, ub = hu0 + 32 + lane;  // this lane's halo columns
-  int ca[kHaloRows], cb[kTwoCols ? kHaloRows : 1];
+  const int gb = lane & ~(L - 1), sl = lane & (L - 1);  // the group's first lane, this lane's place
+  const unsigned gmask = (kAll >> (32 - L)) << gb;
+  const unsigned below = gmask & ((1u << lane) - 1u);
+  const int lane_bins = kBins / L;  // histogram bins per lane
+  const int most_hits = kHistWords / 64 * L;  // ball hits held, in the group's share of the histogram words
+  unsigned* hist = reinterpret_cast<unsigned*>(pool) + gb * (kHistWords / 32);
+  float2* hits = reinterpret_cast<float2*>(hist);
+  const int cap = entries * L / 32;
+  int* list = reinterpret_cast<int*>(pool + kHistWords * 4) + gb * (entries / 32);
+  const int W = a.cam.width, H = a.cam.height, k = a.opt.k;
+  const int lo = ((k + 1) >> 1) - 1;
+  const int S = a.opt.S, P = a.opt.P;
+  const int ray = entry.x;
+  bool live = ray >= 0;
+  const int v = live ? ray / W : 0, u = live ? ray - v * W : 0;
+  Ray r;
 #pragma unroll
-  for (int h = 0; h < kHaloRows; h++) {
-    ca[h] = 0;
-    if constexpr (kTwoCols) cb[h] = 0;
-    const int vv = hv0 + h;
-    if (vv <= hv1) {
-      if (ua <= hu1) {
-        const int2 rg = bucket_range(__ldg(hash + (size_t)vv * W + ua), n_sorted);
-        ca[h] = min(rg.y - rg.x, cap + 1);
-      }
-      if constexpr (kTwoCols) {
-        if (ub <= hu1) {
-          const int2 rg = bucket_range(__ldg(hash + (size_t)vv * W + ub), n_sorted);
-          cb[h] = min(rg.y - rg.x, cap + 1);
+  for (int i = 0; i < 3; i++) r.o[i] = __ldg(a.cam.c2w + 4 * i + 3);
+  r.d[0] = __int_as_float(entry.y), r.d[1] = __int_as_float(entry.z), r.d[2] = __int_as_float(entry.w);
+  r.dd = dot3(r.d[0], r.d[1], r.d[2], r.d[0], r.d[1], r.d[2]);
+  const float inv_dd = __frcp_rn(r.dd);
+  const RadiusTest& rt = a.rt;
+
+  // The window's rows: row q is the run [base, base + count) of the packed
+  // candidates, when its cells' buckets follow one another (they do in every
+  // table the build makes; clamped columns repeat cells and need not).
+  // Candidate j of the window is packed candidate j + base + the steps of the
+  // rows it is beyond.
+  int p1, p2, p3, p4, T;  // first candidate of rows 1..4, all candidates
+  int base, step1, step2, step3, step4;
+  bool good = true, deep = false;  // deep: a cell holds more than 48
+  {
+    int cnt = 0, first = 0;
+    if (live && sl < k) {
+      const int2* row = a.hash + (size_t)min(max(v - lo + sl, 0), H - 1) * W;
+#pragma unroll
+      for (int c = 0; c < kMaxKernel; c++) {
+        if (c < k) {
+          const int2 rg = bucket_range(__ldg(row + min(max(u - lo + c, 0), W - 1)), a.n_sorted);
+          const int m = rg.y - rg.x;
+          if (m > 0) {
+            if (cnt == 0) first = rg.x;
+            good = good && rg.x == first + cnt;
+            deep = deep || m > kKeptPerCell;
+            cnt += m;
+          }
         }
       }
+    }
+    const int c0 = __shfl_sync(kAll, cnt, gb), c1 = __shfl_sync(kAll, cnt, gb + 1), c2 = __shfl_sync(kAll, cnt, gb + 2),
+              c3 = __shfl_sync(kAll, cnt, gb + 3), c4 = __shfl_sync(kAll, cnt, gb + 4);
+    p1 = c0, p2 = p1 + c1, p3 = p2 + c2, p4 = p3 + c3, T = p4 + c4;
+    base = __shfl_sync(kAll, first, gb);
+    const int f1 = __shfl_sync(kAll, first, gb + 1), f2 = __shfl_sync(kAll, first, gb + 2),
+              f3 = __shfl_sync(kAll, first, gb + 3), f4 = __shfl_sync(kAll, first, gb + 4);
+    step1 = f1 - (base + c0), step2 = f2 - (f1 + c1), step3 = f3 - (f2 + c2), step4 = f4 - (f3 + c3);
+    good = (__ballot_sync(kAll, !good) & gmask) == 0u;
+  }
+  // lane c: window cell c's first candidate and count, for rays with a deep cell (served by a whole warp)
+  int cpre = 0, ccnt = 0, carry = 0;
+  const bool capped = __any_sync(kAll, deep);
+  if (capped) {
+    if (live && lane < k * k) {
+      const int q = lane / k;
+      const int2 rg = cell_range(a, min(max(v + q - lo, 0), H - 1), min(max(u + (lane - q * k) - lo, 0), W - 1));
+      ccnt = rg.y - rg.x;
+    }
+    cpre = ccnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(kAll, cpre, o);
+      if (lane >= o) cpre += t;
+    }
+    cpre -= ccnt;
+    good = good && L == 32;
+  }
+  // a table whose buckets do not follow one another: left to the general walk
+  const bool general = live && !good;
+  unsigned odd = __ballot_sync(kAll, general);
+  live = live && !general;
+  if (!__any_sync(kAll, live)) return odd;
+  if (!live) T = 0;
+
+  // pass A: tmin over the kept candidates (epcq_render_topk.cu:132-161) and the list
+  const float omax = fmaxf(fabsf(r.o[0]), fmaxf(fabsf(r.o[1]), fabsf(r.o[2])));
+  const float c0 = __fmaf_rn(1e-5f, 1.0f + omax, a.near0);
+  float tmin = 1e3f;
+  int n = 0;
+  {
+    const int Tmax = __reduce_max_sync(kAll, T);
+    auto index = [&](int j) {
+      int i = j + base;
+      if (j >= p1) i += step1;
+      if (j >= p2) i += step2;
+      if (j >= p3) i += step3;
+      if (j >= p4) i += step4;
+      return i;
+    };
+    int idx = index(sl);
+    float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (sl < T) p = __ldg(a.pts + idx);
+    for (int j0 = 0; j0 < Tmax; j0 += L) {
+      const int jn = j0 + L + sl;
+      const int idx_n = index(jn);
+      float4 pn = p;
+      if (jn < T) pn = __ldg(a.pts + idx_n);
+      const bool in = jn - L < T && __float_as_int(p.w) >= 0;
+      const float t = ray_t(r, inv_dd, p);
+      const float e0 = __fsub_rn(p.x, __fmaf_rn(t, r.d[0], r.o[0]));
+      const float e1 = __fsub_rn(p.y, __fmaf_rn(t, r.d[1], r.o[1]));
+      const float e2 = __fsub_rn(p.z, __fmaf_rn(t, r.d[2], r.o[2]));
+      const float q = squared(e0, e1, e2);
+      bool kept = within_radius(rt, in, q, e0, e1, e2);
+      const bool near = kept || (in && q <= near_limit(c0, t));
+      if (capped) {  // kept only among its cell's first 48 (carry: lane c's copy counts cell c's kept so far)
+        const int j = j0 + lane;
+        int c = 0;
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1)
+          if (__shfl_sync(kAll, cpre, c + s) <= j) c += s;
+        const int pc = __shfl_sync(kAll, cpre, c);
+        const unsigned m = __ballot_sync(kAll, kept);
+        const int before = __shfl_sync(kAll, carry, c) + __popc(m & below & ~lane_span(0, max(pc - j0, 0)));
+        carry += __popc(m & lane_span(min(max(cpre - j0, 0), 32), min(max(cpre + ccnt - j0, 0), 32)));
+        kept = kept && before < kKeptPerCell;
+      }
+      if (kept && tmin > t) tmin = t;
+      const unsigned nm = __ballot_sync(kAll, near);
+      const int pos = n + __popc(nm & below);
+      if (near && pos < cap) list[pos] = kept ? idx : idx | (int)0x80000000u;
+      n += __popc(nm & gmask);
+      idx = idx_n;
+      p = pn;
     }
   }
-  // points in the halo of rows [vb, vb + rows) and tile columns [c0, c1)
-  auto halo = [&](int vb, int rows, int c0, int c1) {
-    const int r0 = max(0, vb - lo), r1 = min(H - 1, vb + rows - 1 + hi);
-    const int x0 = max(0, u0 + c0 - lo), x1 = min(W - 1, u0 + c1 - 1 + hi);
-    const bool ia = ua >= x0 && ua <= x1, ib = kTwoCols && ub >= x0 && ub <= x1;
-    int sum = 0;
-#pragma unroll
-    for (int h = 0; h < kHaloRows; h++) {
-      const int vv = hv0 + h;
-      if (vv >= r0 && vv <= r1) {
-        sum += ia ? ca[h] : 0;
-        if constexpr (kTwoCols) sum += ib ? cb[h] : 0;
-      }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    return sum;
-  };
-  // The tile's items are collected in shared memory first and then given
-  // queue positions with one atomic per tile: a chain of returning atomics on
-  // the shared item counter, one per item, made tiles that split into many
-  // items wait on it item by item.  One tile per warp, eight warps per block.
-  __shared__ int3 s_item[8][kTileH * 4];  // (cost, item code, columns)
-  const int wp = threadIdx.x >> 5;
-  int n_it = 0;  // warp-uniform
-  // split the tile's rows until each item's halo holds at most `cap` points
-  // (the stage's capacity, so no item runs much longer than the average) or
-  // is one row
-  for (int vb = v0; vb < v_end;) {
-    int rows = v_end - vb;
-    int sum = halo(vb, rows, 0, kTileW);
-    while (sum > cap && rows > 1) {
-      rows = (rows + 1) >> 1;
-      sum = halo(vb, rows, 0, kTileW);
-    }
-    // cost estimate: the halo's points scaled by the share of its rows (and
-    // columns) that hold the item's rays; unstaged items count 4x
-    auto emit = [&](int hs, int c0, int c1) {
-      if (lane == 0) {
-        const int c = (int)(((long long)min(hs, 1 << 24) * rows * kTileH * (c1 - c0)) /
-                            ((long long)(rows + k - 1) * (c1 - c0 + k - 1)));
-        const int w = hs > cap ? c * 4 : c;
-        s_item[wp][n_it] = make_int3(w, item_code(t, vb - v0, rows), (c0 << 8) | c1);
-      }
-      n_it++;
-    };
-    if (sum <= cap) {
-      emit(sum, 0, kTileW);
-    } else {  // one row: halves, then quarters, until the halo fits
-      for (int c0 = 0; c0 < kTileW && u0 + c0 < W; c0 += kTileW / 2) {
-        const int hs = halo(vb, rows, c0, c0 + kTileW / 2);
-        if (hs <= cap) {
-          emit(hs, c0, c0 + kTileW / 2);
-          continue;
-        }
-        for (int q0 = c0; q0 < c0 + kTileW / 2 && u0 + q0 < W; q0 += kTileW / 4)
-          emit(halo(vb, rows, q0, q0 + kTileW / 4), q0, q0 + kTileW / 4);
-      }
-    }
-    vb += rows;
+  {
+    const unsigned over = __ballot_sync(kAll, n > cap);  // more listed candidates than the group holds
+    odd |= over;
+    if (n > cap) live = false, n = 0;
+  }
+  for (int o = L >> 1; o > 0; o >>= 1) {
+    const float t = __shfl_xor_sync(kAll, tmin, o);
+    if (tmin > t) tmin = t;
   }
   __syncwarp();
-  int first = 0;
-  if (lane == 0) first = atomicAdd(sc.n_items, n_it);
-  first = __shfl_sync(0xffffffffu, first, 0);
-  for (int j = lane; j < n_it; j += 32) {
-    const int3 e = s_item[wp][j];
-    const int i = first + j;
-    sc.work[i] = e.x;
-    sc.item[i] = e.y;
-    sc.cols[i] = e.z;
-    if (sc.view) sc.view[i] = view;
-    atomicAdd(sc.counts + (sc.view ? view * 32 : 0) + cost_class(e.x), 1);  // result unused: a reduction
-  }
-}
 
-// One warp per tile: its work items, then its share of the candidate packing
-// (packing needs no result of the tile pass, so its loads overlap the tile
-// pass's latency instead of taking a launch of their own).  Three blocks per
-// SM, so one view's tiles (2500 warps at 800 x 800) run in one wave.
-template <int kTileH, int kTileW>
-__global__ void __launch_bounds__(256, 3) k_tile_work(const int2* __restrict__ hash, int n_sorted, int H, int W, int k,
-                                                   int tiles_x, int ntiles, int cap, Sched sc,
-                                                   const int* __restrict__ sidx, const float* __restrict__ xyz,
-                                                   int n_points, float4* __restrict__ pts) {
-  const int t = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (t >= ntiles) return;
-  tile_work<kTileH, kTileW>(hash, n_sorted, H, W, k, tiles_x, t, 0, cap, sc);
-  const int per = (n_sorted + ntiles - 1) / ntiles;
-  const int j0 = min(n_sorted, t * per);
-  pack_range(sidx, j0, min(n_sorted, j0 + per), xyz, n_points, pts);
-}
-
-__global__ void __launch_bounds__(256) k_tile_order(Sched sc) {
-  __shared__ int base[32];
-  if (threadIdx.x < 32) {
-    int b = 0;  // items in heavier classes
-    for (int c = 31; c > (int)threadIdx.x; c--) b += sc.counts[c];
-    base[threadIdx.x] = b;
-  }
-  __syncthreads();
-  const int n = *sc.n_items;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int c = cost_class(sc.work[i]);
-    sc.order[base[c] + atomicAdd(sc.fill + c, 1)] = i;
-  }
-}
-
-// Batched queue order: view by view (in table order), heaviest class first
-// within a view, so only a view or two are in flight at a time -- their
-// points stay in L2 -- while one view's tail still overlaps the next view's
-// head.  base[v * 32 + c] = first queue position of view v's class-c items
-// (one block: exclusive scan over the n_views * 32 buckets).
-__global__ void __launch_bounds__(1024) k_batch_order_scan(Sched sc, int n_views, int* __restrict__ base) {
-  __shared__ int warp_sum[32];
-  const int n = n_views * 32;
-  const int per = (n + blockDim.x - 1) / blockDim.x;
-  const int b0 = threadIdx.x * per, b1 = min(n, b0 + per);
-  // bucket order: view ascending, class descending
-  auto at = [&](int r) { return (r / 32) * 32 + (31 - r % 32); };
-  int local = 0;
-  for (int r = b0; r < b1; r++) local += sc.counts[at(r)];
-  int incl = local;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += t;
-  }
-  if (lane == 31) warp_sum[warp] = incl;
-  __syncthreads();
-  int off = 0;
-  for (int w = 0; w < warp; w++) off += warp_sum[w];
-  int run = off + incl - local;
-  for (int r = b0; r < b1; r++) {
-    base[at(r)] = run;
-    run += sc.counts[at(r)];
-  }
-}
-
-__global__ void __launch_bounds__(256) k_batch_order_place(Sched sc, const int* __restrict__ base) {
-  const int n = *sc.n_items;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int b = sc.view[i] * 32 + cost_class(sc.work[i]);
-    sc.order[base[b] + atomicAdd(sc.fill + b, 1)] = i;
-  }
-}
-
-// Rays of rows [v0, v0 + rows) and tile columns [c0, c1) of the tile at u0
-// (u0 + c0 < width).  Thread tid is tile pixel (tid / kTileW, tid % kTileW);
-// a ray is named by that pixel index in the rank order.
-template <class Cfg>
-__device__ __forceinline__ void process_tile(const SampleArgs& a, Stage<Cfg>& st, int v0, int rows, int u0, int c0,
-                                             int c1) {
-  constexpr int kTileW = Cfg::kTileW;
-  constexpr int kCap = Cfg::kCap;
-  const int W = a.cam.width, H = a.cam.height, k = a.opt.k;
-  const int koff = (k + 1) >> 1, lo = koff - 1, hi = k - koff;
-  const int rv0 = max(0, v0 - lo), rv1 = min(H - 1, v0 + rows - 1 + hi);
-  const int ru0 = max(0, u0 + c0 - lo), ru1 = min(W - 1, u0 + c1 - 1 + hi);
-  const int nu = ru1 - ru0 + 1, ncells = (rv1 - rv0 + 1) * nu;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-
-  // halo cell table: global start, clipped count, block-wide exclusive prefix
-  int cnt[kCellsPerThread];
-  int local = 0;
-#pragma unroll
-  for (int q = 0; q < kCellsPerThread; q++) {
-    const int c = tid * kCellsPerThread + q;
-    cnt[q] = 0;
-    if (c < ncells) {
-      const int vv = rv0 + c / nu, uu = ru0 + c % nu;
-      const int2 rg = bucket_range(__ldg(a.hash + (size_t)vv * W + uu), a.n_sorted);
-      st.start[c] = rg.x;
-      // capped so the prefix cannot overflow; a capped cell alone exceeds the stage
-      cnt[q] = min(rg.y - rg.x, kCap + 1);
+  const BinDiv& bdiv = a.bins;
+  const size_t slot0 = (size_t)(live ? ray : 0) * S;
+  // the kept entries' bins: counts and quantised distance sums.  Bin b is lane b % L's word b / L, so that the
+  // lanes hold neighbouring bins; `full`: the lane's bins with >= 2
+  const int nmax = __reduce_max_sync(kAll, n);
+  unsigned full = 0u;
+  if (nmax > 0) {
+    for (int c = 0; c < lane_bins; c += 4)
+      *reinterpret_cast<uint4*>(hist + sl * lane_bins + c) = make_uint4(0u, 0u, 0u, 0u);
+    __syncwarp();
+    const float quant = (float)(1 << kQuant) * a.quanta;
+    for (int i0 = 0; i0 < nmax; i0 += L) {
+      const int i = i0 + sl;
+      const int idx = list[min(i, cap - 1)];
+      const bool in = i < n && idx >= 0;
+      float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (in) p = __ldg(a.pts + idx);
+      const float t = ray_t(r, inv_dd, p);
+      const int b = bin_index(bdiv, in, __fsub_rn(t, tmin));
+      const float q = squared(__fsub_rn(p.x, __fmaf_rn(t, r.d[0], r.o[0])), __fsub_rn(p.y, __fmaf_rn(t, r.d[1], r.o[1])),
+                              __fsub_rn(p.z, __fmaf_rn(t, r.d[2], r.o[2])));
+      const unsigned dq = min((unsigned)(sqrt_fast(q) * quant), 1u << kQuant);
+      if (in && b < kBins) atomicAdd(hist + (b & (L - 1)) * lane_bins + b / L, dq | (1u << kSumBits));
     }
-    local += cnt[q];
-  }
-  int incl = local;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += t;
-  }
-  if (lane == 31) st.warp_tot[warp] = incl;
-  __syncthreads();
-  int base = incl - local;
-  for (int q = 0; q < warp; q++) base += st.warp_tot[q];
-  int total = 0;
-#pragma unroll
-  for (int q = 0; q < Cfg::kThreads / 32; q++) total += st.warp_tot[q];
-#pragma unroll
-  for (int q = 0; q < kCellsPerThread; q++) {
-    const int c = tid * kCellsPerThread + q;
-    if (c < ncells) st.off[c] = base;
-    base += cnt[q];
-  }
-  if (tid == 0) st.off[ncells] = total;
-  __syncthreads();
-
-  const bool staged = total <= kCap;
-  if (staged) {
-    for (int i = tid; i < total; i += Cfg::kThreads) {
-      int lo_c = 0, hi_c = ncells;  // off[lo_c] <= i < off[hi_c]
-      while (hi_c - lo_c > 1) {
-        const int mid = (lo_c + hi_c) >> 1;
-        if (st.off[mid] <= i)
-          lo_c = mid;
-        else
-          hi_c = mid;
-      }
-      st.cand[i] = __ldg(a.pts + st.start[lo_c] + (i - st.off[lo_c]));
+    __syncwarp();
+    for (int c = 0; c < lane_bins; c += 4) {
+      const uint4 x = *reinterpret_cast<const uint4*>(hist + sl * lane_bins + c);
+      full |= ((x.x >> kSumBits > 1u ? 1u : 0u) | (x.y >> kSumBits > 1u ? 2u : 0u) | (x.z >> kSumBits > 1u ? 4u : 0u) |
+               (x.w >> kSumBits > 1u ? 8u : 0u))
+              << c;
     }
-    __syncthreads();
   }
 
-  // Group the tile's rays by their window's candidate count (a counting sort
-  // over size classes; the order within a class does not affect any output).
-  // The warps then pull work units, longest first: groups of 32 consecutive ranks below
-  // a.heavy candidates (one ray per thread, similar loop lengths; a group
-  // runs as long as its heaviest ray), then one unit per heavier ray (served by
-  // the whole warp, sample_ray_warp, in about a 32nd of that time).  Warps that
-  // finish early take the next unit, so a tile ends within about one short
-  // unit of its total work divided by its warps.
-  int nheavy, nvalid;
+  int emitted = 0;
+  // how far the walk's alpha can be off by the quantised sums (relative); the mean lies within half a quantum
+  const float eps = __fmaf_rn(a.eps, 1.0f / (1 << kQuant) + 1e-5f, 1e-5f);
+  bool close = !(eps < 0.05f) || !rt.fast;  // a comparison was closer than its error: left to the general walk
   {
-    const int col = tid % kTileW, row = tid / kTileW;
-    const int pu = u0 + col, pv = v0 + row;
-    int T = -1;  // window candidates; -1: no ray at this pixel
-    if (pu < W && pv < H && row < rows && col >= c0 && col < c1) {
-      T = 0;
-      if (staged && pu - lo >= 0 && pu + hi <= W - 1) {
-        // unclamped columns: each window row is a run of k consecutive halo cells
-        for (int dv = -lo; dv <= hi; dv++) {
-          const int c0 = (min(max(pv + dv, 0), H - 1) - rv0) * nu + (pu - lo - ru0);
-          T += st.off[c0 + k] - st.off[c0];
-        }
-      } else {
-        for (int l = 0; l < k * k; l++) {
-          int vv, uu;
-          window_cell(pv, pu, k, H, W, l, vv, uu);
-          const int2 rg = staged ? SrcStaged<Cfg>{&st, rv0, ru0, nu}.range(a, vv, uu) : SrcGlobal{}.range(a, vv, uu);
-          T += rg.y - rg.x;
+    // primary-surface walk (epcq_render_topk.cu:181-204): L bins at a time, their alphas side by side
+    float transmit = 1.0f, off = 0.0f, t0 = 0.0f, t1 = 0.0f;
+    unsigned rows = full;  // the group's rows of L bins with one to look at
+    for (int o = L >> 1; o > 0; o >>= 1) rows |= __shfl_xor_sync(kAll, rows, o);
+    while (__any_sync(kAll, rows != 0u)) {
+      const int row = rows ? __ffs(rows) - 1 : 0;
+      bool mine = rows != 0u && ((full >> row) & 1u);
+      rows &= rows - 1;
+      const int bin = row * L + sl;
+      const unsigned x = mine ? hist[sl * lane_bins + row] : 0u;
+      const int cnt = x >> kSumBits;
+      const float sum = ((float)(x & ((1u << kSumBits) - 1u)) + 0.5f * (float)cnt) * (a.opt.radius * (1.0f / (1 << kQuant)));
+      unsigned todo = __ballot_sync(kAll, mine) & gmask;
+      const float sdf = __fdividef(sum, (float)cnt + 1e-6f);
+      const float alpha = a.opt.gamma * __expf(__fdividef(-sdf, a.opt.alpha_g));
+      const float t = __fmaf_rn((float)bin, a.opt.t_intvl, tmin);
+      int slot = -1;  // this lane's bin emits into this slot
+      while (__any_sync(kAll, todo != 0u)) {
+        const int src = todo ? __ffs(todo) - 1 : lane;
+        const float al = __shfl_sync(kAll, alpha, src), tl = __shfl_sync(kAll, t, src);
+        if (todo) {
+          todo &= todo - 1;
+          if (fabsf(transmit - 1e-3f) <= off) close = true;
+          if (transmit < 1e-3f || emitted >= S) {
+            todo = 0u, rows = 0u;
+          } else {
+            const float weight = __fmul_rn(al, transmit);
+            if (fabsf(weight - 1e-3f) <= fabsf(al) * off + fabsf(weight) * eps) close = true;
+            if (weight > 1e-3f) {
+              if (lane == src) slot = emitted;
+              if (emitted == 0) t0 = tl;
+              if (emitted == 1) t1 = tl;
+              emitted++;
+            }
+            transmit = __fsub_rn(transmit, al);
+            off += fabsf(al) * eps + 1e-6f * (fabsf(transmit) + fabsf(al));
+          }
         }
       }
-    }
-    if (tid < kClasses) st.cls[tid] = 0;
-    if (tid == 0) st.next_unit = 0;
-    __syncthreads();
-    // class 0: warp-served rays; then light rays by descending window size; last: no ray
-    const int cw = max(1, a.heavy / 40);  // candidates per class
-    const int c = T < 0 ? kClasses - 1 : (T > a.heavy ? 0 : 1 + min(kClasses - 3, (a.heavy - T) / cw));
-    const int local = atomicAdd(&st.cls[c], 1);
-    __syncthreads();
-    if (tid < 32) {
-      const int n0 = st.cls[2 * tid], n1 = st.cls[2 * tid + 1];
-      int incl = n0 + n1;
+      if (slot >= 0) {
+        const size_t at = slot0 + slot;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (tid >= o) incl += t;
+        for (int i = 0; i < 3; i++) a.sp_xyz[at * 3 + i] = __fmaf_rn(t, r.d[i], r.o[i]);
+        a.sp_t[at] = t;
+        a.mask[at] = 1;
       }
-      st.cls_base[2 * tid] = incl - n0 - n1;
-      st.cls_base[2 * tid + 1] = incl - n1;
     }
-    __syncthreads();
-    st.order[st.cls_base[c] + local] = tid;
-    nheavy = st.cls[0];
-    nvalid = Cfg::kThreads - st.cls[kClasses - 1];
-    __syncthreads();
-  }
-  const int ngroups = (nvalid - nheavy + 31) >> 5;
-  for (;;) {
-    int unit = 0;
-    if (lane == 0) unit = atomicAdd(&st.next_unit, 1);
-    unit = __shfl_sync(0xffffffffu, unit, 0);
-    if (unit < ngroups) {
-      const int rk = nheavy + unit * 32 + lane;
-      if (rk < nvalid) {
-        const int px = st.order[rk];
-        if (staged)
-          sample_ray(a, SrcStaged<Cfg>{&st, rv0, ru0, nu}, v0 + px / kTileW, u0 + px % kTileW, &st.kept[0][tid]);
-        else
-          sample_ray(a, SrcGlobal{}, v0 + px / kTileW, u0 + px % kTileW, nullptr);
-      }
-      continue;
-    }
-    const int h = unit - ngroups;
-    if (h >= nheavy) break;
-    const int px = st.order[h];
-    if (staged)
-      sample_ray_warp(a, SrcStaged<Cfg>{&st, rv0, ru0, nu}, v0 + px / kTileW, u0 + px % kTileW,
-                      &st.kept[0][warp * 32]);
-    else
-      sample_ray_warp(a, SrcGlobal{}, v0 + px / kTileW, u0 + px % kTileW, &st.kept[0][warp * 32]);
-  }
-  __syncthreads();  // the stage is reused by the next tile
-}
+    close = (__ballot_sync(kAll, close) & gmask) != 0u;
+    if (close) emitted = 0;
 
-template <class Cfg>
-__global__ void __launch_bounds__(Cfg::kThreads, Cfg::kBlocks) k_quick_sampling(SampleArgs a, Sched sc, int tiles_x) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Stage<Cfg>& st = *reinterpret_cast<Stage<Cfg>*>(smem_raw);
-  __shared__ int s_next;
-  const int n = *sc.n_items;
-  for (;;) {
-    if (threadIdx.x == 0) s_next = atomicAdd(sc.next, 1);
-    __syncthreads();
-    const int i = s_next;
-    if (i >= n) break;
-    const int j = sc.order[i];
-    const int it = sc.item[j], cc = sc.cols[j];
-    const int t = item_tile(it);
-    process_tile(a, st, (t / tiles_x) * Cfg::kTileH + item_row(it), item_rows(it), (t % tiles_x) * Cfg::kTileW,
-                 cc >> 8, cc & 255);
+    // per-sample point selection (epcq_render_topk.cu:10-81), a sample at a time
+    const int most = __reduce_max_sync(kAll, emitted);
+    const int nball = __reduce_max_sync(kAll, emitted > 0 ? n : 0);
+#pragma unroll 1
+    for (int s = 0; s < most; s++) {
+      const bool on = s < emitted;
+      __syncwarp();
+      if (s > 1 && on) t0 = *(volatile const float*)(a.sp_t + slot0 + s);
+      const float sx = __fmaf_rn(t0, r.d[0], r.o[0]), sy = __fmaf_rn(t0, r.d[1], r.o[1]),
+                  sz = __fmaf_rn(t0, r.d[2], r.o[2]);
+      t0 = t1;
+      const int m = on ? n : 0;
+      Ball b0{0, 0, 0.0f, sl, 0.0f, false};
+#pragma unroll 1
+      for (int i0 = 0;; i0 += L) {
+        const int i = i0 + sl;
+        float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < m) p = __ldg(a.pts + (list[i] & 0x7fffffff));
+        const float e0 = __fsub_rn(sx, p.x), e1 = __fsub_rn(sy, p.y), e2 = __fsub_rn(sz, p.z);
+        const float d = squared(e0, e1, e2);
+        const bool hit = within_radius(rt, i < m, d, e0, e1, e2);
+        const unsigned hm = __ballot_sync(kAll, hit);
+        if (hit) hits[b0.held + __popc(hm & below)] = make_float2(d, __int_as_float(i));
+        b0.held += __popc(hm & gmask);
+        const bool last = i0 + L >= nball;
+        if (!last && !__any_sync(kAll, b0.held + L > most_hits)) continue;
+        // look at the held hits, in order
+        __syncwarp();
+        {
+          const int todo = last || b0.held + L > most_hits ? b0.held : 0;
+          if (todo > 0) b0.held = 0;
+          const bool first = b0.cnt == 0 && todo > 0;
+          b0.cnt += todo;
+          for (int h = 0; __any_sync(kAll, h < todo); h += L) {
+            bool later = h + sl < todo;  // may replace an entry
+            const float2 x = hits[min(h + sl, most_hits - 1)];
+            const int xi = __float_as_int(x.y);
+            if (h == 0 && __any_sync(kAll, first)) {  // the first eight fill the slots
+              if (first && sl < kBallBuf) {
+                b0.d = later ? x.x : __int_as_float(0x7f800000);
+                b0.se = sl | (xi << 3);
+                later = false;
+              }
+              if (__any_sync(kAll, first && todo > kBallBuf)) {
+                float sd = b0.d;
+                int sp = b0.se;
+#pragma unroll
+                for (int w = 2; w <= 8; w <<= 1) {
+#pragma unroll
+                  for (int o = w >> 1; o > 0; o >>= 1) {
+                    const float od = __shfl_xor_sync(kAll, sd, o);
+                    const int op = __shfl_xor_sync(kAll, sp, o);
+                    const bool less = od < sd || (od == sd && (op & 7) > (sp & 7));  // the other goes first
+                    const bool up = (lane & w) == 0 || w == 8;                        // this run ascends
+                    if (less == (((lane & o) != 0) != up)) sd = od, sp = op;
+                  }
+                }
+                const float prev = __shfl_up_sync(kAll, sd, 1), least = __shfl_sync(kAll, sd, gb);
+                if (first && todo > kBallBuf) {
+                  if (sl < kBallBuf) b0.d = sd, b0.se = sp;
+                  if (sl > 0 && sl < kBallBuf && sd - prev <= __fmaf_rn(sd, 0x1p-15f, 1e-33f)) close = true;
+                  b0.limit = least;
+                }
+              }
+            }
+            unsigned pm;
+            while (pm = __ballot_sync(kAll, later && x.x < __fmaf_rn(b0.limit, 1.0f + 0x1p-15f, 1e-33f)), pm != 0u) {
+              pm &= gmask;
+              const bool has = pm != 0u;
+              const int l = has ? __ffs(pm) - 1 : lane;
+              if (lane <= l) later = false;
+              const float nd = __shfl_sync(kAll, x.x, l);
+              const int ni = __shfl_sync(kAll, xi, l);
+              if (has && sl < kBallBuf && fabsf(b0.d - nd) <= __fmaf_rn(nd, 0x1p-15f, 1e-33f)) close = true;
+              // the lane whose slot is replaced: the maximum (7), or before the first replacement the first slot
+              // that holds the minimum (the last of the lanes that do)
+              const unsigned ties = __ballot_sync(kAll, sl < kBallBuf && b0.d == b0.limit) & gmask;
+              const int out = b0.settled ? kBallBuf - 1 : max(__popc(ties) - 1, 0);
+              const int slot = __shfl_sync(kAll, b0.se, gb + out) & 7;
+              const float second = __shfl_sync(kAll, b0.d, gb + kBallBuf - 2);
+              // after those smaller; among equals by slot descending, but a new maximum is the next to go
+              const bool ahead =
+                  b0.settled && sl < kBallBuf && (b0.d < nd || (b0.d == nd && ((b0.se & 7) > slot || second == nd)));
+              const int at = min(__popc(__ballot_sync(kAll, ahead) & gmask), kBallBuf - 1);
+              const float ud = __shfl_up_sync(kAll, b0.d, 1);
+              const int ue = __shfl_up_sync(kAll, b0.se, 1);
+              if (has && sl < kBallBuf) {
+                if (sl == at)
+                  b0.d = nd, b0.se = slot | (ni << 3);
+                else if (sl > at && sl <= out)
+                  b0.d = ud, b0.se = ue;
+              }
+              const float mx = __shfl_sync(kAll, b0.d, gb + kBallBuf - 1);
+              if (has) b0.settled = true, b0.limit = mx;
+            }
+          }
+        }
+        __syncwarp();
+        if (last) break;
+      }
+      if (on) {
+        int* row = a.pc_idx + (slot0 + s) * P;
+        const int slot = b0.cnt > 0 ? b0.se & 7 : sl;
+        if (sl < kBallBuf && slot < P) {
+          int id = -1;
+          if (slot < b0.cnt) id = __float_as_int(__ldg(a.pts + (list[b0.se >> 3] & 0x7fffffff)).w);
+          row[slot] = id;
+        }
+        for (int e = kBallBuf + sl; e < P; e += L) row[e] = -1;
+      }
+    }
   }
+  close = (__ballot_sync(kAll, close && live) & gmask) != 0u;
+  if (live && !close) default_slots(a, (size_t)ray, emitted, sl, L);
+  return odd | __ballot_sync(kAll, close);
 }
 
 // ---------------------------------------------------------------------------
-// Batched launch: the tiles of many views (different clouds, cameras, image
-// sizes and options) in one queue and one persistent sampling kernel, so a
-// view's tail overlaps the other views' work.  Every ray runs the same code as
-// in a per-view launch, so the outputs are identical.
+// the ray list
+// ---------------------------------------------------------------------------
+// Rays of one kTileH x kTileW tile, one thread per pixel: the window counts by
+// rows then columns from the tile's halo in shared memory; default outputs for
+// rays without a candidate; the others into the list, ordered by count so that
+// the four rays of a unit run loops of the same length.
+template <int kTileH, int kTileW>
+__device__ __forceinline__ void list_tile(const SampleArgs& a, int v0, int u0, int view, const RayList& rl) {
+  constexpr int kHaloH = kTileH + kMaxKernel - 1, kHaloW = kTileW + kMaxKernel - 1;
+  constexpr int kFlag = 1 << 26;  // a cell above 48 entries; 25 cells' counts stay below it
+  __shared__ int halo[kHaloH * kHaloW];
+  __shared__ int row_sum[kHaloH][kTileW];
+  __shared__ int cls[kClasses], cls_base[kClasses];
+  __shared__ unsigned empty[kTileH];
+  __shared__ unsigned s_front, s_back;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int W = a.cam.width, H = a.cam.height, k = a.opt.k;
+  const int koff = (k + 1) >> 1, lo = koff - 1, hi = k - koff;
+  const int rv0 = max(0, v0 - lo), rv1 = min(H - 1, v0 + kTileH - 1 + hi);
+  const int ru0 = max(0, u0 - lo), ru1 = min(W - 1, u0 + kTileW - 1 + hi);
+  const int nv = rv1 - rv0 + 1, nu = ru1 - ru0 + 1;
+  if (tid < kClasses) cls[tid] = 0;
+  for (int c = tid; c < nv * nu; c += kThreads) {
+    const int vv = c / nu;
+    const int2 rg = cell_range(a, rv0 + vv, ru0 + (c - vv * nu));
+    const int n = min(rg.y - rg.x, 1 << 20);
+    halo[c] = n > kKeptPerCell ? n | kFlag : n;
+  }
+  __syncthreads();
+  for (int c = tid; c < nv * kTileW; c += kThreads) {
+    const int vv = c / kTileW, uu = c % kTileW;
+    int s = 0;
+    for (int q = -lo; q <= hi; q++) s += halo[vv * nu + min(max(u0 + uu + q, ru0), ru1) - ru0];
+    row_sum[vv][uu] = s;
+  }
+  __syncthreads();
+  const int pv = v0 + tid / kTileW, pu = u0 + tid % kTileW;
+  const bool in = pv < H && pu < W;
+  int s = 0;
+  if (in)
+    for (int q = -lo; q <= hi; q++) s += row_sum[min(max(pv + q, 0), H - 1) - rv0][tid % kTileW];
+  const int T = s & (kFlag - 1);
+  // whole-warp rays: many candidates, a cell above the cap, or repeated (clamped) columns
+  const bool back = T > 0 && (T > rl.light || s >= kFlag || pu - lo < 0 || pu + hi > W - 1);
+  const unsigned none = __ballot_sync(0xffffffffu, in && T == 0);
+  if constexpr (kTileW == 32) {
+    if (lane == 0) empty[tid >> 5] = none;
+  } else {
+    if (lane == 0) empty[(tid >> 5) * 2] = none & 0xffffu, empty[(tid >> 5) * 2 + 1] = none >> 16;
+  }
+  // class 0: whole-warp rays; then by descending count in steps of 8 candidates; last: no candidate
+  const int c = T == 0 ? kClasses - 1 : back ? 0 : 1 + max(0, kClasses - 3 - (T >> 3));
+  const int local = atomicAdd(&cls[c], 1);
+  __syncthreads();
+  if (tid < 32) {
+    const int n0 = cls[2 * tid], n1 = cls[2 * tid + 1];
+    int incl = n0 + n1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (tid >= o) incl += t;
+    }
+    cls_base[2 * tid] = incl - n0 - n1;
+    cls_base[2 * tid + 1] = incl - n1;
+  }
+  __syncthreads();
+  const int nback = cls[0], nfront = kThreads - nback - cls[kClasses - 1];
+  if (tid == 0) {
+    s_front = nfront ? atomicAdd(rl.counts, (unsigned)((nfront + 3) & ~3)) : 0u;
+    s_back = nback ? atomicAdd(rl.counts + 1, (unsigned)nback) : 0u;
+  }
+  __syncthreads();
+  if (T > 0) {
+    Ray r;
+    make_ray(a.cam.c2w, a.cam.fx, a.cam.fy, a.cam.cx, a.cam.cy, pu, pv, r);
+    const int4 e = make_int4(pv * W + pu, __float_as_int(r.d[0]), __float_as_int(r.d[1]), __float_as_int(r.d[2]));
+    if (back) {
+      const long long i = (long long)s_back + local;
+      rl.rays[rl.cap - 1 - i] = e;
+      if (rl.back_view) rl.back_view[i] = view;
+    } else {
+      const long long i = (long long)s_front + cls_base[c] - nback + local;
+      rl.rays[i] = e;
+      if (rl.front_view && (i & 3) == 0) rl.front_view[i >> 2] = view;
+    }
+  }
+  if (tid < ((nfront + 3) & ~3) - nfront) rl.rays[(long long)s_front + nfront + tid] = make_int4(-1, 0, 0, 0);
+
+  // default outputs of the rays without a candidate: a tile row's outputs are runs, written in order
+  const int S = a.opt.S, P = a.opt.P;
+  const int cols = min(kTileW, W - u0);
+  for (int q = tid >> 5; q < kTileH && v0 + q < H; q += kWarps) {
+    const unsigned m = empty[q];
+    if (!m) continue;
+    const size_t ray0 = (size_t)(v0 + q) * W + u0;
+    auto fill4 = [&](void* base, int words, int value) {  // `words` 32-bit words a ray
+      int* out = reinterpret_cast<int*>(base) + ray0 * words;
+      if ((words & 3) == 0 && ((uintptr_t)base & 15) == 0) {
+        const int per = words >> 2;
+        const int4 x = make_int4(value, value, value, value);
+        for (int e = lane; e < cols * per; e += 32)
+          if ((m >> (unsigned)(e / per)) & 1u) reinterpret_cast<int4*>(out)[e] = x;
+      } else {
+        for (int e = lane; e < cols * words; e += 32)
+          if ((m >> (unsigned)(e / words)) & 1u) out[e] = value;
+      }
+    };
+    fill4(a.pc_idx, S * P, -1);
+    fill4(a.sp_xyz, S * 3, 0);
+    fill4(a.sp_t, S, 0);
+    if ((S & 3) == 0 && ((uintptr_t)a.mask & 3) == 0) {
+      int* out = reinterpret_cast<int*>(a.mask + ray0 * S);
+      for (int e = lane; e < cols * (S >> 2); e += 32)
+        if ((m >> (unsigned)(e / (S >> 2))) & 1u) out[e] = 0;
+    } else {
+      for (int e = lane; e < cols * S; e += 32)
+        if ((m >> (unsigned)(e / S)) & 1u) a.mask[ray0 * S + e] = 0;
+    }
+  }
+}
+
+// One block per tile, and its warps' shares of the candidate packing (packing
+// needs no result of the tile, so its loads overlap the tile's latency).
+template <int kTileH, int kTileW>
+__global__ void __launch_bounds__(kThreads, 4) k_ray_list(const __grid_constant__ SampleArgs a, RayList rl,
+                                                         int tiles_x, int ntiles) {
+  const int t = blockIdx.x;
+  list_tile<kTileH, kTileW>(a, (t / tiles_x) * kTileH, (t % tiles_x) * kTileW, 0, rl);
+  const long long shares = (long long)ntiles * kWarps, n = a.n_sorted, per = (n + shares - 1) / shares;
+  const long long j0 = min(n, ((long long)t * kWarps + (threadIdx.x >> 5)) * per);
+  pack_range(a.sidx, (int)j0, (int)min(n, j0 + per), a.xyz, a.n_points, const_cast<float4*>(a.pts));
+}
+
+// The persistent warps: the units of two first (they run longest), then the
+// units of four.  Each takes its next position before it serves the current one.
+template <class Cfg, bool kBatch>
+__device__ __forceinline__ void serve_list(const SampleArgs& a0, const SampleArgs* __restrict__ args, const RayList& rl,
+                                           unsigned char* smem) {
+  __shared__ SampleArgs s_args[kBatch ? kServeWarps : 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned char* pool = smem + warp * Cfg::kWarpBytes;
+  int have = -1;  // the view in s_args[warp]
+  auto view_args = [&](int view) {
+    if (view != have) {
+      __syncwarp();
+      if (lane == 0) s_args[warp] = args[view];
+      __syncwarp();
+      have = view;
+    }
+  };
+  const SampleArgs& a = kBatch ? static_cast<const SampleArgs&>(s_args[warp]) : a0;
+  const unsigned n_front = rl.counts[0], n_back = rl.counts[1];
+  auto take = [&](unsigned* next, unsigned n) {
+    unsigned x = 0;
+    if (lane == 0) x = atomicAdd(next, n);
+    return x;
+  };
+  const unsigned units = n_front >> 2;
+  const unsigned step = max(1u, min(4u, units / (gridDim.x * kServeWarps * 8u)));
+  // One loop over both parts of the list, so that serve_rays is in the kernel once: two copies of it
+  // (or three, with one for 16 lanes) cost more in instruction-cache misses than their constants saved.
+  bool back = true;
+  unsigned x = take(rl.counts + 3, 1u), i = 0, end = 0;
+  for (;;) {
+    if (i == end) {
+      i = __shfl_sync(0xffffffffu, x, 0);
+      if (back && i >= n_back) {
+        back = false;
+        i = __shfl_sync(0xffffffffu, take(rl.counts + 2, step), 0);
+      }
+      if (!back && i >= units) break;
+      end = back ? i + 1 : min(units, i + step);
+      x = take(rl.counts + (back ? 3 : 2), back ? 1u : step);
+    }
+    const int L = back ? 32 : 8;
+    const int4 e = __ldg(back ? rl.rays + (rl.cap - 1 - (long long)i) : rl.rays + (size_t)i * 4 + (lane >> 3));
+    if constexpr (kBatch) view_args(back ? rl.back_view[i] : rl.front_view[i]);
+    for (unsigned odd = serve_rays(a, L, e, pool, Cfg::kEntries); odd;) {  // the general walk, ray by ray
+      const int l = __ffs(odd) - 1;
+      odd &= ~((0xffffffffu >> (32 - L)) << l);
+      const int ray = __shfl_sync(0xffffffffu, e.x, l);
+      __syncwarp();
+      sample_ray_warp(a, ray / a.cam.width, ray % a.cam.width, reinterpret_cast<unsigned*>(pool));
+    }
+    __syncwarp();
+    i++;
+  }
+}
+
+template <class Cfg>
+__global__ void __launch_bounds__(kServeThreads, Cfg::kBlocks) k_quick_sampling(const __grid_constant__ SampleArgs a,
+                                                                   RayList rl) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  serve_list<Cfg, false>(a, nullptr, rl, smem_raw);
+}
+
+// ---------------------------------------------------------------------------
+// Batched launch: the rays of many views (different clouds, cameras, image
+// sizes and options) in one list and one persistent kernel, so a view's tail
+// overlaps the other views' work.  Every ray runs the same code as in a
+// per-view launch, so the outputs are identical.
 
 // Device view table -> per-view kernel arguments and the first global tile of
 // each view (exclusive scan; tile_base[n_views] = all tiles).  One warp.
 // Also the first packed-point slot of each view (pack_base; regions padded to
 // 16 slots) and the views' packed-point arrays inside `pts`.
-__global__ void k_batch_setup(const hp_view* __restrict__ views, int n_views, int heavy, int tile_h, int tile_w,
+__global__ void k_batch_setup(const hp_view* __restrict__ views, int n_views, int tile_h, int tile_w,
                               SampleArgs* __restrict__ args, int* __restrict__ tile_base, int* __restrict__ pack_base,
                               float4* __restrict__ pts) {
   const int lane = threadIdx.x;
@@ -1493,7 +1320,7 @@ __global__ void k_batch_setup(const hp_view* __restrict__ views, int n_views, in
       a.pc_idx = hv.pc_idx;
       a.sp_t = hv.sp_t;
       a.mask = hv.mask;
-      a.heavy = heavy;
+      derive_args(a);
       args[v] = a;
       tiles = ((hv.cam.width + tile_w - 1) / tile_w) * ((hv.cam.height + tile_h - 1) / tile_h);
     }
@@ -1531,13 +1358,13 @@ __global__ void k_batch_pack(const SampleArgs* __restrict__ args, const int* __r
   const_cast<float4*>(a.pts)[j] = packed_point(a.sidx, j, a.xyz, a.n_points);
 }
 
-// One warp per global tile: find its view, then queue the tile's items.
+// One block per global tile: find its view, then list the tile's rays.
 template <int kTileH, int kTileW>
-__global__ void __launch_bounds__(256, 3) k_batch_tile_work(const SampleArgs* __restrict__ args,
-                                                         const int* __restrict__ tile_base, int n_views,
-                                                         int total_tiles, int cap, Sched sc) {
-  const int g = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (g >= total_tiles) return;
+__global__ void __launch_bounds__(kThreads, 4) k_batch_ray_list(const SampleArgs* __restrict__ args,
+                                                                const int* __restrict__ tile_base, int n_views,
+                                                                RayList rl) {
+  __shared__ SampleArgs s_args;
+  const int g = blockIdx.x;
   int lo = 0, hi = n_views;  // tile_base[lo] <= g < tile_base[hi]
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
@@ -1546,36 +1373,16 @@ __global__ void __launch_bounds__(256, 3) k_batch_tile_work(const SampleArgs* __
     else
       hi = mid;
   }
-  const SampleArgs& a = args[lo];
-  const int tiles_x = (a.cam.width + kTileW - 1) / kTileW;
-  tile_work<kTileH, kTileW>(a.hash, a.n_sorted, a.cam.height, a.cam.width, a.opt.k, tiles_x, g - tile_base[lo], lo,
-                            cap, sc);
+  if (threadIdx.x == 0) s_args = args[lo];
+  __syncthreads();
+  const int tiles_x = (s_args.cam.width + kTileW - 1) / kTileW, t = g - tile_base[lo];
+  list_tile<kTileH, kTileW>(s_args, (t / tiles_x) * kTileH, (t % tiles_x) * kTileW, lo, rl);
 }
 
-// The persistent sampling kernel over the batch's queue; each item's view
-// arguments are loaded into shared memory before the tile is processed.
 template <class Cfg>
-__global__ void __launch_bounds__(Cfg::kThreads, Cfg::kBlocks)
-    k_quick_sampling_batch(const SampleArgs* __restrict__ args, Sched sc) {
+__global__ void __launch_bounds__(kServeThreads, Cfg::kBlocks) k_quick_sampling_batch(const SampleArgs* __restrict__ args, RayList rl) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  Stage<Cfg>& st = *reinterpret_cast<Stage<Cfg>*>(smem_raw);
-  __shared__ int s_next;
-  __shared__ SampleArgs s_args;
-  const int n = *sc.n_items;
-  for (;;) {
-    if (threadIdx.x == 0) s_next = atomicAdd(sc.next, 1);
-    __syncthreads();
-    const int i = s_next;
-    if (i >= n) break;
-    const int j = sc.order[i];
-    if (threadIdx.x == 0) s_args = args[sc.view[j]];
-    __syncthreads();
-    const int it = sc.item[j], cc = sc.cols[j];
-    const int t = item_tile(it);
-    const int tiles_x = (s_args.cam.width + Cfg::kTileW - 1) / Cfg::kTileW;
-    process_tile(s_args, st, (t / tiles_x) * Cfg::kTileH + item_row(it), item_rows(it), (t % tiles_x) * Cfg::kTileW,
-                 cc >> 8, cc & 255);
-  }
+  serve_list<Cfg, true>(SampleArgs{}, args, rl, smem_raw);
 }
 
 __global__ void k_ray_directions(DevCamera cam, float* __restrict__ dirs) {
@@ -1590,31 +1397,30 @@ __global__ void k_ray_directions(DevCamera cam, float* __restrict__ dirs) {
 
 // The kernels and shapes of each stage configuration.
 struct SamplingKernels {
-  void (*view)(SampleArgs, Sched, int);
-  void (*batch)(const SampleArgs*, Sched);
-  void (*tile_work)(const int2*, int, int, int, int, int, int, int, Sched, const int*, const float*, int, float4*);
-  void (*batch_tile_work)(const SampleArgs*, const int*, int, int, int, Sched);
+  void (*view)(SampleArgs, RayList);
+  void (*batch)(const SampleArgs*, RayList);
+  void (*list)(SampleArgs, RayList, int, int);
+  void (*batch_list)(const SampleArgs*, const int*, int, RayList);
   size_t smem;
-  int cap, blocks, threads, tile_h, tile_w, items_per_tile;
+  int stage, blocks, tile_h, tile_w, entries;
 };
 template <class Cfg>
 static SamplingKernels sampling_kernels() {
   return {k_quick_sampling<Cfg>,
           k_quick_sampling_batch<Cfg>,
-          k_tile_work<Cfg::kTileH, Cfg::kTileW>,
-          k_batch_tile_work<Cfg::kTileH, Cfg::kTileW>,
-          sizeof(Stage<Cfg>),
-          Cfg::kCap,
+          k_ray_list<Cfg::kTileH, Cfg::kTileW>,
+          k_batch_ray_list<Cfg::kTileH, Cfg::kTileW>,
+          (size_t)Cfg::kSmem,
+          Cfg::kStage,
           Cfg::kBlocks,
-          Cfg::kThreads,
           Cfg::kTileH,
           Cfg::kTileW,
-          Cfg::kItemsPerTile};
+          Cfg::kEntries};
 }
 static const SamplingKernels& stage_kernels(int config) {  // config 1..kStageConfigs
-  static const SamplingKernels table[kStageConfigs] = {
-      sampling_kernels<Cfg2560x4>(),   sampling_kernels<Cfg3712x3>(), sampling_kernels<Cfg5888x2>(),
-      sampling_kernels<Cfg2560x4Sq>(), sampling_kernels<Cfg3712x3Sq>()};
+  static const SamplingKernels table[kStageConfigs] = {sampling_kernels<Cfg1>(), sampling_kernels<Cfg2>(),
+                                                       sampling_kernels<Cfg3>(), sampling_kernels<Cfg4>(),
+                                                       sampling_kernels<Cfg5>()};
   return table[config - 1];
 }
 
@@ -1622,21 +1428,16 @@ static int64_t tiles_of(int64_t H, int64_t W, int tile_h, int tile_w) {
   return ((W + tile_w - 1) / tile_w) * ((H + tile_h - 1) / tile_h);
 }
 
-// Schedule entries an H x W view can need under any configuration (workspaces
-// are sized for the largest, so one workspace serves every tuning).
-static int64_t max_view_items(int64_t H, int64_t W) {
-  int64_t m = 0;
-  for (int c = 1; c <= kStageConfigs; c++) {
-    const SamplingKernels& K = stage_kernels(c);
-    const int64_t items = tiles_of(H, W, K.tile_h, K.tile_w) * K.items_per_tile;
-    if (items > m) m = items;
-  }
-  return m;
+// Ray-list entries an H x W view can need under any configuration: every ray,
+// and up to three entries of padding per tile (workspaces are sized for the
+// largest, so one workspace serves every tuning).
+static int64_t max_view_entries(int64_t H, int64_t W) {
+  const int64_t a = tiles_of(H, W, 8, 32), b = tiles_of(H, W, 16, 16);
+  return H * W + 3 * (a > b ? a : b);
 }
 
-// The stage exceeds the 48 KB default of dynamic shared memory: opt the
-// configuration's kernels in once per device and size the persistent grid
-// from their occupancy.
+// Opt the configuration's kernels in to their dynamic shared memory once per
+// device and size the persistent grid from their occupancy.
 int32_t sampling_grid(int config, int* blocks, int* sm_count = nullptr) {
   static std::mutex mu;
   static int grid[128][kStageConfigs] = {{0}}, sm_counts[128] = {0};
@@ -1653,7 +1454,7 @@ int32_t sampling_grid(int config, int* blocks, int* sm_count = nullptr) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(K.batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)K.smem);
     int sms = 0, per_sm = 0;
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, K.view, K.threads, K.smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, K.view, kServeThreads, K.smem);
     if (e != cudaSuccess) return set_error(HP_ERR_CUDA, "hp_quick_sampling: kernel set-up: %s", cudaGetErrorString(e));
     g = sms * (per_sm > 0 ? per_sm : 1);
     sm_counts[dev] = sms;
@@ -1683,48 +1484,36 @@ static int32_t read_tuning(const char* who, const hp_tuning* tuning, Tune& t) {
 
 static constexpr size_t align256s(size_t x) { return (x + 255) & ~(size_t)255; }
 
-struct SchedLayout {
-  size_t work, item, cols, order, view, small, pts, total;
+struct ListLayout {
+  size_t counts, rays, pts, total;
 };
 
-// up to items_per_tile items per tile (every row its own item, in quarters)
-static SchedLayout sched_layout(int64_t H, int64_t W, int64_t n_sorted) {
-  const size_t per = align256s(sizeof(int) * (size_t)max_view_items(H, W));
-  SchedLayout L;
-  L.work = 0;
-  L.item = per;
-  L.cols = 2 * per;
-  L.order = 3 * per;
-  L.view = 0;  // single view: none
-  L.small = 4 * per;
-  L.pts = L.small + 512;  // counts[32], fill[32], next, n_items
+static ListLayout list_layout(int64_t H, int64_t W, int64_t n_sorted) {
+  ListLayout L;
+  L.counts = 0;
+  L.rays = 256;
+  L.pts = L.rays + align256s(sizeof(int4) * (size_t)max_view_entries(H, W));
   L.total = L.pts + align256s(sizeof(float4) * (size_t)n_sorted);
   return L;
 }
 
-// Batched launch: the queue over all views' tiles, then the per-view
-// arguments, the views' first tiles and room for a copy of the view table.
+// Batched launch: the list over all views' rays with each unit's view, then the
+// per-view arguments, the views' first tiles and room for a copy of the view table.
 struct BatchLayout {
-  SchedLayout q;
-  size_t args, tile_base, pack_base, views, buckets, pts, total;
+  size_t counts, rays, front_view, back_view, args, tile_base, pack_base, views, pts, total;
 };
 
-static BatchLayout batch_layout(int64_t total_items, int n_views, int64_t total_slots) {
+static BatchLayout batch_layout(int64_t entries, int n_views, int64_t total_slots) {
   BatchLayout B;
-  const size_t per = align256s(sizeof(int) * (size_t)total_items);
-  B.q.work = 0;
-  B.q.item = per;
-  B.q.cols = 2 * per;
-  B.q.order = 3 * per;
-  B.q.view = 4 * per;
-  B.q.small = 5 * per;
-  B.q.total = B.q.small + 512;  // next, n_items (counts and fill live in `buckets`)
-  B.args = B.q.total;
+  B.counts = 0;
+  B.rays = 256;
+  B.front_view = B.rays + align256s(sizeof(int4) * (size_t)entries);
+  B.back_view = B.front_view + align256s(sizeof(int) * (size_t)(entries / 4 + 1));
+  B.args = B.back_view + align256s(sizeof(int) * (size_t)entries);
   B.tile_base = B.args + align256s(sizeof(SampleArgs) * (size_t)n_views);
   B.pack_base = B.tile_base + align256s(sizeof(int) * (size_t)(n_views + 1));
   B.views = B.pack_base + align256s(sizeof(int) * (size_t)(n_views + 1));
-  B.buckets = B.views + align256s(sizeof(hp_view) * (size_t)n_views);  // counts, fill, base: n_views * 32 each
-  B.pts = B.buckets + 3 * align256s(sizeof(int) * 32 * (size_t)n_views);
+  B.pts = B.views + align256s(sizeof(hp_view) * (size_t)n_views);
   B.total = B.pts + sizeof(float4) * (size_t)total_slots;
   return B;
 }
@@ -1768,7 +1557,7 @@ using namespace hp;
 
 extern "C" size_t hp_quick_sampling_workspace_size(int64_t n_sorted, int32_t height, int32_t width) {
   if (height <= 0 || width <= 0 || n_sorted < 0) return 0;
-  return sched_layout(height, width, n_sorted).total;
+  return list_layout(height, width, n_sorted).total;
 }
 
 // Argument checks shared by the per-view and batched entry points.
@@ -1811,7 +1600,7 @@ extern "C" int32_t hp_stage_config_info(int32_t config, int32_t* tile_h, int32_t
   const SamplingKernels& K = stage_kernels(config);
   if (tile_h) *tile_h = K.tile_h;
   if (tile_w) *tile_w = K.tile_w;
-  if (stage_points) *stage_points = K.cap;
+  if (stage_points) *stage_points = K.stage;
   if (blocks_per_sm) *blocks_per_sm = K.blocks;
   return HP_OK;
 }
@@ -1826,7 +1615,7 @@ extern "C" int32_t hp_quick_sampling_tuned(const float* xyz, int64_t n_points, c
     return rc;
   Tune tn;
   if (int32_t rc = read_tuning("hp_quick_sampling", tuning, tn)) return rc;
-  const SchedLayout L = sched_layout(cam->height, cam->width, n_sorted);
+  const ListLayout L = list_layout(cam->height, cam->width, n_sorted);
   if (!workspace || workspace_bytes < L.total || ((uintptr_t)workspace & 255) != 0)
     return set_error(HP_ERR_WORKSPACE, "hp_quick_sampling: workspace needs %zu bytes, 256-byte aligned (got %zu)",
                      L.total, workspace_bytes);
@@ -1843,7 +1632,7 @@ extern "C" int32_t hp_quick_sampling_tuned(const float* xyz, int64_t n_points, c
   a.pc_idx = pc_idx;
   a.sp_t = sp_t;
   a.mask = mask;
-  a.heavy = tn.heavy;
+  derive_args(a);
   int blocks = 0, sms = 0;
   if (int32_t rc = sampling_grid(tn.config, &blocks, &sms)) return rc;
   if (tn.per_sm > 0 && tn.per_sm * sms < blocks) blocks = tn.per_sm * sms;
@@ -1851,28 +1640,20 @@ extern "C" int32_t hp_quick_sampling_tuned(const float* xyz, int64_t n_points, c
   const int tiles_x = (cam->width + K.tile_w - 1) / K.tile_w;
   const int ntiles = (int)tiles_of(cam->height, cam->width, K.tile_h, K.tile_w);
   char* ws = (char*)workspace;
-  Sched sc;
-  sc.work = (int*)(ws + L.work);
-  sc.item = (int*)(ws + L.item);
-  sc.cols = (int*)(ws + L.cols);
-  sc.order = (int*)(ws + L.order);
-  sc.view = nullptr;
-  sc.counts = (int*)(ws + L.small);
-  sc.fill = sc.counts + 32;
-  sc.next = sc.counts + 64;
-  sc.n_items = sc.counts + 65;
+  RayList rl;
+  rl.rays = (int4*)(ws + L.rays);
+  rl.cap = max_view_entries(cam->height, cam->width);
+  rl.counts = (unsigned*)(ws + L.counts);
+  rl.front_view = rl.back_view = nullptr;
+  rl.light = tn.heavy < K.entries / 4 ? tn.heavy : K.entries / 4;
   cudaStream_t st = (cudaStream_t)stream;
-  if (cudaMemsetAsync(sc.counts, 0, 512, st) != cudaSuccess)
+  if (cudaMemsetAsync(rl.counts, 0, 4 * sizeof(unsigned), st) != cudaSuccess)
     return set_error(HP_ERR_CUDA, "hp_quick_sampling: cudaMemsetAsync failed");
-  K.tile_work<<<(ntiles + 7) / 8, 256, 0, st>>>(a.hash, a.n_sorted, cam->height, cam->width, opt->kernel_size, tiles_x,
-                                                 ntiles, K.cap, sc, sorted_point_idx, xyz, (int)n_points,
-                                                 (float4*)(ws + L.pts));
-  if (int32_t rc = check_launch("k_tile_work")) return rc;
-  k_tile_order<<<(ntiles + 255) / 256 < 148 ? (ntiles + 255) / 256 : 148, 256, 0, st>>>(sc);
-  if (int32_t rc = check_launch("k_tile_order")) return rc;
-  // a split tile yields up to items_per_tile items: size the persistent grid by those, not by tiles
-  const int64_t max_items = (int64_t)ntiles * K.items_per_tile;
-  K.view<<<blocks < max_items ? blocks : (int)max_items, K.threads, K.smem, st>>>(a, sc, tiles_x);
+  K.list<<<ntiles, kThreads, 0, st>>>(a, rl, tiles_x, ntiles);
+  if (int32_t rc = check_launch("k_ray_list")) return rc;
+  // at least a unit of four rays a warp
+  const int64_t most = (int64_t)ntiles * (kThreads / 4 / kServeWarps);
+  K.view<<<blocks < most ? blocks : (int)most, kServeThreads, K.smem, st>>>(a, rl);
   return check_launch("k_quick_sampling");
 }
 
@@ -1897,22 +1678,18 @@ static int64_t batch_tiles(const hp_view* views, int32_t n_views, int tile_h, in
   return total;
 }
 
-// Schedule entries a batch can need under any configuration.
-static int64_t batch_max_items(const hp_view* views, int32_t n_views) {
-  int64_t m = 0;
-  for (int c = 1; c <= kStageConfigs; c++) {
-    const SamplingKernels& K = stage_kernels(c);
-    const int64_t items = batch_tiles(views, n_views, K.tile_h, K.tile_w) * K.items_per_tile;
-    if (items > m) m = items;
-  }
-  return m;
+// Ray-list entries a batch can need under any configuration.
+static int64_t batch_entries(const hp_view* views, int32_t n_views) {
+  int64_t total = 0;
+  for (int32_t v = 0; v < n_views; v++) total += max_view_entries(views[v].cam.height, views[v].cam.width);
+  return total;
 }
 
 extern "C" size_t hp_quick_sampling_batch_workspace_size(const hp_view* views, int32_t n_views) {
   if (!views || n_views <= 0) return 0;
   for (int32_t v = 0; v < n_views; v++)
     if (views[v].cam.width <= 0 || views[v].cam.height <= 0 || views[v].n_sorted < 0) return 0;
-  return batch_layout(batch_max_items(views, n_views), n_views, batch_slots(views, n_views)).total;
+  return batch_layout(batch_entries(views, n_views), n_views, batch_slots(views, n_views)).total;
 }
 
 extern "C" int32_t hp_quick_sampling_batch(const hp_view* views, const hp_view* views_device, int32_t n_views,
@@ -1931,11 +1708,11 @@ extern "C" int32_t hp_quick_sampling_batch(const hp_view* views, const hp_view* 
       return set_error(rc, "%s (view %d)", msg, v);
     }
   }
-  const int64_t max_items = batch_max_items(views, n_views);
+  const int64_t entries = batch_entries(views, n_views);
   const int64_t total_slots = batch_slots(views, n_views);
-  if (max_items >= (1ll << 31) || total_slots >= (1ll << 31))
+  if (entries >= (1ll << 32) || total_slots >= (1ll << 31))
     return set_error(HP_ERR_INVALID_ARGUMENT, "%s: too many tiles or points in one batch", who);
-  const BatchLayout B = batch_layout(max_items, n_views, total_slots);
+  const BatchLayout B = batch_layout(entries, n_views, total_slots);
   if (!workspace || workspace_bytes < B.total || ((uintptr_t)workspace & 255) != 0)
     return set_error(HP_ERR_WORKSPACE, "%s: workspace needs %zu bytes, 256-byte aligned (got %zu)", who, B.total,
                      workspace_bytes);
@@ -1952,40 +1729,29 @@ extern "C" int32_t hp_quick_sampling_batch(const hp_view* views, const hp_view* 
       return set_error(HP_ERR_CUDA, "%s: copying the view table failed", who);
     views_device = (const hp_view*)(ws + B.views);
   }
-  Sched sc;
-  sc.work = (int*)(ws + B.q.work);
-  sc.item = (int*)(ws + B.q.item);
-  sc.cols = (int*)(ws + B.q.cols);
-  sc.order = (int*)(ws + B.q.order);
-  sc.view = (int*)(ws + B.q.view);
-  const size_t bucket_bytes = align256s(sizeof(int) * 32 * (size_t)n_views);
-  sc.counts = (int*)(ws + B.buckets);
-  sc.fill = (int*)(ws + B.buckets + bucket_bytes);
-  int* base = (int*)(ws + B.buckets + 2 * bucket_bytes);
-  sc.next = (int*)(ws + B.q.small);
-  sc.n_items = sc.next + 1;
+  RayList rl;
+  rl.rays = (int4*)(ws + B.rays);
+  rl.cap = entries;
+  rl.counts = (unsigned*)(ws + B.counts);
+  rl.front_view = (int*)(ws + B.front_view);
+  rl.back_view = (int*)(ws + B.back_view);
+  rl.light = tn.heavy < K.entries / 4 ? tn.heavy : K.entries / 4;
   SampleArgs* args = (SampleArgs*)(ws + B.args);
   int* tile_base = (int*)(ws + B.tile_base);
-  if (cudaMemsetAsync(ws + B.q.small, 0, 512, st) != cudaSuccess ||
-      cudaMemsetAsync(ws + B.buckets, 0, 2 * bucket_bytes, st) != cudaSuccess)
-    return set_error(HP_ERR_CUDA, "%s: memset failed", who);
   int* pack_base = (int*)(ws + B.pack_base);
-  k_batch_setup<<<1, 32, 0, st>>>(views_device, n_views, tn.heavy, K.tile_h, K.tile_w, args, tile_base, pack_base,
+  if (cudaMemsetAsync(rl.counts, 0, 4 * sizeof(unsigned), st) != cudaSuccess)
+    return set_error(HP_ERR_CUDA, "%s: memset failed", who);
+  k_batch_setup<<<1, 32, 0, st>>>(views_device, n_views, K.tile_h, K.tile_w, args, tile_base, pack_base,
                                   (float4*)(ws + B.pts));
   if (int32_t rc = check_launch("k_batch_setup")) return rc;
   if (total_slots > 0) {
     k_batch_pack<<<(unsigned)((total_slots + 255) / 256), 256, 0, st>>>(args, pack_base, n_views, (int)total_slots);
     if (int32_t rc = check_launch("k_batch_pack")) return rc;
   }
-  const int nt = (int)total_tiles;
-  K.batch_tile_work<<<(nt + 7) / 8, 256, 0, st>>>(args, tile_base, n_views, nt, K.cap, sc);
-  if (int32_t rc = check_launch("k_batch_tile_work")) return rc;
-  k_batch_order_scan<<<1, 1024, 0, st>>>(sc, n_views, base);
-  if (int32_t rc = check_launch("k_batch_order_scan")) return rc;
-  k_batch_order_place<<<(nt + 255) / 256 < 148 ? (nt + 255) / 256 : 148, 256, 0, st>>>(sc, base);
-  if (int32_t rc = check_launch("k_batch_order_place")) return rc;
-  const int64_t grid_items = (int64_t)nt * K.items_per_tile;
-  K.batch<<<blocks < grid_items ? blocks : (int)grid_items, K.threads, K.smem, st>>>(args, sc);
+  K.batch_list<<<(unsigned)total_tiles, kThreads, 0, st>>>(args, tile_base, n_views, rl);
+  if (int32_t rc = check_launch("k_batch_ray_list")) return rc;
+  const int64_t most = total_tiles * (kThreads / 4 / kServeWarps);
+  K.batch<<<blocks < most ? blocks : (int)most, kServeThreads, K.smem, st>>>(args, rl);
   return check_launch("k_quick_sampling_batch");
 }
 

@@ -244,31 +244,32 @@ HP_API int32_t hp_aggregator_forward(const void* packed, const float* pc_xyz, co
 HP_API int32_t hp_aggregator_status(const void* workspace, int64_t n_samples, hp_stream_t stream);
 
 /* Scratch bytes hp_quick_sampling needs for n_sorted ids and an image of this
- * size (its tile schedule and the ids' points packed as 16-byte records);
+ * size (its list of rays and the ids' points packed as 16-byte records);
  * workspace must be 256-byte aligned. */
 HP_API size_t hp_quick_sampling_workspace_size(int64_t n_sorted, int32_t height, int32_t width);
 
 /* Launch tuning of hp_quick_sampling_tuned and hp_quick_sampling_batch (NULL
  * or 0 fields = defaults).  Outputs never depend on it.
  *   heavy_window   rays whose window holds more candidates are served by a
- *                  whole warp instead of one thread (0..4096; default 320).
+ *                  whole warp instead of 8 lanes (0..4096; default 320, and at
+ *                  most what 8 lanes hold on chip: stage_points / 16).
  *   blocks_per_sm  resident blocks of the persistent sampling kernel per SM
  *                  (default: as many as fit).
- *   stage_config   stage and tile of the sampling kernel (0 = 4):
- *                  1: 2560 staged points per tile, 4 blocks per SM, 8 x 32 tiles;
- *                  2: 3712 points, 3 blocks per SM, 8 x 32;
- *                  3: 5888 points, 2 blocks per SM, 8 x 32;
- *                  4: 2560 points, 4 blocks per SM, 16 x 16 tiles;
- *                  5: 3712 points, 3 blocks per SM, 16 x 16.
- *                  Tiles whose window halo holds more points are split into
- *                  row bands and column ranges, or read from global memory. */
+ *   stage_config   candidates a block holds on chip, resident blocks, and the
+ *                  tile whose rays are ordered together (0 = 4):
+ *                  1: 3840 listed candidates, 8 blocks per SM, 8 x 32 tiles;
+ *                  2: 3968, 6 blocks per SM, 8 x 32;
+ *                  3: 4096, 5 blocks per SM, 8 x 32;
+ *                  4: 3840, 8 blocks per SM, 16 x 16 tiles;
+ *                  5: 3968, 6 blocks per SM, 16 x 16.
+ *                  A ray with more takes the general walk (same outputs). */
 typedef struct hp_tuning {
   int32_t heavy_window;
   int32_t blocks_per_sm;
   int32_t stage_config;
 } hp_tuning;
 
-/* The tile (tile_h x tile_w pixels), staged points per tile and resident
+/* The tile (tile_h x tile_w pixels), listed candidates per block and resident
  * blocks per SM of a stage configuration (0 reads as 4); any output pointer
  * may be NULL.  HP_ERR_INVALID_ARGUMENT outside 0..5.  No counterpart in the
  * reference. */

@@ -1,0 +1,79 @@
+"""The sampling kernel's paths against one another, bit for bit.
+
+A ray is served by 8 lanes, by a whole warp, or -- where its window's buckets
+do not follow one another in the sorted ids, its list overflows or a decision
+is too close for the fast arithmetic -- by the general walk.  Storing the same
+buckets in reversed pixel order sends every ray with two non-empty cells in a
+window row to the general walk, so each scene is sampled with both tables and
+with heavy windows from "every ray" to "none".
+"""
+import numpy as np
+import pytest
+import torch
+
+from hashpoint import native, ops, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _reversed_buckets(sidx, table):
+    """The same buckets, stored last pixel first."""
+    sidx, h = sidx.cpu().numpy(), table.cpu().numpy().copy()
+    out, at = np.full_like(sidx, -1), 0
+    for p in np.nonzero(h[:, 1] > 0)[0][::-1]:
+        s, c = h[p]
+        out[at:at + c] = sidx[s:s + c]
+        h[p, 0] = at
+        at += c
+    return torch.from_numpy(out).cuda(), torch.from_numpy(h).cuda()
+
+
+def _scene(kind, n, W, H, rng):
+    if kind == "plane":  # a tilted plane and a parallel one behind it: many bins, several samples a ray
+        u, v = rng.uniform(-1.2, 1.2, n), rng.uniform(-1.0, 1.0, n)
+        z = 0.8 * u + 0.15 * rng.integers(0, 3, n)
+        xyz = np.stack([u, v, z], 1).astype(np.float32)
+    elif kind == "twins":  # every point three times: equal distances everywhere
+        xyz = synth.sphere_cloud(rng, n // 3)
+        xyz = np.concatenate([xyz, xyz, xyz])[rng.permutation(3 * len(xyz))]
+    elif kind == "pile":  # buckets far above 48 entries
+        xyz = synth.sphere_cloud(rng, n, noise=0.05) * 0.3
+    else:
+        xyz = synth.shapes_cloud(rng, n)
+    cam = synth.look_at_camera((0.3, 0.2, 4.0), (0, 0, 0), W, H, 0.9 * W)
+    return xyz.astype(np.float32), cam
+
+
+@pytest.mark.parametrize("kind,n,W,H,opt", [
+    ("plane", 30_000, 97, 61, dict(kernel_size=5, radius_threshold=0.05)),
+    # slow transmittance: up to S samples a ray, odd S and P
+    ("plane", 30_000, 97, 61, dict(kernel_size=4, radius_threshold=0.05, sdf2weight_gaussian_gamma=0.05,
+                                   num_sample_points_per_ray=7, num_point_cloud_per_sp=3)),
+    ("plane", 9_000, 40, 33, dict(kernel_size=3, radius_threshold=0.1, sdf2weight_gaussian_gamma=0.2, t_intvl=0.003,
+                                  num_sample_points_per_ray=5, num_point_cloud_per_sp=12)),
+    # mean distances that the quantised sums cannot tell apart, and ones they can
+    ("plane", 9_000, 40, 33, dict(kernel_size=3, radius_threshold=0.1, sdf2weight_gaussian_alpha=0.0005)),
+    ("plane", 9_000, 40, 33, dict(kernel_size=3, radius_threshold=0.1, sdf2weight_gaussian_alpha=0.02)),
+    ("twins", 20_000, 65, 49, dict(kernel_size=5, radius_threshold=0.04, num_point_cloud_per_sp=8)),
+    ("pile", 60_000, 40, 31, dict(kernel_size=5, radius_threshold=0.03, num_point_cloud_per_sp=8)),
+    ("pile", 60_000, 33, 16, dict(kernel_size=2, radius_threshold=0.5, num_point_cloud_per_sp=8)),
+    ("shapes", 40_000, 160, 120, dict(kernel_size=1, radius_threshold=0.02, num_point_cloud_per_sp=4)),
+    ("shapes", 3, 5, 1, dict(kernel_size=5, radius_threshold=2.0, num_point_cloud_per_sp=1)),
+])
+def test_paths_agree(kind, n, W, H, opt):
+    native.build()
+    xyz, cam = _scene(kind, n, W, H, np.random.default_rng(n + W))
+    o = synth.Options(**{"num_point_cloud_per_sp": 8, **opt})
+    X, c2w, w2c, K = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (xyz, cam.c2w, cam.w2c, cam.K)]
+    sidx, _, table = ops.pts2plane(X, w2c, K, H, W)
+
+    def run(ids, h, **tuning):
+        out = ops.quick_sampling(X, c2w, cam.fx, cam.fy, cam.cx, cam.cy, W, H, o, ids, h,
+                                 tuning=ops.make_tuning(**tuning))
+        return [t.cpu().numpy().view(np.uint8) for t in out]
+
+    want = run(*_reversed_buckets(sidx, table))
+    for heavy in (0, 1, 40, 4096):
+        for stage in (3, 4):
+            for a, b in zip(run(sidx, table, heavy_window=heavy, stage_config=stage), want):
+                assert np.array_equal(a, b), (heavy, stage)
