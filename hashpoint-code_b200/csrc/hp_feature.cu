@@ -344,18 +344,55 @@ __global__ void __launch_bounds__(256) k_feature_query_vec(FeatArgs a) {
 }
 
 // clamp_t: gaps outside (1e-8, 2 vsize], and the last sample's, become vsize.
-__device__ __forceinline__ float clamped_gap(const float* t, int s, int S, float vsize) {
-  const float d = s + 1 < S ? __fsub_rn(t[s + 1], t[s]) : vsize;
+__device__ __forceinline__ float clamp_gap(float d, float vsize) {
   const float m = (d < 1e-8f || d > __fmul_rn(2.0f, vsize)) ? 1.0f : 0.0f;
   return __fadd_rn(__fmul_rn(d, __fsub_rn(1.0f, m)), __fmul_rn(m, vsize));
 }
 
-// one thread per (ray, sample): consecutive threads read and write consecutive elements
-__global__ void k_clamp_t(const float* __restrict__ t_val, int64_t rays, int S, float vsize, float* __restrict__ out) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rays * S) return;
-  const int s = i < 0x7fffffff ? (int)((unsigned)i % (unsigned)S) : (int)(i % S);
-  out[i] = clamped_gap(t_val + (i - s), s, S, vsize);
+__device__ __forceinline__ float clamped_gap(const float* t, int s, int S, float vsize) {
+  return clamp_gap(s + 1 < S ? __fsub_rn(t[s + 1], t[s]) : vsize, vsize);
+}
+
+// Four consecutive elements per thread, whatever S: one 16-byte load (the
+// element after them comes from the next lane, lane 31 loads its own) and one
+// 16-byte store.  Unaligned arrays (kVec 0) go one by one, 256 apart.  Bound by
+// HBM.
+template <int kVec>
+__global__ void __launch_bounds__(256) k_clamp_t(const float* __restrict__ t_val, int64_t n, int S, float vsize,
+                                                 float* __restrict__ out) {
+  const int64_t block0 = (int64_t)blockIdx.x * 1024;
+  const int64_t i = block0 + (kVec ? threadIdx.x * 4 : threadIdx.x);
+  auto slot = [&](int64_t e) { return e < 0x7fffffff ? (int)((unsigned)e % (unsigned)S) : (int)(e % S); };
+  if constexpr (kVec) {
+    const bool whole = i + 4 <= n;
+    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (whole) t = *reinterpret_cast<const float4*>(t_val + i);
+    float next = __shfl_down_sync(0xffffffffu, t.x, 1);
+    const bool next_whole = __shfl_down_sync(0xffffffffu, whole, 1);
+    if (i >= n) return;
+    int s = slot(i);
+    if (whole) {
+      if (((threadIdx.x & 31) == 31 || !next_whole) && i + 4 < n) next = t_val[i + 4];
+      const float v[5] = {t.x, t.y, t.z, t.w, next};
+      float g[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        g[q] = clamp_gap(s + 1 < S ? __fsub_rn(v[q + 1], v[q]) : vsize, vsize);
+        s = s + 1 < S ? s + 1 : 0;
+      }
+      *reinterpret_cast<float4*>(out + i) = make_float4(g[0], g[1], g[2], g[3]);
+    } else {
+      for (int64_t e = i; e < n; e++) {
+        out[e] = clamped_gap(t_val + (e - s), s, S, vsize);
+        s = s + 1 < S ? s + 1 : 0;
+      }
+    }
+  } else {
+    for (int64_t e = i; e < n && e < block0 + 1024; e += 256) {
+      const int s = slot(e);
+      out[e] = clamped_gap(t_val + (e - s), s, S, vsize);
+    }
+  }
 }
 
 // render (with the deltas given, or derived from t_val by clamp_t when deltas is null)
@@ -529,7 +566,11 @@ extern "C" int32_t hp_clamp_t(const float* t_val, int64_t n_rays, int32_t S, flo
     return set_error(HP_ERR_INVALID_ARGUMENT, "hp_clamp_t: sizes out of range");
   if (n_rays == 0) return HP_OK;
   if (!t_val || !t_dist) return set_error(HP_ERR_INVALID_ARGUMENT, "hp_clamp_t: null pointer");
-  k_clamp_t<<<(unsigned)((n_rays * S + 255) / 256), 256, 0, (cudaStream_t)stream>>>(t_val, n_rays, S, vsize, t_dist);
+  const unsigned blocks = (unsigned)((n_rays * S + 1023) / 1024);
+  if ((((uintptr_t)t_val | (uintptr_t)t_dist) & 15) == 0)
+    k_clamp_t<1><<<blocks, 256, 0, (cudaStream_t)stream>>>(t_val, n_rays * S, S, vsize, t_dist);
+  else
+    k_clamp_t<0><<<blocks, 256, 0, (cudaStream_t)stream>>>(t_val, n_rays * S, S, vsize, t_dist);
   return check_launch("k_clamp_t");
 }
 
