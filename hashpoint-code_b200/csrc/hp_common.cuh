@@ -10,6 +10,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 
 #include "../../include/hashpoint_b200.h"
@@ -107,6 +108,66 @@ __device__ __forceinline__ void window_cell(int v, int u, int k, int H, int W, i
 __device__ __forceinline__ float4 load_point(const float* __restrict__ xyz, int id) {
   const float* p = xyz + 3 * (size_t)id;
   return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), 0.f);
+}
+
+// The reference keeps a candidate when norm3df(e) < radius (e = point minus its
+// projection on the ray).  The squared length e2 (three roundings) decides it
+// without the square root whenever e2 is outside a band of relative width
+// 2^-16 around radius^2 -- far wider than the few-ulp errors of e2 and
+// norm3df -- and norm3df decides inside the band, so the result is identical.
+struct RadiusTest {
+  float r, lo2, hi2;
+  bool fast;  // else the band is everything
+};
+
+__host__ __device__ inline RadiusTest make_radius_test(float r) {
+  RadiusTest rt;
+  rt.r = r;
+  const double r2 = (double)r * (double)r;
+  rt.fast = r2 > 1e-30 && r2 < 1e30;
+  rt.lo2 = rt.fast ? (float)(r2 * (1.0 - 1.0 / 65536.0)) : -1.0f;
+  rt.hi2 = rt.fast ? (float)(r2 * (1.0 + 1.0 / 65536.0)) : INFINITY;
+  return rt;
+}
+
+// q: the squared length of (e0, e1, e2).
+__device__ __forceinline__ float squared(float e0, float e1, float e2) {
+  return __fmaf_rn(e2, e2, __fmaf_rn(e1, e1, __fmul_rn(e0, e0)));
+}
+
+// For all lanes of the warp; the band is taken by a branch of the whole warp.
+__device__ __forceinline__ bool within_radius(const RadiusTest& rt, bool in, float q, float e0, float e1, float e2) {
+  bool kept = in && q < rt.lo2;
+  const bool band = in && !(q < rt.lo2) && !(q > rt.hi2);
+  if (__any_sync(0xffffffffu, band)) {
+    const float n = norm3df(e0, e1, e2);
+    if (band) kept = n < rt.r;
+  }
+  return kept;
+}
+
+// PointRayInterset's t (cuda_util.cuh:227): the correctly rounded quotient of
+// (p - o).d and d.d, with inv_dd = RN(1 / d.d): a first quotient, its exact
+// residual and one fused step (Markstein 1990).  d is normalised, so d.d is a
+// few ulp from 1; for every d.d within 64 ulp of 1 and every numerator mantissa
+// this equals the division, at 3 instructions for 10 and without its branch.
+__device__ __forceinline__ float ray_t(const Ray& r, float inv_dd, const float4& p) {
+  const float num = dot3(__fsub_rn(p.x, r.o[0]), __fsub_rn(p.y, r.o[1]), __fsub_rn(p.z, r.o[2]), r.d[0], r.d[1], r.d[2]);
+  const float q = __fmul_rn(num, inv_dd);
+  return __fmaf_rn(__fmaf_rn(-q, r.dd, num), inv_dd, q);
+}
+
+// Clipped bucket range of a hash entry: [x, x + count) within [0, n_sorted).
+__device__ __forceinline__ int2 bucket_range(int2 h, int n_sorted) {
+  if (h.x < 0 || h.y <= 0 || h.x >= n_sorted) return make_int2(0, 0);
+  return make_int2(h.x, h.x + min(h.y, n_sorted - h.x));
+}
+
+// Lanes [lo, hi) of a warp as a bit mask (0 <= lo <= hi <= 32).
+__device__ __forceinline__ unsigned lane_span(int lo, int hi) {
+  const unsigned below_hi = hi >= 32 ? 0xffffffffu : (1u << hi) - 1u;
+  const unsigned below_lo = lo >= 32 ? 0xffffffffu : (1u << lo) - 1u;
+  return below_hi & ~below_lo;
 }
 
 }  // namespace hp

@@ -5,10 +5,11 @@
 // gives each window cell a lane that gathers up to 32 ids within the ray
 // radius and then reserves output slots with atomicAdd, so the order of a
 // row -- and which ids survive when the row overflows -- depends on atomic
-// timing.  Here one warp serves one ray: lanes count their cell's ids, a warp
-// prefix sum assigns each cell its offset in window-cell order, and a second
-// pass writes the ids, so rows are deterministic (window-cell order, bucket
-// order) and an overflowing row keeps its first num_point_per_ray ids.
+// timing.  Here a warp serves one ray at a time with its lanes over the
+// candidates: 32 window cells at a time, their buckets concatenated, a
+// candidate's place in the row from a ballot.  Rows are deterministic
+// (window-cell order, bucket order) and an overflowing row keeps its first
+// num_point_per_ray ids.
 //
 // hp_scatter replaces _C.scatter (epcq/csrc/rasterization.cu:88-128, kernel
 // :36-86): per pixel the `bins` nearest points by depth, sorted ascending.
@@ -21,69 +22,111 @@ DevCamera dev_camera(const hp_camera* cam);
 DevOptions dev_options(const hp_options* o);
 
 constexpr int kQueryWarps = 4;
+constexpr int kQueryRays = 8;  // rays a warp serves in turn, their directions computed side by side
 
+// Bound by the latency of the dependent loads (bucket, id, point) and the
+// instructions of each ray's set-up; the rows themselves are 67 MB for 65,536
+// rays of 256 (10 us).  65,536 rays of a 1M-point view at 800 x 800, 5 x 5
+// window: 72 us (ncu, cold; the call 126 -> 68 us); a lane per cell left a warp
+// waiting for its longest bucket, twice, with a division and a norm a
+// candidate: 179 us.  2, 4 or 8 rays a warp are level.
 __global__ void __launch_bounds__(kQueryWarps * 32) k_quick_query(const float* __restrict__ xyz, int n_points,
                                                                   const int* __restrict__ sidx, int n_sorted,
                                                                   const int2* __restrict__ hash, DevCamera cam,
-                                                                  DevOptions opt, const int* __restrict__ ray_ids,
-                                                                  int n_rays, int* __restrict__ out) {
+                                                                  DevOptions opt, RadiusTest rt,
+                                                                  const int* __restrict__ ray_ids, int n_rays,
+                                                                  int* __restrict__ out) {
+  constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  const int i = blockIdx.x * kQueryWarps + (threadIdx.x >> 5);
-  if (i >= n_rays) return;
-  const int cap = opt.num_point_per_ray;
-  int* row = out + (size_t)i * cap;
-  const int W = cam.width, H = cam.height;
-  const int ray = ray_ids[i];
-  int written = 0;
-  if (0 <= ray && ray < W * H) {
-    const int u = ray % W, v = ray / W;
+  const unsigned below = (1u << lane) - 1u;
+  const int64_t r0 = ((int64_t)blockIdx.x * kQueryWarps + (threadIdx.x >> 5)) * kQueryRays;
+  if (r0 >= n_rays) return;
+  const int cap = opt.num_point_per_ray, k = opt.k, k2 = k * k, W = cam.width, H = cam.height;
+  int my_ray = -1;
+  Ray mine{};
+  if (lane < kQueryRays && r0 + lane < n_rays) {
+    my_ray = __ldg(ray_ids + r0 + lane);
+    if (my_ray < 0 || my_ray >= W * H) my_ray = -1;
+    if (my_ray >= 0) make_ray(cam.c2w, cam.fx, cam.fy, cam.cx, cam.cy, my_ray % W, my_ray / W, mine);
+  }
+  // clipped bucket of cell c0 + lane of a ray's window
+  auto bucket = [&](int ray, int c0) -> int2 {
+    const int l = c0 + lane;
+    if (ray < 0 || l >= k2) return make_int2(0, 0);
+    int vv, uu;
+    window_cell(ray / W, ray % W, k, H, W, l, vv, uu);
+    return bucket_range(__ldg(hash + (size_t)vv * W + uu), n_sorted);
+  };
+  const int rays = (int)(n_rays - r0 < kQueryRays ? n_rays - r0 : kQueryRays);
+  int2 ahead = bucket(__shfl_sync(kAll, my_ray, 0), 0);
+  for (int q = 0; q < rays; q++) {
+    const int ray = __shfl_sync(kAll, my_ray, q);
     Ray r;
-    make_ray(cam.c2w, cam.fx, cam.fy, cam.cx, cam.cy, u, v, r);
-    const int k2 = opt.k * opt.k;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      r.o[i] = __shfl_sync(kAll, mine.o[i], q);
+      r.d[i] = __shfl_sync(kAll, mine.d[i], q);
+    }
+    r.dd = __shfl_sync(kAll, mine.dd, q);
+    const float inv_dd = __frcp_rn(r.dd);
+    int2 rg = ahead;
+    if (q + 1 < rays) ahead = bucket(__shfl_sync(kAll, my_ray, q + 1), 0);
+    int* row = out + (r0 + q) * cap;
     int base = 0;
-    for (int c0 = 0; c0 < k2 && base < cap; c0 += 32) {
-      const int l = c0 + lane;
-      int2 h = make_int2(0, -1);
-      if (l < k2) {
-        int vv, uu;
-        window_cell(v, u, opt.k, H, W, l, vv, uu);
-        h = __ldg(hash + (size_t)vv * W + uu);
-        if (h.x < 0) h.y = -1;
-        h.y = min(h.y, n_sorted - h.x);  // clip the range to the id list
-      }
-      // count this cell's ids (<= 32)
-      int cnt = 0;
-      for (int j = h.x; j < h.x + h.y && cnt < kQueryPerCell; j++) {
-        const int id = __ldg(sidx + j);
-        if ((unsigned)id >= (unsigned)n_points) continue;
-        const float4 p = load_point(xyz, id);
-        float t, dist;
-        intersect(r, p.x, p.y, p.z, t, dist);
-        if (dist < opt.radius) cnt++;
-      }
-      int incl = cnt;
+    for (int c0 = 0; c0 < k2 && base < cap && ray >= 0; c0 += 32) {
+      if (c0 > 0) rg = bucket(ray, c0);
+      const int cnt = rg.y - rg.x;
+      int pre = cnt;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
+        const int t = __shfl_up_sync(kAll, pre, o);
+        if (lane >= o) pre += t;
       }
-      int pos = base + incl - cnt;
-      for (int j = h.x, c = 0; j < h.x + h.y && c < cnt && pos < cap; j++) {
-        const int id = __ldg(sidx + j);
-        if ((unsigned)id >= (unsigned)n_points) continue;
-        const float4 p = load_point(xyz, id);
-        float t, dist;
-        intersect(r, p.x, p.y, p.z, t, dist);
-        if (dist < opt.radius) {
-          row[pos++] = id;
-          c++;
+      const int total = __shfl_sync(kAll, pre, 31);
+      pre -= cnt;
+      const bool deep = __any_sync(kAll, cnt > kQueryPerCell);
+      int carry = 0;  // lane c's copy: cell c's ids of earlier chunks
+      for (int j0 = 0; j0 < total && base < cap; j0 += 32) {
+        const int j = j0 + lane;
+        int c = 0;
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1)
+          if (__shfl_sync(kAll, pre, c + s) <= j) c += s;
+        const int first = __shfl_sync(kAll, pre, c);
+        const int at = __shfl_sync(kAll, rg.x, c) + (j - first);
+        int id = -1;
+        float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (j < total) {
+          id = __ldg(sidx + at);
+          if ((unsigned)id < (unsigned)n_points) p = load_point(xyz, id);
+          else id = -1;
         }
+        const float t = ray_t(r, inv_dd, p);
+        const float e0 = __fsub_rn(p.x, __fmaf_rn(t, r.d[0], r.o[0]));
+        const float e1 = __fsub_rn(p.y, __fmaf_rn(t, r.d[1], r.o[1]));
+        const float e2 = __fsub_rn(p.z, __fmaf_rn(t, r.d[2], r.o[2]));
+        bool in = within_radius(rt, id >= 0, squared(e0, e1, e2), e0, e1, e2);
+        unsigned m = __ballot_sync(kAll, in);
+        if (deep) {  // only a cell's first kQueryPerCell
+          const int before = __shfl_sync(kAll, carry, c) + __popc(m & below & ~lane_span(0, max(first - j0, 0)));
+          carry += __popc(m & lane_span(min(max(pre - j0, 0), 32), min(max(pre + cnt - j0, 0), 32)));
+          in = in && before < kQueryPerCell;
+          m = __ballot_sync(kAll, in);
+        }
+        const int pos = base + __popc(m & below);
+        if (in && pos < cap) row[pos] = id;
+        base += __popc(m);
       }
-      base += __shfl_sync(0xffffffffu, incl, 31);
     }
-    written = base < cap ? base : cap;
+    const int written = min(base, cap);
+    if ((cap & 3) == 0 && ((uintptr_t)out & 15) == 0) {
+      const int whole = (written + 3) & ~3;
+      if (written + lane < whole) row[written + lane] = -1;
+      for (int e = whole + 4 * lane; e < cap; e += 128) *reinterpret_cast<int4*>(row + e) = make_int4(-1, -1, -1, -1);
+    } else {
+      for (int e = written + lane; e < cap; e += 32) row[e] = -1;
+    }
   }
-  for (int q = written + lane; q < cap; q += 32) row[q] = -1;
 }
 
 // Per pixel: first index of its run by binary search over the sorted pixel
@@ -170,10 +213,10 @@ extern "C" int32_t hp_quick_query_for_nearby_point(const float* xyz, int64_t n_p
     return set_error(HP_ERR_INVALID_ARGUMENT, "hp_quick_query_for_nearby_point: null pointer");
   if (((uintptr_t)hash_table & 7) != 0)
     return set_error(HP_ERR_INVALID_ARGUMENT, "hp_quick_query_for_nearby_point: hash_table must be 8-byte aligned");
-  const int blocks = (int)((n_rays + kQueryWarps - 1) / kQueryWarps);
-  k_quick_query<<<blocks, kQueryWarps * 32, 0, (cudaStream_t)stream>>>(
+  const int64_t per = kQueryWarps * kQueryRays;
+  k_quick_query<<<(unsigned)((n_rays + per - 1) / per), kQueryWarps * 32, 0, (cudaStream_t)stream>>>(
       xyz, (int)n_points, sorted_point_idx, (int)n_sorted, (const int2*)hash_table, dev_camera(cam), dev_options(opt),
-      ray_ids, (int)n_rays, out);
+      make_radius_test(opt->radius_threshold), ray_ids, (int)n_rays, out);
   return check_launch("k_quick_query");
 }
 

@@ -77,3 +77,44 @@ def test_paths_agree(kind, n, W, H, opt):
         for stage in (3, 4):
             for a, b in zip(run(sidx, table, heavy_window=heavy, stage_config=stage), want):
                 assert np.array_equal(a, b), (heavy, stage)
+
+
+@pytest.mark.parametrize("kind,n,W,H,k,radius,cap,rays", [
+    ("shapes", 20_000, 120, 90, 5, 0.02, 256, 3_001),
+    ("pile", 60_000, 40, 31, 5, 0.03, 256, 1_240),   # buckets above the 32 ids a cell gives, rows that overflow
+    ("pile", 60_000, 40, 31, 7, 0.03, 30, 333),      # more than 32 window cells, an odd row length
+    ("plane", 9_000, 40, 33, 31, 0.3, 101, 100),
+    ("plane", 9_000, 40, 33, 1, 0.1, 7, 9),
+])
+def test_listed_ray_query_vs_oracle(kind, n, W, H, k, radius, cap, rays):
+    import oracle as O
+    native.build()
+    rng = np.random.default_rng(n + k)
+    xyz, cam = _scene(kind, n, W, H, rng)
+    o = synth.Options(kernel_size=k, radius_threshold=radius, num_point_per_ray=cap)
+    X, c2w, w2c, K = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (xyz, cam.c2w, cam.w2c, cam.K)]
+    sidx, _, table = ops.pts2plane(X, w2c, K, H, W)
+    ids = rng.integers(-2, W * H + 2, rays).astype(np.int32)  # rays off the image give empty rows
+    out = ops.quick_query(X, c2w, cam.fx, cam.fy, cam.cx, cam.cy, W, H, o, sidx, table, torch.from_numpy(ids).cuda())
+    dirs = ops.ray_directions(c2w, cam.fx, cam.fy, cam.cx, cam.cy, W, H)
+    want, _, _ = O.quick_query(xyz, O.camera_from(cam), o, sidx.cpu().numpy(), table.cpu().numpy(), ids,
+                               dirs=dirs.cpu().numpy())
+    diff = np.nonzero((out.cpu().numpy() != want).any(1))[0]
+    # the oracle's norm is rounded correctly, the GPU's norm3df within an ulp: a row may differ only by a point
+    # whose distance is that close to the radius
+    _, _, margin = O.quick_query(xyz, O.camera_from(cam), o, sidx.cpu().numpy(), table.cpu().numpy(), ids,
+                                 dirs=dirs.cpu().numpy())
+    assert np.all(margin[diff] < 1e-6) and len(diff) <= max(1, rays // 100)
+
+
+@pytest.mark.parametrize("rays,S", [(1, 1), (1, 3), (3, 5), (257, 4), (255, 7), (1025, 8), (400, 16), (33, 31)])
+@pytest.mark.parametrize("off", [0, 1])
+def test_clamp_t_any_shape(rays, S, off):
+    native.build()
+    g = torch.Generator(device="cuda").manual_seed(rays * 37 + S)
+    buf = torch.empty(rays * S + off, device="cuda")
+    t = buf[off:].view(rays, S)
+    t.copy_(torch.cumsum(torch.rand((rays, S), device="cuda", generator=g) * 0.02 - 0.002, 1))
+    d = torch.cat([t[:, 1:] - t[:, :-1], torch.full_like(t[:, :1], 0.004)], 1)
+    m = ((d < 1e-8) | (d > 2 * torch.tensor(0.004, device="cuda"))).float()
+    assert torch.equal(ops.clamp_t(t, 0.004), d * (1 - m) + m * 0.004)
