@@ -13,30 +13,35 @@
 // accumulation in TMEM:
 //
 //   k_agg_pairs   one tile = 128 pair rows (128 / P samples), one CTA per SM,
-//                 warp-specialised:
-//                   warps 0-15 build the tile's 284-wide inputs (positional
-//                              encodings: one __sincosf per channel, higher
-//                              bands by the double-angle formulas) into the
-//                              layer-1 operand A0, and run the epilogues: read
-//                              the accumulator with tcgen05.ld, add the bias,
+//                 two tiles in flight, warp-specialised:
+//                   warps 0-7 and 8-15 (a team per tile) build the tile's
+//                              284-wide inputs (positional encodings: one
+//                              __sincosf per channel, higher bands by the
+//                              double-angle formulas) into the team's operand
+//                              A, and run the epilogues: read the team's
+//                              accumulator with tcgen05.ld, add the bias,
 //                              LeakyReLU, write the next layer's bf16 operand
-//                              A1 in 64-column blocks, each released to the
-//                              MMA warp by its own barrier, so the next layer
-//                              starts while later blocks are being written
-//                              (block3's seven extra inputs go to a separate
-//                              16-wide operand E);
+//                              over the last one's (block3's seven extra
+//                              inputs beside it, columns 256..271)
 //                              (warp w: TMEM lane quarter w % 4, columns
-//                              64 (w / 4) .. + 63 of its row);
-//                   warp 16    issues tcgen05.mma (M 128, N 256, K 16) from
-//                              A0 / A1 / E and the streamed weights;
+//                              32 (w / 4 % 2) .. + 31 of each 64);
+//                   warp 16    issues tcgen05.mma (M 128, N 256, K 16) from A
+//                              and the streamed weights, a layer of one team's
+//                              tile, then the same layer of the other's;
 //                   warp 17    streams the pre-packed weights (256 outputs x 32
 //                              K, 16 KB, 64-byte swizzled) from L2 into a
 //                              4-stage ring with cp.async.bulk.
-//                 Two TMEM accumulators (layers alternate), so the next
-//                 tile's layer 1 runs while this tile's last epilogue
-//                 computes the alpha branch and the weighted reduction over
-//                 each sample's rows, and the next tile's inputs are built
-//                 while this tile's layer 4 runs.
+//                 While one team's layer runs on the tensor cores the other
+//                 team is in its epilogue or builds its next tile's inputs: a
+//                 tile's own steps are one chain, so with one tile at a time
+//                 the tensor cores waited for every epilogue and the warps for
+//                 every layer.  60,000 samples x 8: 500 -> 382 us, tensor pipe
+//                 26 -> 34% active (143,000 x 8: 1141 -> ~800 us).  Of that the
+//                 second tile gave 6%, the MMA loop run by a whole warp 15%
+//                 (one lane took 590 cycles a chunk of two 128-cycle MMAs), the
+//                 biases and alpha weights from shared memory 9%.  What is left
+//                 is each team's chain: inputs 6 k cycles, three epilogues 2 k
+//                 each, the last one 7 k, four layers 2.1 k each.
 //   k_agg_color   one CTA = 128 samples: the colour-branch input tile arrives
 //                 with one bulk copy, three layers on the tensor cores, the
 //                 final 128->3 layer and the sigmoid on the CUDA cores.
@@ -61,7 +66,9 @@
 namespace hp {
 
 constexpr int kAggRows = 128;                      // pair rows (or samples) per tile = MMA M
-constexpr int kMathThreads = 512;                  // warps 0..15
+constexpr int kTeams = 2;                          // tiles in flight per CTA
+constexpr int kTeamThreads = 256;                  // math warps of a team
+constexpr int kMathThreads = kTeams * kTeamThreads;  // warps 0..15
 constexpr int kPairThreads = kMathThreads + 64;    // + MMA warp + load warp
 constexpr int kColorThreads = 256;
 constexpr int kMmaWarp = 16, kLoadWarp = 17;
@@ -84,9 +91,7 @@ __host__ __device__ constexpr int color_real_k(int L) { return L == 0 ? 280 : 12
 constexpr int kColorN = 128;
 constexpr int kColorChunks = (320 + 128 + 128) / kChunkK;  // 9
 constexpr int kWideK = 320;
-constexpr unsigned kATileBytes = kAggRows * kWideK * 2;     // 80 KB: A0, or one colour-input tile
-constexpr unsigned kA1Bytes = kAggRows * 256 * 2;           // 64 KB
-constexpr unsigned kEBytes = kAggRows * 16 * 2;             // extras operand, no swizzle
+constexpr unsigned kATileBytes = kAggRows * kWideK * 2;     // 80 KB: one colour-input tile
 constexpr unsigned kW3bBytes = kPairN * 16 * 2;             // block3.0 columns 256..262 (+ zeros), no swizzle
 
 // packed weight buffer: pair chunks, W3b, colour chunks, fp32 parameters
@@ -101,35 +106,55 @@ enum : int {
 };
 constexpr size_t kPackedBytes = kParamOff + (size_t)kParams * 4;
 
+// A pair operand: columns 0..255 in four 128-byte-swizzled blocks, then columns
+// 256..287 in a 64-byte-swizzled one (layer 1's last inputs, block3.0's extra
+// ones).  The packed weights' columns 288..319 of layer 1 are zeros and are
+// neither streamed nor multiplied.
+constexpr int kPairInputK = 288;
+static_assert(kPairInputK == 256 + kPairChunkK, "one chunk beyond the 128-byte-swizzled blocks");
+constexpr unsigned kTail = kAggRows * 256 * 2;                 // byte offset of the 64-byte-swizzled block
+constexpr unsigned kABytes = kTail + kAggRows * 32 * 2;        // 72 KB
+__host__ __device__ constexpr int pair_chunks(int L) { return (L == 0 ? kPairInputK : 256) / kPairChunkK; }
+__host__ __device__ constexpr int pair_chunk0(int L) { return L == 0 ? 0 : (320 + 256 * (L - 1)) / kPairChunkK; }
+
 // pair kernel shared memory (from a 1024-byte aligned base)
-constexpr unsigned kPA0 = 0;
-constexpr unsigned kPA1 = kPA0 + kATileBytes;
-constexpr unsigned kPStages = kPA1 + kA1Bytes;
-constexpr unsigned kPE = kPStages + kStages * kChunkBytes;
-constexpr unsigned kPW3b = kPE + kEBytes;
+constexpr unsigned kPA = 0;
+constexpr unsigned kPStages = kPA + kTeams * kABytes;
+constexpr unsigned kPW3b = kPStages + kStages * kChunkBytes;
 constexpr unsigned kPBar = kPW3b + kW3bBytes;
 constexpr unsigned kPScratch = kPBar + 256;
+constexpr unsigned kPParams = kPScratch + 2 * 4 * kAggRows * 4;  // block1.2 bias, block3.2 bias, alpha weights
 // colour kernel shared memory
 constexpr unsigned kCStages = kATileBytes;
 constexpr unsigned kCBar = kCStages + kStages * kChunkBytes;
 constexpr unsigned kCScratch = kCBar + 256;
-constexpr int kRed = 32;  // the last epilogue's transpose buffer: 32 x 32 floats per warp, column c of row r at c ^ r
 
 struct PairBars {
   uint64_t full[kStages];
   uint64_t empty[kStages];
-  uint64_t acc_full[2];  // MMA warp -> math warps: a layer completed into accumulator i
-  uint64_t a0_ready;     // math warps -> MMA warp: a tile's layer-1 operand is written (256 arrivals)
-  uint64_t a1_blk[4];    // math warps -> MMA warp: 64-column block i of the next layer's operand is written
-  uint64_t w3b;          // W3b landed
-  uint64_t idle;         // MMA warp: everything it issued has completed
+  uint64_t acc_full[kTeams];  // MMA warp -> team: a layer completed into its accumulator
+  uint64_t a_ready[kTeams];   // team -> MMA warp: the next layer's operand is written
+  uint64_t w3b;               // W3b landed
+  uint64_t idle;              // MMA warp: everything it issued has completed
   uint32_t tmem;
   int abort;
 };
 
-struct PairScratch {
-  float wgt[2][kAggRows];    // aggregation weight of each row, by tile parity
-  float apart[4][kAggRows];  // alpha-branch partial dot products (column quarters)
+// The order in which the CTA's layers run on the tensor cores, walked alike by
+// the load warp and the MMA warp: layer L of team 0's tile, of team 1's, then
+// layer L + 1 (f returns false to stop).  A whole tile of one team at a time,
+// or team 1 two layers behind, were within 2%.
+template <class F>
+__device__ __forceinline__ void each_layer(long long my_tiles, F&& f) {
+  for (long long i = 0; i < my_tiles; i += kTeams) {
+#pragma unroll 1
+    for (int s = 0; s < 4 * kTeams; s++)
+      if (i + s % kTeams < my_tiles && !f(s % kTeams, s / kTeams)) return;
+  }
+}
+
+struct PairScratch {           // of one team
+  float apart[4][kAggRows];    // alpha-branch partial dot products (column quarters)
 };
 
 struct Ring {  // colour kernel: barriers and bookkeeping of one CTA's weight stream (thread 0)
@@ -215,6 +240,12 @@ __device__ __forceinline__ uint4 pack8(const float* v) {
   return make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
 }
 
+// columns 8u .. 8u + 7 of row r of a pair operand
+__device__ __forceinline__ void store_pair_unit(uint8_t* A, int r, int u, const float* v) {
+  const uint32_t at = u < 32 ? tc::operand_offset(r, u * 8, kAggRows) : kTail + tc::sw64_offset(r, u * 8 - 256);
+  *reinterpret_cast<uint4*>(A + at) = pack8(v);
+}
+
 // columns 8u .. 8u + 7 of row r of a 128-row swizzled operand
 __device__ __forceinline__ void store_unit(uint8_t* A, int r, int u, const float* v) {
   *reinterpret_cast<uint4*>(A + tc::operand_offset(r, u * 8, kAggRows)) = pack8(v);
@@ -231,6 +262,11 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
 
 // LeakyReLU(0.01): max(x, 0.01 x) is x for x >= 0 and 0.01 x below.
 __device__ __forceinline__ float leaky(float x) { return fmaxf(x, __fmul_rn(x, 0.01f)); }
+
+__device__ __forceinline__ float2 leaky2(float2 x) {
+  const float2 y = tc::mul2(x, make_float2(0.01f, 0.01f));
+  return make_float2(fmaxf(x.x, y.x), fmaxf(x.y, y.y));
+}
 
 __device__ __forceinline__ float softplus(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
 
@@ -264,12 +300,15 @@ struct AggArgs {
   int withhold_w3b;            // a test of those waits: W3b is never loaded, so its wait gives up
 };
 
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // Layer-1 operand units U0 .. U1-1 of row r: columns 0..31 feat, 32..223 PE(feat, 3)
 // (argument a = channel * 3 + band at columns 32 + 2a (sin), 33 + 2a (cos)), 224..283
 // PE(dist_feat, 5), 284 the constant 1 (its weight column holds block1.0's bias),
-// 285..319 zeros.
+// 285..287 zeros.  (Rows beyond the last sample are encoded like zeros: their weight is 0
+// and no sample of theirs is written.)
 template <int U0, int U1>
-__device__ __forceinline__ void input_units(uint8_t* A0, int r, bool in, const float* feat, const float* df) {
+__device__ __forceinline__ void input_units(uint8_t* A, int r, const float* feat, const float* df) {
   float sf[3], cf[3], sd[5], cd[5];
   int chf = -1, chd = -1;
 #pragma unroll
@@ -298,17 +337,16 @@ __device__ __forceinline__ void input_units(uint8_t* A0, int r, bool in, const f
       } else if (col == 284) {
         x = 1.0f;
       }
-      v[i] = in ? x : 0.0f;
+      v[i] = x;
     }
-    store_unit(A0, r, u, v);
+    store_pair_unit(A, r, u, v);
   }
 }
 
-// The math warps' view of one tile's inputs: builds A0 and the rows' aggregation weights.
-__device__ __forceinline__ void build_inputs(const AggArgs& g, long long t, int spt, uint8_t* A0, float* wgt,
-                                             int tid) {
+// A team's view of one tile's inputs: builds A; returns the aggregation weight of the thread's row.
+__device__ __forceinline__ float build_inputs(const AggArgs& g, long long t, int spt, uint8_t* A, int tid) {
   const int P = g.P;
-  const int r = tid & (kAggRows - 1), h = tid >> 7;  // h: which 10 of the row's 40 units
+  const int r = tid & (kAggRows - 1), h = tid >> 7;  // h: which 18 of the row's 36 units
   const long long m = t * spt + r / P;
   const int p = r % P;
   const bool in = r < spt * P && m < g.M;
@@ -336,84 +374,76 @@ __device__ __forceinline__ void build_inputs(const AggArgs& g, long long t, int 
     }
     if (__ldg(g.valid + e)) inv = __fdiv_rn(1.0f, __fadd_rn(sqrtf(d2), 1e-6f));
   }
-  if (h == 0) {
-    // aggregation weight: inv / (sum over the sample's P rows + 1e-6); the rows are adjacent lanes
-    float sum = inv;
-    for (int o = 1; o < P; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    wgt[r] = __fdiv_rn(inv, __fadd_rn(sum, 1e-6f));
-    input_units<0, 10>(A0, r, in, feat, df);
-  } else if (h == 1) {
-    input_units<10, 20>(A0, r, in, feat, df);
-  } else if (h == 2) {
-    input_units<20, 30>(A0, r, in, feat, df);
-  } else {
-    input_units<30, 40>(A0, r, in, feat, df);
-  }
+  // aggregation weight: inv / (sum over the sample's P rows + 1e-6); the rows are adjacent lanes
+  float sum = inv;
+  for (int o = 1; o < P; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if (h == 0)
+    input_units<0, 18>(A, r, feat, df);
+  else
+    input_units<18, 36>(A, r, feat, df);
+  return __fdiv_rn(inv, __fadd_rn(sum, 1e-6f));
 }
 
-// Epilogue of a hidden layer, written in K order so the next layer's MMAs can
-// start on a block while later blocks are still being written: in round kb
-// every math thread converts columns 64 kb + 16 g .. + 15 (g = warp / 4) of its
-// row er -> LeakyReLU(x + bias) -> bf16 into the next operand (A1), then
-// arrives on block kb's barrier.  `last` runs before the final arrival.  bias is
-// null for the layers whose bias came in through the MMA.
-template <class Last>
-__device__ __forceinline__ void epilogue_hidden(uint32_t acc_addr, const float* bias, uint8_t* A1, int er, int g,
-                                                uint64_t* blk, Last&& last) {
+// Epilogue of a hidden layer: LeakyReLU(x + bias) -> bf16 into the next operand,
+// over the one the layer has read.  A thread takes columns 64 kb + 32 g .. + 31 of
+// its row er, kb = 0..3.  bias is null for the layers whose bias came in through
+// the MMA.
+__device__ __forceinline__ void epilogue_hidden(uint32_t acc_addr, const float* bias, uint8_t* A, int er, int g) {
 #pragma unroll 1
   for (int kb = 0; kb < 4; kb++) {
-    const int col0 = 64 * kb + 16 * g;
-    float v[16];
-    tc::tmem_ld16(acc_addr + (uint32_t)col0, v);
+    const int col0 = 64 * kb + 32 * g;
+    float v[32];
+    tc::tmem_ld32(acc_addr + (uint32_t)col0, v);
     if (bias) {
       const float4* b4 = reinterpret_cast<const float4*>(bias + col0);
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const float4 b = __ldg(b4 + q);
-        v[4 * q] = __fadd_rn(v[4 * q], b.x);
-        v[4 * q + 1] = __fadd_rn(v[4 * q + 1], b.y);
-        v[4 * q + 2] = __fadd_rn(v[4 * q + 2], b.z);
-        v[4 * q + 3] = __fadd_rn(v[4 * q + 3], b.w);
+      for (int q = 0; q < 8; q++) {
+        const float4 b = b4[q];
+        const float2 lo = tc::add2(make_float2(v[4 * q], v[4 * q + 1]), make_float2(b.x, b.y));
+        const float2 hi = tc::add2(make_float2(v[4 * q + 2], v[4 * q + 3]), make_float2(b.z, b.w));
+        v[4 * q] = lo.x, v[4 * q + 1] = lo.y, v[4 * q + 2] = hi.x, v[4 * q + 3] = hi.y;
       }
     }
 #pragma unroll
-    for (int i = 0; i < 16; i++) v[i] = leaky(v[i]);
-    store_unit(A1, er, col0 / 8, v);
-    store_unit(A1, er, col0 / 8 + 1, v + 8);
-    if (kb == 3) last();
-    tc::tc_fence_before();
-    tc::fence_async_smem();
-    tc::mbar_arrive(&blk[kb]);
+    for (int i = 0; i < 32; i += 2) {
+      const float2 y = leaky2(make_float2(v[i], v[i + 1]));
+      v[i] = y.x, v[i + 1] = y.y;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) store_unit(A, er, col0 / 8 + q, v + 8 * q);
   }
 }
 
-// Column sums over each sample's P rows of one warp's 32 x 32 transpose buffer (row =
-// pair row, column = this lane's feature column; written in place into rows 0..G-1),
-// then the sums to the colour-input rows, 8 columns per store.
+// The last epilogue's transpose buffer of a warp: 32 rows x 64 columns fp32, 16-byte
+// piece c of row r at piece c ^ (r % 16).
+constexpr int kRedBytes = 32 * 64 * 4;
+__device__ __forceinline__ uint32_t red_offset(int r, int c) { return (uint32_t)(r * 256 + ((c ^ (r & 15)) << 4)); }
+
+// Sums over each sample's P rows of a warp's transpose buffer, rows in order; lane l
+// takes columns 2 l and 2 l + 1 and stores their bf16 pair, so a sample's 64 columns
+// (col0 ..) are one 128-byte row of the colour-input tile.
 template <int P>
-__device__ __forceinline__ void sample_sums(float* red, int lane, long long m0, long long M, uint8_t* color_in,
+__device__ __forceinline__ void sample_sums(const uint8_t* red, int lane, long long m0, long long M, uint8_t* color_in,
                                             int col0) {
   constexpr int G = 32 / P;
-#pragma unroll
+  constexpr int kAhead = P < 8 ? P : 8;  // rows loaded before they are added
+#pragma unroll 1
   for (int gs = 0; gs < G; gs++) {
-    float v[P];
+    float2 acc = make_float2(0.f, 0.f);
+#pragma unroll 1
+    for (int p0 = 0; p0 < P; p0 += kAhead) {
+      float2 v[kAhead];
 #pragma unroll
-    for (int p = 0; p < P; p++) v[p] = red[(gs * P + p) * kRed + (lane ^ (gs * P + p))];
-    float acc = v[0];
+      for (int p = 0; p < kAhead; p++)
+        v[p] = *reinterpret_cast<const float2*>(red + red_offset(gs * P + p0 + p, lane >> 1) + (lane & 1) * 8);
 #pragma unroll
-    for (int p = 1; p < P; p++) acc = __fadd_rn(acc, v[p]);
-    if (P > 1) red[gs * kRed + (lane ^ gs)] = acc;  // rows below gs * P are read already
-  }
-  __syncwarp();
-  for (int un = lane; un < G * 4; un += 32) {
-    const int gs = un >> 2, q = un & 3;
-    const long long m = m0 + gs;
-    if (m < M) {
-      float o[8];
-#pragma unroll
-      for (int i = 0; i < 8; i++) o[i] = red[gs * kRed + ((8 * q + i) ^ gs)];
-      store_unit(color_in + (size_t)(m / kAggRows) * kATileBytes, (int)(m % kAggRows), col0 / 8 + q, o);
+      for (int p = 0; p < kAhead; p++) acc = p0 + p == 0 ? v[0] : tc::add2(acc, v[p]);
     }
+    const long long m = m0 + gs;
+    if (m < M)
+      *reinterpret_cast<uint32_t*>(color_in + (size_t)(m / kAggRows) * kATileBytes +
+                                   tc::operand_offset((int)(m % kAggRows), col0 + 2 * lane, kAggRows)) =
+          pack2(acc.x, acc.y);
   }
 }
 
@@ -423,27 +453,31 @@ __device__ __forceinline__ void sample_sums(float* red, int lane, long long m0, 
 __global__ void __launch_bounds__(kPairThreads, 1) k_agg_pairs(AggArgs g, long long n_tiles) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
-  uint8_t* A0 = smem + kPA0;
-  uint8_t* A1 = smem + kPA1;
   uint8_t* stages = smem + kPStages;
-  uint8_t* E = smem + kPE;
   uint8_t* W3b = smem + kPW3b;
   PairBars& bar = *reinterpret_cast<PairBars*>(smem + kPBar);
-  PairScratch& sc = *reinterpret_cast<PairScratch*>(smem + kPScratch);
   volatile int* abort = &bar.abort;
   const float* prm = reinterpret_cast<const float*>(g.packed + kParamOff);
+  float* s_b2 = reinterpret_cast<float*>(smem + kPParams);  // read from shared memory: from L2 each epilogue waited
+  float* s_b4 = s_b2 + kPairN;                              // for them (the operands leave next to no L1)
+  float* s_wa = s_b4 + kPairN;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int P = g.P, spt = kAggRows / P;
+  if (tid < kPairN) {
+    s_b2[tid] = prm[kPB2 + tid];
+    s_b4[tid] = prm[kPB4 + tid];
+    s_wa[tid] = prm[kPWA + tid];
+  }
 
   if (tid == 0) {
     for (int i = 0; i < kStages; i++) {
       tc::mbar_init(&bar.full[i], 1);
       tc::mbar_init(&bar.empty[i], 1);
     }
-    tc::mbar_init(&bar.acc_full[0], 1);
-    tc::mbar_init(&bar.acc_full[1], 1);
-    tc::mbar_init(&bar.a0_ready, kMathThreads);
-    for (int i = 0; i < 4; i++) tc::mbar_init(&bar.a1_blk[i], kMathThreads);
+    for (int i = 0; i < kTeams; i++) {
+      tc::mbar_init(&bar.acc_full[i], 1);
+      tc::mbar_init(&bar.a_ready[i], kTeamThreads);
+    }
     tc::mbar_init(&bar.w3b, 1);
     tc::mbar_init(&bar.idle, 1);
     bar.abort = 0;
@@ -454,26 +488,29 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_agg_pairs(AggArgs g, long l
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem = bar.tmem;
+  // the CTA's tiles blockIdx.x + i * gridDim.x; team i % 2 serves tile i
   const long long my_tiles = blockIdx.x < n_tiles ? (n_tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
   bool fail = false;
 
   if (warp == kLoadWarp) {
-    // ---- weight loads: W3b once, then the pair chunk stream, 34 chunks per tile
+    // ---- weight loads: W3b once, then each layer's chunks for one team's tile and again for the other's
     if (lane == 0) {
       if (!g.withhold_w3b) {
         tc::mbar_arrive_expect_tx(&bar.w3b, kW3bBytes);
         tc::bulk_load(W3b, g.packed + kW3bOff, kW3bBytes, &bar.w3b);
       }
-      const long long total = my_tiles * kPairChunks;
       long long q = 0;
-      for (; q < total; q++) {
-        const int st = (int)(q % kStages);
-        if (q >= kStages && !wait_or_abort(&bar.empty[st], (unsigned)(((q / kStages) - 1) & 1), abort, g.wait_ns))
-          break;
-        tc::mbar_arrive_expect_tx(&bar.full[st], kChunkBytes);
-        tc::bulk_load(stages + (size_t)st * kChunkBytes, g.packed + (size_t)(q % kPairChunks) * kChunkBytes,
-                      kChunkBytes, &bar.full[st]);
-      }
+      each_layer(my_tiles, [&](int, int L) -> bool {
+        const uint8_t* src = g.packed + (size_t)pair_chunk0(L) * kChunkBytes;
+        for (int kc = 0; kc < pair_chunks(L); kc++, q++) {
+          const int st = (int)(q % kStages);
+          if (q >= kStages && !wait_or_abort(&bar.empty[st], (unsigned)(((q / kStages) - 1) & 1), abort, g.wait_ns))
+            return false;
+          tc::mbar_arrive_expect_tx(&bar.full[st], kChunkBytes);
+          tc::bulk_load(stages + (size_t)st * kChunkBytes, src + (size_t)kc * kChunkBytes, kChunkBytes, &bar.full[st]);
+        }
+        return true;
+      });
       // the last copy into each stage has landed before the CTA ends
       for (long long d = q - 1; d >= 0 && d >= q - kStages; d--)
         if (!tc::mbar_wait(&bar.full[d % kStages], (unsigned)((d / kStages) & 1))) fail = true;
@@ -481,131 +518,156 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_agg_pairs(AggArgs g, long l
     }
     __syncwarp();  // the warp's other lanes wait for lane 0 here, not at the block barrier
   } else if (warp == kMmaWarp) {
-    // ---- MMA issue: per tile, layers 0..3 into accumulators 0, 1, 0, 1
-    if (lane == 0) {
-      const uint32_t idesc = tc::idesc_bf16(kAggRows, kPairN);
-      unsigned a0_ph = 0, a1_ph = 0;
-      long long q = 0;
-      bool ok = wait_or_abort(&bar.w3b, 0, abort, g.wait_ns);
-      for (long long t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
-        for (int L = 0; L < 4 && ok; L++) {
-          if (L == 0) {
-            if (!(ok = wait_or_abort(&bar.a0_ready, (a0_ph++) & 1, abort, g.wait_ns))) break;
-            tc::tc_fence_after();
-          }
-          const uint32_t acc = tmem + (uint32_t)(L & 1) * 256u;
-          const uint32_t a_addr = tc::smem_addr(L == 0 ? A0 : A1);
-          const int nk = pair_k(L) / kPairChunkK;
-          for (int kc = 0; kc < nk; kc++, q++) {
-            if (L > 0 && (kc & 1) == 0) {  // A1's 64-column block kc / 2 is written
-              if (!(ok = wait_or_abort(&bar.a1_blk[kc >> 1], a1_ph & 1, abort, g.wait_ns))) break;
-              tc::tc_fence_after();
-            }
-            const int st = (int)(q % kStages);
-            if (!(ok = wait_or_abort(&bar.full[st], (unsigned)((q / kStages) & 1), abort, g.wait_ns))) break;
-            tc::tc_fence_after();
-            const uint32_t b_addr = tc::smem_addr(stages + (size_t)st * kChunkBytes);
-#pragma unroll
-            for (int j = 0; j < kPairChunkK / 16; j++) {
-              const int k0 = kc * kPairChunkK + 16 * j;  // A: 64-wide 128-byte-swizzled blocks
-              tc::mma_bf16(acc, tc::smem_desc_sw128(a_addr + (uint32_t)(k0 >> 6) * (kAggRows * 128) + (k0 & 63) * 2),
-                           tc::smem_desc_sw64(b_addr + 32u * j), idesc, (kc > 0 || j > 0) ? 1u : 0u);
-            }
-            tc::mma_commit(&bar.empty[st]);
-          }
-          if (ok && L == 2)  // block3.0's extra inputs: E (K 16, written before block 3's arrival) times W3b
-            tc::mma_bf16(acc, tc::smem_desc_plain(tc::smem_addr(E), 128u, 256u),
-                         tc::smem_desc_plain(tc::smem_addr(W3b), 128u, 256u), idesc, 1u);
-          if (L > 0) a1_ph++;
-          tc::mma_commit(&bar.acc_full[L & 1]);
-        }
+    // ---- MMA issue: layer L of team 0's tile, of team 1's, then layer L + 1.  The whole warp runs the
+    // loop, so that descriptors and barrier phases are warp-uniform; lane 0 issues.  (One lane running it
+    // took 590 cycles a chunk of two 128-cycle MMAs.)
+    const uint32_t idesc = tc::idesc_bf16(kAggRows, kPairN);
+    const uint64_t w3b_desc = tc::smem_desc_plain(tc::smem_addr(W3b), 128u, 256u);
+    const uint64_t b_base = tc::smem_desc_sw64(tc::smem_addr(stages));
+    unsigned a_ph = 0;  // bit team: phase of its operand
+    uint32_t q = 0;     // weight chunks consumed
+    // the same answer in every lane, also when one of them gives up
+    auto wait = [&](uint64_t* b, unsigned parity) -> bool {
+      return __all_sync(0xffffffffu, wait_or_abort(b, parity, abort, g.wait_ns));
+    };
+    bool ok = wait(&bar.w3b, 0);
+    // a chunk of K: two K = 16 steps of the operand at `a`
+    auto chunk = [&](uint32_t acc, uint64_t a, bool first) -> bool {
+      const uint32_t st = q % kStages;
+      if (!wait(&bar.full[st], (q / kStages) & 1)) return false;
+      if (lane == 0) {
+        const uint64_t b = b_base + st * (kChunkBytes >> 4);
+        tc::mma_bf16(acc, a, b, idesc, first ? 0u : 1u);
+        tc::mma_bf16(acc, a + 2, b + 2, idesc, 1u);
+        tc::mma_commit(&bar.empty[st]);
       }
-      if (!ok) fail = true;
+      __syncwarp();
+      q++;
+      return true;
+    };
+    if (ok) {
+      each_layer(my_tiles, [&](int team, int L) -> bool {
+        if (!(ok = wait(&bar.a_ready[team], (a_ph >> team) & 1))) return false;
+        a_ph ^= 1u << team;
+        tc::tc_fence_after();
+        const uint32_t acc = tmem + (uint32_t)team * 256u;
+        const uint32_t a_addr = tc::smem_addr(smem + kPA + team * kABytes);
+        const uint64_t a_base = tc::smem_desc_sw128(a_addr), a_tail = tc::smem_desc_sw64(a_addr + kTail);
+#pragma unroll
+        for (int kc = 0; kc < 256 / kPairChunkK && ok; kc++)
+          ok = chunk(acc, a_base + (uint32_t)((kc >> 1) * (kAggRows * 128 / 16) + (kc & 1) * 4), kc == 0);
+        if (ok && L == 0) ok = chunk(acc, a_tail, false);
+        if (lane == 0) {
+          if (ok && L == 2)  // block3.0's extra inputs (columns 256..271) times W3b
+            tc::mma_bf16(acc, a_tail, w3b_desc, idesc, 1u);
+          tc::mma_commit(&bar.acc_full[team]);
+        }
+        __syncwarp();
+        return ok;
+      });
+    }
+    if (!ok) fail = true;
+    if (lane == 0) {
       tc::mma_commit(&bar.idle);
       if (!tc::mbar_wait(&bar.idle, 0)) fail = true;
     }
     __syncwarp();
   } else {
-    // ---- math warps: inputs, epilogues, reductions
-    const int er = 32 * (warp & 3) + lane, cq = warp >> 2;  // cq: also the column group of the epilogues
-    const uint32_t lane_addr = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
-    auto nothing = [] {};
-    unsigned acc_ph[2] = {0, 0};
-    int stop = 0, slot = 0;
-    if (my_tiles > 0) {
-      build_inputs(g, blockIdx.x, spt, A0, sc.wgt[0], tid);
+    // ---- a team: inputs, epilogues, reductions of its tiles
+    const int team = warp >> 3, ttid = tid & (kTeamThreads - 1);
+    const int er = 32 * (warp & 3) + lane, cq = (warp >> 2) & 1;  // row, column group
+    uint8_t* A = smem + kPA + team * kABytes;
+    PairScratch& sc = reinterpret_cast<PairScratch*>(smem + kPScratch)[team];
+    const uint32_t acc = tmem + (uint32_t)team * 256u + ((uint32_t)(32 * (warp & 3)) << 16);
+    unsigned acc_ph = 0;
+    int stop = 0;
+    auto ready = [&] {  // the operand is written and the accumulator read
+      tc::tc_fence_before();
       tc::fence_async_smem();
-      tc::mbar_arrive(&bar.a0_ready);
-    }
-    for (long long t = blockIdx.x; t < n_tiles && !stop; t += gridDim.x, slot ^= 1) {
-      // layer 1 -> A1
-      if (!wait_or_abort(&bar.acc_full[0], (acc_ph[0]++) & 1, abort, g.wait_ns)) fail = true;
+      tc::mbar_arrive(&bar.a_ready[team]);
+    };
+    auto layer = [&] {  // the layer is in the accumulator
+      if (!wait_or_abort(&bar.acc_full[team], (acc_ph++) & 1, abort, g.wait_ns)) fail = true;
       tc::tc_fence_after();
-      epilogue_hidden(lane_addr, nullptr, A1, er, cq, bar.a1_blk, nothing);  // bias: A0 column 284
-      // layer 2 -> A1, and block3's extra inputs -> E
-      if (!wait_or_abort(&bar.acc_full[1], (acc_ph[1]++) & 1, abort, g.wait_ns)) fail = true;
-      tc::tc_fence_after();
-      epilogue_hidden(lane_addr + 256u, prm + kPB2, A1, er, cq, bar.a1_blk, [&] {
-      if (cq == 3) {
+    };
+    for (long long i = team; i < my_tiles && !stop; i += kTeams) {
+      const long long t = blockIdx.x + i * gridDim.x;
+      const float w = build_inputs(g, t, spt, A, ttid);  // of row er, which is the row the thread built
+      ready();
+      // layer 1 (its bias: column 284 of the inputs)
+      layer();
+      epilogue_hidden(acc, nullptr, A, er, cq);
+      ready();
+      // layer 2, and block3's extra inputs
+      float ex[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      if (cq == 1) {
         const long long m = t * spt + er / P;
         const long long e = m * P + er % P;
-        float ex[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         if (er < spt * P && m < g.M) {
           float dot = 0.0f;
 #pragma unroll
-          for (int i = 0; i < 3; i++) {
-            const float dv = __ldg(g.pc_dir + e * 3 + i), rd = __ldg(g.rays_d + m * 3 + i);
-            ex[i] = __ldg(g.pc_rgb + e * 3 + i);
-            ex[3 + i] = __fsub_rn(dv, rd);
-            dot = i == 0 ? __fmul_rn(dv, rd) : __fmaf_rn(dv, rd, dot);
+          for (int c = 0; c < 3; c++) {
+            const float dv = __ldg(g.pc_dir + e * 3 + c), rd = __ldg(g.rays_d + m * 3 + c);
+            ex[c] = __ldg(g.pc_rgb + e * 3 + c);
+            ex[3 + c] = __fsub_rn(dv, rd);
+            dot = c == 0 ? __fmul_rn(dv, rd) : __fmaf_rn(dv, rd, dot);
           }
           ex[6] = dot;
           ex[7] = 1.0f;  // its W3b column holds block3.0's bias
         }
-        *reinterpret_cast<uint4*>(E + tc::plain16_offset(er, 0)) = pack8(ex);
-        *reinterpret_cast<uint4*>(E + tc::plain16_offset(er, 8)) = make_uint4(0, 0, 0, 0);
       }
-      });
-      // layer 3 -> A1
-      if (!wait_or_abort(&bar.acc_full[0], (acc_ph[0]++) & 1, abort, g.wait_ns)) fail = true;
-      tc::tc_fence_after();
-      epilogue_hidden(lane_addr, nullptr, A1, er, cq, bar.a1_blk, nothing);  // bias: E column 7
-      // the next tile's inputs (A0's reader, this tile's layer 1, has completed) while layer 4 runs
-      if (t + gridDim.x < n_tiles) {
-        build_inputs(g, t + gridDim.x, spt, A0, sc.wgt[slot ^ 1], tid);
-        tc::fence_async_smem();
-        tc::mbar_arrive(&bar.a0_ready);
+      layer();
+      if (cq == 1) {
+        store_pair_unit(A, er, 32, ex);
+        *reinterpret_cast<uint4*>(A + kTail + tc::sw64_offset(er, 8)) = make_uint4(0, 0, 0, 0);
+      }
+      epilogue_hidden(acc, s_b2, A, er, cq);
+      ready();
+      // layer 3 (its bias: column 7 of the extra inputs)
+      layer();
+      epilogue_hidden(acc, nullptr, A, er, cq);
+      ready();
+      if (i + kTeams < my_tiles) {  // the next tile's inputs on their way to L2
+        const long long e = ((t + (long long)kTeams * gridDim.x) * spt) * P + (ttid & (kAggRows - 1));
+        if (e < g.M * P) {
+          if (ttid < kAggRows)
+            prefetch_l2(g.pc_feat + e * kFeatDim);
+          else if ((ttid & 7) == 0)
+            prefetch_l2(g.pc_xyz + e * 3);
+        }
       }
       // layer 4: alpha-branch dot product per row, and the weighted sum over each sample's
-      // rows: the warp's 32 rows x 32 columns go through a transpose buffer (in A1, whose
+      // rows: the warp's 32 rows x 32 columns go through a transpose buffer (in A, whose
       // last reader, layer 4, has completed), lane l sums column l of each sample in place,
       // and the sums are written to the colour-input rows 8 columns at a time.
-      if (!wait_or_abort(&bar.acc_full[1], (acc_ph[1]++) & 1, abort, g.wait_ns)) fail = true;
-      tc::tc_fence_after();
+      layer();
       {
-        const float w = sc.wgt[slot][er];
-        const float* wa = prm + kPWA;
-        const float* bias = prm + kPB4;
-        float* red = reinterpret_cast<float*>(A1) + warp * (32 * kRed);
+        const float2 w2 = make_float2(w, w);
+        uint8_t* red = A + (warp & 7) * kRedBytes;
         const long long m0 = (t * kAggRows + 32 * (warp & 3)) / P;  // the warp's first sample
-        float adot = 0.0f;
 #pragma unroll 1
         for (int cc = 0; cc < 2; cc++) {
-          const int col0 = 64 * cq + 32 * cc;
-          float v[32];
-          tc::tmem_ld32(lane_addr + 256u + (uint32_t)col0, v);
+          const int col0 = 128 * cq + 64 * cc;
+          float adot = 0.0f;
 #pragma unroll
-          for (int q = 0; q < 8; q++) {
-            const float4 b = __ldg(reinterpret_cast<const float4*>(bias + col0) + q);
-            const float4 a = __ldg(reinterpret_cast<const float4*>(wa + col0) + q);
-            const float bb[4] = {b.x, b.y, b.z, b.w}, aa[4] = {a.x, a.y, a.z, a.w};
+          for (int half = 0; half < 2; half++) {
+            float v[32];
+            tc::tmem_ld32(acc + (uint32_t)(col0 + 32 * half), v);
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-              const float f = leaky(__fadd_rn(v[4 * q + i], bb[i]));
-              adot = __fmaf_rn(f, aa[i], adot);
-              red[lane * kRed + ((4 * q + i) ^ lane)] = __fmul_rn(f, w);
+            for (int q = 0; q < 8; q++) {
+              const float4 b = reinterpret_cast<const float4*>(s_b4 + col0 + 32 * half)[q];
+              const float4 a = reinterpret_cast<const float4*>(s_wa + col0 + 32 * half)[q];
+              const float2 f0 = leaky2(tc::add2(make_float2(v[4 * q], v[4 * q + 1]), make_float2(b.x, b.y)));
+              const float2 f1 = leaky2(tc::add2(make_float2(v[4 * q + 2], v[4 * q + 3]), make_float2(b.z, b.w)));
+              adot = __fmaf_rn(f0.x, a.x, adot);
+              adot = __fmaf_rn(f0.y, a.y, adot);
+              adot = __fmaf_rn(f1.x, a.z, adot);
+              adot = __fmaf_rn(f1.y, a.w, adot);
+              const float2 x0 = tc::mul2(f0, w2), x1 = tc::mul2(f1, w2);
+              *reinterpret_cast<float4*>(red + red_offset(lane, 8 * half + q)) = make_float4(x0.x, x0.y, x1.x, x1.y);
             }
           }
+          sc.apart[2 * cq + cc][er] = adot;
           __syncwarp();
           switch (P) {
             case 1: sample_sums<1>(red, lane, m0, g.M, g.color_in, col0); break;
@@ -617,22 +679,21 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_agg_pairs(AggArgs g, long l
           }
           __syncwarp();
         }
-        sc.apart[cq][er] = adot;
         const long long m = t * spt + er / P;
-        if (cq == 3 && er % P == 0 && er < spt * P && m < g.M) {  // PE(ray_d, 4) -> columns 256..279, zeros to 319
+        if (cq == 1 && er % P == 0 && er < spt * P && m < g.M) {  // PE(ray_d, 4) -> columns 256..279, zeros to 319
           uint8_t* crow = g.color_in + (size_t)(m / kAggRows) * kATileBytes;
           const int cr = (int)(m % kAggRows);
           float s4[3][4], c4[3][4];
 #pragma unroll
-          for (int i = 0; i < 3; i++) bands<4>(__ldg(g.rays_d + m * 3 + i), s4[i], c4[i]);
+          for (int c = 0; c < 3; c++) bands<4>(__ldg(g.rays_d + m * 3 + c), s4[c], c4[c]);
 #pragma unroll
           for (int u = 0; u < 3; u++) {
             float v[8];
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-              const int a = 4 * u + i;
-              v[2 * i] = s4[a / 4][a % 4];
-              v[2 * i + 1] = c4[a / 4][a % 4];
+            for (int c = 0; c < 4; c++) {
+              const int a = 4 * u + c;
+              v[2 * c] = s4[a / 4][a % 4];
+              v[2 * c + 1] = c4[a / 4][a % 4];
             }
             store_unit(crow, cr, 32 + u, v);
           }
@@ -641,11 +702,11 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_agg_pairs(AggArgs g, long l
         }
       }
       tc::tc_fence_before();
-      stop = tc::named_sync_or(fail || *abort, kMathThreads);
+      stop = tc::named_sync_or(fail || *abort, 1 + team, kTeamThreads);
       if (stop) break;
       // alpha: softplus(branch - 1) of each valid row, weighted sum over the sample
-      if (tid < kAggRows) {
-        const int r = tid;
+      if (ttid < kAggRows) {
+        const int r = ttid;
         const long long m = t * spt + r / P;
         const int p = r % P;
         const bool in = r < spt * P && m < g.M;
@@ -655,11 +716,12 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_agg_pairs(AggArgs g, long l
                                               __fadd_rn(sc.apart[2][r], sc.apart[3][r])), prm[kPBA]);
           a = softplus(__fsub_rn(z, 1.0f));
         }
-        float x = __fmul_rn(a, sc.wgt[slot][r]);
+        float x = __fmul_rn(a, w);
         for (int o = 1; o < P; o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
         if (in && p == 0) g.alpha[m] = x;
       }
-      stop = tc::named_sync_or(fail || *abort, kMathThreads);  // apart and A1 are rewritten next tile
+      // apart is rewritten next tile
+      if (i + kTeams < my_tiles) stop = tc::named_sync_or(fail || *abort, 1 + team, kTeamThreads);
     }
   }
 
@@ -920,11 +982,12 @@ AggLayout agg_layout(long long M) {
   return L;
 }
 
-constexpr unsigned kPairSmem = kPScratch + sizeof(PairScratch) + 1024;
+constexpr unsigned kPairSmem = kPParams + 3 * kPairN * 4 + 1024;
+static_assert(kTeams * sizeof(PairScratch) == kPParams - kPScratch, "scratch");
 constexpr unsigned kColorSmem = kCScratch + sizeof(ColorScratch) + 1024;
 static_assert(sizeof(PairBars) <= 256 && sizeof(Ring) <= 256, "barrier block");
 static_assert(kPairSmem <= 227 * 1024 && kColorSmem <= 227 * 1024, "shared memory");
-static_assert(kMathThreads / 32 * 32 * kRed * 4 <= kA1Bytes, "transpose buffers fit in A1");
+static_assert(kTeamThreads / 32 * kRedBytes <= kABytes && kABytes % 1024 == 0, "transpose buffers fit in A");
 }  // namespace
 
 extern "C" size_t hp_aggregator_packed_size(void) { return kPackedBytes; }

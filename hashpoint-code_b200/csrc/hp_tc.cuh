@@ -137,12 +137,11 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int m, int n) {
 // D[tmem] (+)= A[smem] * B[smem]^T, M x N x 16; issued by one thread.
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                          uint32_t accumulate) {
-  const uint32_t z = 0;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(z), "r"(z), "r"(z), "r"(z)
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 
@@ -199,19 +198,38 @@ __host__ __device__ __forceinline__ uint32_t plain16_offset(int r, int k) {
   return (uint32_t)((r >> 3) * 256 + (k >> 3) * 128 + (r & 7) * 16 + (k & 7) * 2);
 }
 
-// Barrier 1 over the first n threads of the block (warps 0 .. n/32 - 1), with
-// an OR of pred over them returned to all.
-__device__ __forceinline__ int named_sync_or(int pred, int n) {
+// Barrier `id` (1..15) over n threads (whole warps), with an OR of pred over
+// them returned to all.
+__device__ __forceinline__ int named_sync_or(int pred, int id, int n) {
   int r;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.s32 p, %1, 0;\n\t"
-      "bar.red.or.pred q, 1, %2, p;\n\t"
+      "bar.red.or.pred q, %2, %3, p;\n\t"
       "selp.s32 %0, 1, 0, q;\n\t}"
       : "=r"(r)
-      : "r"(pred), "r"(n)
+      : "r"(pred), "r"(id), "r"(n)
       : "memory");
   return r;
+}
+
+// Two fp32 lanes in one instruction, each rounded as the single one rounds.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+      "add.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+      "mul.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
 }
 
 // Byte offset of element (r, k) in a K-major 128-byte-swizzled operand of R rows.
