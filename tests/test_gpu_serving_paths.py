@@ -4,7 +4,7 @@ A ray is served by 8 lanes, by a whole warp, or -- where its window's buckets
 do not follow one another in the sorted ids, its list overflows or a decision
 is too close for the fast arithmetic -- by the general walk.  Storing the same
 buckets in reversed pixel order sends every ray with two non-empty cells in a
-window row to the general walk, so each scene is sampled with both tables and
+window row (so not kernel_size 1) to the general walk, so each scene is sampled with both tables and
 with heavy windows from "every ray" to "none".
 """
 import numpy as np
@@ -14,6 +14,9 @@ import torch
 from hashpoint import native, ops, synth
 
 pytestmark = pytest.mark.gpu
+
+
+EYE = (0.3, 0.2, 4.0)
 
 
 def _reversed_buckets(sidx, table):
@@ -38,9 +41,22 @@ def _scene(kind, n, W, H, rng):
         xyz = np.concatenate([xyz, xyz, xyz])[rng.permutation(3 * len(xyz))]
     elif kind == "pile":  # buckets far above 48 entries
         xyz = synth.sphere_cloud(rng, n, noise=0.05) * 0.3
+    elif kind == "rings":  # a ninth point as near to each pixel's ray as the nearest of eight, but for a part in 2^13 or less
+        d = np.stack([(np.arange(W * H) % W + 0.5 - W / 2) / (0.9 * W), (np.arange(W * H) // W + 0.5 - H / 2) / (0.9 * W),
+                      np.ones(W * H)], 1) @ synth.look_at_camera(EYE, (0, 0, 0), W, H, 0.9 * W).c2w[:3, :3].T.astype(np.float64)
+        d /= np.linalg.norm(d, axis=1, keepdims=True)
+        a = np.cross(d, [0.3, 0.5, 0.8])
+        a /= np.linalg.norm(a, axis=1, keepdims=True)
+        rings = n // (W * H)
+        phi = rng.uniform(0, 2 * np.pi, (rings, W * H, 1))
+        rho = 0.0025 * (1 + 0.05 * np.array([3, 5, 1, 7, 2, 4, 0, 6]))  # the first eight well apart,
+        later = rho.min() * (1 + 0.07 * np.arange(rings - 8))  # the later ones next to the least, or apart
+        rho = np.concatenate([rho, later])[:, None, None] * np.ones((1, W * H, 1))
+        rho[8] *= 1 + np.linspace(0, 2.0 ** -13, W * H)[:, None]
+        xyz = (np.asarray(EYE) + 4 * d + rho * (np.cos(phi) * a + np.sin(phi) * np.cross(d, a))).reshape(-1, 3)
     else:
         xyz = synth.shapes_cloud(rng, n)
-    cam = synth.look_at_camera((0.3, 0.2, 4.0), (0, 0, 0), W, H, 0.9 * W)
+    cam = synth.look_at_camera(EYE, (0, 0, 0), W, H, 0.9 * W)
     return xyz.astype(np.float32), cam
 
 
@@ -55,6 +71,9 @@ def _scene(kind, n, W, H, rng):
     ("plane", 9_000, 40, 33, dict(kernel_size=3, radius_threshold=0.1, sdf2weight_gaussian_alpha=0.0005)),
     ("plane", 9_000, 40, 33, dict(kernel_size=3, radius_threshold=0.1, sdf2weight_gaussian_alpha=0.02)),
     ("twins", 20_000, 65, 49, dict(kernel_size=5, radius_threshold=0.04, num_point_cloud_per_sp=8)),
+    # distances around the closeness that sends a ray to the general walk
+    ("rings", 9 * 200 * 150, 200, 150, dict(kernel_size=2, radius_threshold=0.005)),
+    ("rings", 11 * 200 * 150, 200, 150, dict(kernel_size=2, radius_threshold=0.005)),
     ("pile", 60_000, 40, 31, dict(kernel_size=5, radius_threshold=0.03, num_point_cloud_per_sp=8)),
     ("pile", 60_000, 33, 16, dict(kernel_size=2, radius_threshold=0.5, num_point_cloud_per_sp=8)),
     ("shapes", 40_000, 160, 120, dict(kernel_size=1, radius_threshold=0.02, num_point_cloud_per_sp=4)),
