@@ -15,11 +15,11 @@ from hashpoint import ops
 
 
 def _as_float(v):
-    return float(v.item() if isinstance(v, torch.Tensor) else v)
+    return v if type(v) is float else float(v.item() if isinstance(v, torch.Tensor) else v)
 
 
 def _as_int(v):
-    return int(v.item() if isinstance(v, torch.Tensor) else v)
+    return v if type(v) is int else int(v.item() if isinstance(v, torch.Tensor) else v)
 
 
 class _Spec:
@@ -27,25 +27,26 @@ class _Spec:
     _ints = ()
     _tensors = ()
 
+    def __init_subclass__(cls):
+        def tensor(name):
+            def cast(value):
+                if not isinstance(value, torch.Tensor):
+                    raise TypeError("%s.%s must be a torch.Tensor" % (cls.__name__, name))
+                return value
+            return cast
+
+        cls._casts = {**{f: _as_float for f in cls._floats}, **{f: _as_int for f in cls._ints},
+                      **{f: tensor(f) for f in cls._tensors}}
+        cls._defaults = {**{f: 0.0 for f in cls._floats}, **{f: 0 for f in cls._ints}, **{f: None for f in cls._tensors}}
+
     def __init__(self):
-        for f in self._floats:
-            object.__setattr__(self, f, 0.0)
-        for f in self._ints:
-            object.__setattr__(self, f, 0)
-        for f in self._tensors:
-            object.__setattr__(self, f, None)
+        self.__dict__.update(self._defaults)
 
     def __setattr__(self, name, value):
-        if name in self._floats:
-            value = _as_float(value)
-        elif name in self._ints:
-            value = _as_int(value)
-        elif name in self._tensors:
-            if not isinstance(value, torch.Tensor):
-                raise TypeError("%s.%s must be a torch.Tensor" % (type(self).__name__, name))
-        else:
+        cast = self._casts.get(name)
+        if cast is None:
             raise AttributeError("%s has no field %r" % (type(self).__name__, name))
-        object.__setattr__(self, name, value)
+        self.__dict__[name] = cast(value)
 
 
 class NeuralPointsSpec(_Spec):

@@ -79,13 +79,14 @@ class CameraSpec:
         same version (an in-place change bumps a tensor's version), so the calls of one view --
         pts2plane, then render_image_hashtable_topk -- read them once."""
         fields = (self.fx, self.fy, self.cx, self.cy, self.width, self.height)
+        if not any(isinstance(f, torch.Tensor) for f in fields):
+            return fields
         versions = tuple(f._version if isinstance(f, torch.Tensor) else None for f in fields)
         hit = self.__dict__.get("_host_cache")
         if hit is not None and all(a is b for a, b in zip(hit[0], fields)) and hit[1] == versions:
             return hit[2]
         vals = tuple(_host_values(*fields))
-        if any(isinstance(f, torch.Tensor) for f in fields):
-            self.__dict__["_host_cache"] = (fields, versions, vals)
+        self.__dict__["_host_cache"] = (fields, versions, vals)
         return vals
 
     def _to_cpp(self):

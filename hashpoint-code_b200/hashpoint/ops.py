@@ -11,15 +11,16 @@ import torch
 
 from . import native
 
-_vp = ctypes.c_void_p
-
 
 def _ptr(t):
-    return _vp(t.data_ptr()) if t is not None and t.numel() > 0 else _vp(0)
+    """A tensor's device address as an int (ctypes takes it for a pointer); 0 for None or an empty tensor."""
+    return t.data_ptr() if t is not None and t.numel() > 0 else 0
 
 
 def _stream(device):
-    return _vp(torch.cuda.current_stream(device).cuda_stream)
+    """torch's current stream of `device` as an int (without the Stream object current_stream builds)."""
+    i = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if i is None else i)
 
 
 def check_input(t, name, dtype=None):
@@ -43,26 +44,15 @@ def check_matrix(t, name, rows=3, cols=4):
 
 def make_camera(c2w=None, w2c=None, K=None, fx=0.0, fy=0.0, cx=0.0, cy=0.0, width=0, height=0):
     """HpCamera over device tensors (the caller keeps the tensors alive)."""
-    cam = native.HpCamera()
-    cam.c2w = _ptr(c2w).value
-    cam.w2c = _ptr(w2c).value
-    cam.K = _ptr(K).value
-    cam.fx, cam.fy, cam.cx, cam.cy = float(fx), float(fy), float(cx), float(cy)
-    cam.width, cam.height = int(width), int(height)
-    return cam
+    return native.HpCamera(_ptr(c2w), _ptr(w2c), _ptr(K), float(fx), float(fy), float(cx), float(cy), int(width),
+                           int(height))
 
 
 def make_options(opt):
-    o = native.HpOptions()
-    o.kernel_size = int(opt.kernel_size)
-    o.t_intvl = float(opt.t_intvl)
-    o.radius_threshold = float(opt.radius_threshold)
-    o.num_sample_points_per_ray = int(opt.num_sample_points_per_ray)
-    o.num_point_cloud_per_sp = int(opt.num_point_cloud_per_sp)
-    o.num_point_per_ray = int(opt.num_point_per_ray)
-    o.sdf2weight_gaussian_alpha = float(opt.sdf2weight_gaussian_alpha)
-    o.sdf2weight_gaussian_gamma = float(opt.sdf2weight_gaussian_gamma)
-    return o
+    return native.HpOptions(int(opt.kernel_size), float(opt.t_intvl), float(opt.radius_threshold),
+                            int(opt.num_sample_points_per_ray), int(opt.num_point_cloud_per_sp),
+                            int(opt.num_point_per_ray), float(opt.sdf2weight_gaussian_alpha),
+                            float(opt.sdf2weight_gaussian_gamma))
 
 
 def pts2plane(xyz, w2c, K, height, width, sort=False):
@@ -113,8 +103,9 @@ def scatter_hashtable(point_idx, point2img, depth, height, width, sort=False):
 def _hash_view(hash_table, height, width):
     check_input(hash_table, "hashtable", torch.int32)
     if hash_table.dim() == 2:
-        hash_table = hash_table.view(height, width, 2)
-    if hash_table.dim() != 3 or tuple(hash_table.shape) != (height, width, 2):
+        if hash_table.numel() != height * width * 2:
+            hash_table = hash_table.view(height, width, 2)  # raises
+    elif hash_table.dim() != 3 or tuple(hash_table.shape) != (height, width, 2):
         raise RuntimeError("hashtable size error: %s" % (tuple(hash_table.shape),))
     return hash_table
 
@@ -172,11 +163,10 @@ def make_view(xyz, c2w, fx, fy, cx, cy, width, height, opt, sorted_point_idx, ha
     hash_table = _hash_view(hash_table, H, W)
     sp_xyz, pc_idx, sp_t, mask = outputs
     v = native.HpView()
-    v.xyz, v.n_points = _ptr(xyz).value, xyz.shape[0]
-    v.sorted_point_idx, v.n_sorted = _ptr(sorted_point_idx).value, sorted_point_idx.numel()
-    v.hash_table = _ptr(hash_table).value
-    v.sp_xyz, v.pc_idx, v.sp_t, v.mask = (_ptr(sp_xyz).value, _ptr(pc_idx).value, _ptr(sp_t).value,
-                                          _ptr(mask).value)
+    v.xyz, v.n_points = _ptr(xyz), xyz.shape[0]
+    v.sorted_point_idx, v.n_sorted = _ptr(sorted_point_idx), sorted_point_idx.numel()
+    v.hash_table = _ptr(hash_table)
+    v.sp_xyz, v.pc_idx, v.sp_t, v.mask = _ptr(sp_xyz), _ptr(pc_idx), _ptr(sp_t), _ptr(mask)
     v.cam = make_camera(c2w=c2w, fx=fx, fy=fy, cx=cx, cy=cy, width=W, height=H)
     v.opt = make_options(opt)
     return v
@@ -305,7 +295,7 @@ def feature_query(xyz, rgb, dir_, feat, sp_xyz, pc_idx, mask, c2w, fx, fy, cx, c
            torch.empty((M, 3), dtype=torch.float32, device=dev))
     if M == 0:
         return out
-    pts = native.HpPointAttrs(_ptr(xyz).value, _ptr(rgb).value, _ptr(dir_).value, _ptr(feat).value, F,
+    pts = native.HpPointAttrs(_ptr(xyz), _ptr(rgb), _ptr(dir_), _ptr(feat), F,
                               int(feat.dtype == torch.float16), xyz.shape[0])
     cam = make_camera(c2w=c2w, fx=fx, fy=fy, cx=cx, cy=cy, width=width, height=1)
     rc = native.lib().hp_feature_query(ctypes.byref(pts), _ptr(sp_xyz), _ptr(pc_idx), _ptr(mask), n_rays, S, P,
