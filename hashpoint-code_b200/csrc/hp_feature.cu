@@ -87,49 +87,82 @@ __global__ void __launch_bounds__(1024) k_mask_scan_tiles(int* __restrict__ tile
 }
 
 // offsets[i] = valid samples before i (tile base + block-local exclusive scan).
+// kSum: `tile` holds the tiles' counts, and each block adds up those before its
+// own (a few loads a thread while there are at most kSumTiles, and one launch
+// less: FeatureQuery over 5.1M samples went from 299 us to 293, with wider feature stores); the
+// last block writes the total.  Else `tile` holds their scan.
+constexpr int kSumTiles = 4096;
+template <bool kSum>
 __global__ void __launch_bounds__(kScanThreads) k_mask_offsets(const uint8_t* __restrict__ mask, int64_t n,
-                                                               const int* __restrict__ tile_base,
-                                                               int* __restrict__ offsets) {
-  __shared__ int warp_sum[kScanThreads / 32];
-  const int64_t base = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanPerThread;
-  uint8_t v[kScanPerThread];
-  if (base + kScanPerThread <= n && ((uintptr_t)(mask + base) & 15) == 0) {
-    const uint4 w = *reinterpret_cast<const uint4*>(mask + base);
-    const unsigned ws[4] = {w.x, w.y, w.z, w.w};
+                                                               const int* __restrict__ tile, int* __restrict__ offsets,
+                                                               int* __restrict__ count) {
+  int tile_base = 0;
+  if constexpr (kSum) {
+    __shared__ int part[kScanThreads / 32];
+    int sum = 0;
+    for (int q = threadIdx.x; q < (int)blockIdx.x; q += kScanThreads) sum += __ldg(tile + q);
 #pragma unroll
-    for (int q = 0; q < kScanPerThread; q++) v[q] = ((ws[q >> 2] >> (8 * (q & 3))) & 0xffu) != 0;
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sum;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kScanThreads / 32; w++) tile_base += part[w];
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *count = tile_base + __ldg(tile + blockIdx.x);
   } else {
-#pragma unroll
-    for (int q = 0; q < kScanPerThread; q++) v[q] = base + q < n ? mask[base + q] != 0 : 0;
+    tile_base = __ldg(tile + blockIdx.x);
   }
-  int local = 0;
-#pragma unroll
-  for (int q = 0; q < kScanPerThread; q++) local += v[q];
-  int incl = local;
+  // A warp takes 512 mask bytes in four passes of 128 (four a lane), so that each
+  // load and store instruction covers whole lines.  A pass counts at most 128:
+  // the four passes' counts scan as the bytes of one word.
+  constexpr int kPasses = kScanPerThread / 4;
+  static_assert(kPasses == 4, "a byte per pass");
+  __shared__ int warp_sum[kScanThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t base = (int64_t)blockIdx.x * kScanTile + warp * (32 * kScanPerThread) + 4 * lane;
+  const bool aligned = (((uintptr_t)mask & 3) | ((uintptr_t)offsets & 15)) == 0;
+  unsigned w[kPasses], local = 0;
+#pragma unroll
+  for (int k = 0; k < kPasses; k++) {
+    const int64_t i = base + 128 * k;
+    w[k] = 0;
+    if (aligned && i + 4 <= n) {
+      w[k] = __vcmpne4(__ldg(reinterpret_cast<const unsigned*>(mask + i)), 0u) & 0x01010101u;
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+        if (i + q < n) w[k] |= (unsigned)(mask[i + q] != 0) << (8 * q);
+    }
+    local |= (unsigned)__popc(w[k]) << (8 * k);
+  }
+  unsigned incl = local;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
     if (lane >= o) incl += t;
   }
-  if (lane == 31) warp_sum[warp] = incl;
+  const unsigned total = __shfl_sync(0xffffffffu, incl, 31);
+  auto byte = [](unsigned x, int k) { return (int)((x >> (8 * k)) & 0xffu); };
+  if (lane == 0) warp_sum[warp] = byte(total, 0) + byte(total, 1) + byte(total, 2) + byte(total, 3);
   __syncthreads();
-  int run = tile_base[blockIdx.x] + incl - local;
-  for (int w = 0; w < warp; w++) run += warp_sum[w];
-  int o[kScanPerThread];
+  int run = tile_base;
 #pragma unroll
-  for (int q = 0; q < kScanPerThread; q++) {
-    o[q] = run;
-    run += v[q];
-  }
-  if (base + kScanPerThread <= n && ((uintptr_t)(offsets + base) & 15) == 0) {
-    int4* dst = reinterpret_cast<int4*>(offsets + base);  // this thread's 64 contiguous bytes
+  for (int v = 0; v < kScanThreads / 32; v++)
+    if (v < warp) run += warp_sum[v];
+  incl -= local;  // exclusive, byte by byte: no borrow
 #pragma unroll
-    for (int q = 0; q < kScanPerThread / 4; q++) dst[q] = make_int4(o[4 * q], o[4 * q + 1], o[4 * q + 2], o[4 * q + 3]);
-  } else {
-#pragma unroll
-    for (int q = 0; q < kScanPerThread; q++)
-      if (base + q < n) offsets[base + q] = o[q];
+  for (int k = 0; k < kPasses; k++) {
+    const int64_t i = base + 128 * k;
+    const int o0 = run + byte(incl, k), o1 = o0 + (int)(w[k] & 1u);
+    const int o2 = o1 + (int)((w[k] >> 8) & 1u), o3 = o2 + (int)((w[k] >> 16) & 1u);
+    if (aligned && i + 4 <= n) {
+      *reinterpret_cast<int4*>(offsets + i) = make_int4(o0, o1, o2, o3);
+    } else {
+      if (i < n) offsets[i] = o0;
+      if (i + 1 < n) offsets[i + 1] = o1;
+      if (i + 2 < n) offsets[i + 2] = o2;
+      if (i + 3 < n) offsets[i + 3] = o3;
+    }
+    run += byte(total, k);
   }
 }
 
@@ -222,65 +255,90 @@ __global__ void __launch_bounds__(256) k_feature_query(FeatArgs a) {
   }
 }
 
-// The same gather with 16-byte moves, for feature rows whose bytes are a
-// multiple of 16 (F = 32 fp16 or fp32 features, the Aggregator's width): the
-// two half-warps serve two valid samples at a time, each lane moving 16-byte
-// chunks of the feature rows (fp16 chunks widened to two float4 stores) and
-// loading its two chunks or elements before storing either, so a pair of
-// samples waits on one round of gathers.
+// Four features, as the gather moves them: one float4 out.
 template <int kHalf>
-__global__ void __launch_bounds__(256) k_feature_query_vec(FeatArgs a) {
-  constexpr int kEsz = kHalf ? 2 : 4;
-  const unsigned kAll = 0xffffffffu;
-  const int lane = threadIdx.x & 31, hl = lane & 15, half = lane >> 4;
-  const int64_t i0 = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * 32;
-  if (i0 >= a.n_samples) return;
-  const int64_t my = i0 + lane;
-  const bool valid = my < a.n_samples && a.mask[my] != 0;
-  unsigned todo = __ballot_sync(kAll, valid);
-  const int my_off = valid ? a.offsets[my] : 0;
+struct FeatPiece {
+  using type = float4;
+};
+template <>
+struct FeatPiece<1> {
+  using type = uint2;
+};
+
+// The same gather with 16-byte stores, for feature rows whose bytes are a
+// multiple of 16 (F = 32 fp16 or fp32 features, the Aggregator's width).
+//
+// Bound by how many gathers are in flight.  A block lists the valid ones of its
+// 128 samples, so that its warps share them evenly however the mask clumps, and
+// eight lanes serve a sample: nine words of the point attributes and kPieces
+// feature pieces a lane are loaded before any is stored (at P = 8 and F = 32 one
+// round each; the fp16 pieces are 8-byte loads, whose widened stores fill whole
+// lines).  What a sample has one of (position, ray direction with its divisions)
+// is done by a thread a sample beforehand.  The outputs are stored past the L2's
+// table (streaming).  613k samples of 8 points with 32 fp16 features from 1M
+// points, the whole call: 304 us when a warp served its own 32 samples in pairs
+// with both halves' loads two deep, 256 with 16 lanes a sample, 252 so;
+// one lane a word, or ids fetched a sample ahead, made it 310 to 357 (less in
+// flight, fewer warps).
+constexpr int kVecBlock = 128;
+template <int kHalf>
+__global__ void __launch_bounds__(kVecBlock, 12) k_feature_query_vec(FeatArgs a) {
+  using Piece = typename FeatPiece<kHalf>::type;
+  constexpr int kPieces = kHalf ? 8 : 4;  // 16 registers either way
+  __shared__ uint8_t list[kVecBlock];  // the block's valid samples in order
+  __shared__ int rows[kVecBlock];     // and their output rows
+  __shared__ int counts[kVecBlock / 32];
+  const int lane = threadIdx.x & 31, hl = lane & 7, warp = threadIdx.x >> 5;
+  const int64_t i0 = (int64_t)blockIdx.x * kVecBlock;
+  const bool valid = i0 + threadIdx.x < a.n_samples && a.mask[i0 + threadIdx.x] != 0;
+  const unsigned votes = __ballot_sync(0xffffffffu, valid);
+  if (lane == 0) counts[warp] = __popc(votes);
+  __syncthreads();
+  int before = 0, n_valid = 0;
+#pragma unroll
+  for (int w = 0; w < kVecBlock / 32; w++) {
+    if (w < warp) before += counts[w];
+    n_valid += counts[w];
+  }
+  if (valid) {  // what a sample has one of: a thread each, the warp's together
+    const int k = before + __popc(votes & ((1u << lane) - 1));
+    list[k] = (uint8_t)threadIdx.x;
+    const int64_t i = i0 + threadIdx.x, m = a.offsets[i];
+    rows[k] = (int)m;
+    const unsigned ray = (unsigned)i / (unsigned)a.S;  // sample counts are below 2^31: 32-bit division
+    int u, v;
+    if (a.ray_uv) {
+      u = a.ray_uv[2 * (int64_t)ray];
+      v = a.ray_uv[2 * (int64_t)ray + 1];
+    } else {
+      v = (int)(ray / (unsigned)a.width);
+      u = (int)(ray - (unsigned)v * (unsigned)a.width);
+    }
+    const float dx = __fdiv_rn(__fsub_rn((float)u, a.cx), a.fx);
+    const float dy = __fdiv_rn(__fsub_rn((float)v, a.cy), a.fy);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const float* R = a.c2w + 4 * c;
+      a.o_rays[m * 3 + c] = __fadd_rn(__fadd_rn(__fmul_rn(dx, R[0]), __fmul_rn(dy, R[1])), R[2]);
+      a.o_sp[m * 3 + c] = a.sp_xyz[i * 3 + c];
+    }
+  }
+  __syncthreads();
   const int P = a.P, F = a.feat_dim;
-  const int cpp = F * kEsz / 16;  // 16-byte chunks per feature row
+  const int cpp = F / 4;  // pieces (four features) per feature row
   const int cshift = (cpp & (cpp - 1)) == 0 ? __ffs(cpp) - 1 : -1;  // log2(cpp) when a power of two
   const int nch = P * cpp;
   const char* feat = reinterpret_cast<const char*>(a.feat);
-  while (todo) {
-    const int l0 = __ffs(todo) - 1;
-    todo &= todo - 1;
-    int l1 = -1;
-    if (todo) {
-      l1 = __ffs(todo) - 1;
-      todo &= todo - 1;
-    }
-    const int l = half ? l1 : l0;
-    const int64_t m = __shfl_sync(kAll, my_off, l < 0 ? 0 : l);
-    if (l < 0) continue;
-    const int64_t i = i0 + l;
-    const int* ids = a.pc_idx + i * P;  // the same few words for the half-warp (L1)
-    if (hl < 3) a.o_sp[m * 3 + hl] = a.sp_xyz[i * 3 + hl];
-    if (hl >= 3 && hl < 6) {
-      const int c = hl - 3;
-      const unsigned ray = (unsigned)i / (unsigned)a.S;  // sample counts are below 2^31: 32-bit division
-      int u, v;
-      if (a.ray_uv) {
-        u = a.ray_uv[2 * (int64_t)ray];
-        v = a.ray_uv[2 * (int64_t)ray + 1];
-      } else {
-        v = (int)(ray / (unsigned)a.width);
-        u = (int)(ray - (unsigned)v * (unsigned)a.width);
-      }
-      const float dx = __fdiv_rn(__fsub_rn((float)u, a.cx), a.fx);
-      const float dy = __fdiv_rn(__fsub_rn((float)v, a.cy), a.fy);
-      const float* R = a.c2w + 4 * c;
-      a.o_rays[m * 3 + c] = __fadd_rn(__fadd_rn(__fmul_rn(dx, R[0]), __fmul_rn(dy, R[1])), R[2]);
-    }
-    // xyz / rgb / dir rows: element e = (point, component), two per lane per pass
-    for (int e = hl; e < 3 * P; e += 32) {
-      float x[2], g[2], d[2];
-      bool ok[2];
+  for (int k = threadIdx.x >> 3; k < n_valid; k += kVecBlock / 8) {
+    const int64_t m = rows[k], i = i0 + list[k];
+    const int* ids = a.pc_idx + i * P;  // the same few words for the eight lanes (L1)
+    // xyz / rgb / dir rows: element e = (point, component), three per lane per pass
+    for (int e = hl; e < 3 * P; e += 24) {
+      float x[3], g[3], d[3];
+      bool ok[3];
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int ee = e + 16 * h;
+      for (int h = 0; h < 3; h++) {
+        const int ee = e + 8 * h;
         x[h] = g[h] = d[h] = 0.0f;
         ok[h] = false;
         if (ee < 3 * P) {
@@ -295,47 +353,43 @@ __global__ void __launch_bounds__(256) k_feature_query_vec(FeatArgs a) {
         }
       }
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int ee = e + 16 * h;
+      for (int h = 0; h < 3; h++) {
+        const int ee = e + 8 * h;
         if (ee < 3 * P) {
           const int p = ee / 3, c = ee - 3 * p;
           if (c == 0) a.o_valid[m * P + p] = ok[h];
           const int64_t o = (m * P + p) * 3 + c;
-          a.o_xyz[o] = x[h];
-          a.o_rgb[o] = g[h];
-          a.o_dir[o] = d[h];
+          __stcs(a.o_xyz + o, x[h]);
+          __stcs(a.o_rgb + o, g[h]);
+          __stcs(a.o_dir + o, d[h]);
         }
       }
     }
-    // feature rows: chunk q of point p, two per lane per pass
+    // feature rows: piece q of point p, kPieces per lane in flight; each store instruction covers whole lines
     float* of = a.o_feat + m * P * F;
-    for (int c = hl; c < nch; c += 32) {
-      uint4 v[2];
+    for (int c = hl; c < nch; c += 8 * kPieces) {
+      Piece v[kPieces];
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int cc = c + 16 * h;
-        v[h] = make_uint4(0u, 0u, 0u, 0u);
+      for (int h = 0; h < kPieces; h++) {
+        const int cc = c + 8 * h;
+        v[h] = Piece{};
         if (cc < nch) {
           const int p = cshift >= 0 ? cc >> cshift : cc / cpp, q = cc - p * cpp;
           const int id = ids[p];
           if ((unsigned)id < (unsigned)a.n_points)
-            v[h] = __ldg(reinterpret_cast<const uint4*>(feat + ((int64_t)id * cpp + q) * 16));
+            v[h] = __ldg(reinterpret_cast<const Piece*>(feat) + ((int64_t)id * cpp + q));
         }
       }
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int cc = c + 16 * h;
-        if (cc < nch) {
-          const int p = cshift >= 0 ? cc >> cshift : cc / cpp, q = cc - p * cpp;
+      for (int h = 0; h < kPieces; h++) {
+        const int cc = c + 8 * h;
+        if (cc < nch) {  // piece cc of the sample's rows is its floats 4 cc .. + 3
           if constexpr (kHalf) {
             const __half2* hh = reinterpret_cast<const __half2*>(&v[h]);
-            const float2 f0 = __half22float2(hh[0]), f1 = __half22float2(hh[1]), f2 = __half22float2(hh[2]),
-                         f3 = __half22float2(hh[3]);
-            float4* dst = reinterpret_cast<float4*>(of + p * F + q * 8);
-            dst[0] = make_float4(f0.x, f0.y, f1.x, f1.y);
-            dst[1] = make_float4(f2.x, f2.y, f3.x, f3.y);
+            const float2 f0 = __half22float2(hh[0]), f1 = __half22float2(hh[1]);
+            __stcs(reinterpret_cast<float4*>(of) + cc, make_float4(f0.x, f0.y, f1.x, f1.y));
           } else {
-            *reinterpret_cast<uint4*>(of + p * F + q * 4) = v[h];
+            __stcs(reinterpret_cast<float4*>(of) + cc, v[h]);
           }
         }
       }
@@ -496,9 +550,13 @@ extern "C" int32_t hp_mask_scan(const uint8_t* mask, int64_t n, int32_t* offsets
   }
   k_mask_tile_counts<<<tiles, kScanThreads, 0, st>>>(mask, n, tile);
   if (int32_t rc = check_launch("k_mask_tile_counts")) return rc;
+  if (tiles <= kSumTiles) {
+    k_mask_offsets<true><<<tiles, kScanThreads, 0, st>>>(mask, n, tile, offsets, count);
+    return check_launch("k_mask_offsets");
+  }
   k_mask_scan_tiles<<<1, 1024, 0, st>>>(tile, tiles, count);
   if (int32_t rc = check_launch("k_mask_scan_tiles")) return rc;
-  k_mask_offsets<<<tiles, kScanThreads, 0, st>>>(mask, n, tile, offsets);
+  k_mask_offsets<false><<<tiles, kScanThreads, 0, st>>>(mask, n, tile, offsets, count);
   return check_launch("k_mask_offsets");
 }
 
@@ -553,9 +611,9 @@ extern "C" int32_t hp_feature_query(const hp_point_attrs* pts, const float* sp_x
   const bool vec = a.feat_dim > 0 && (a.feat_dim * esz) % 16 == 0 && ((uintptr_t)a.feat & 15) == 0 &&
                    ((uintptr_t)a.o_feat & 15) == 0;
   if (vec && a.feat_half)
-    k_feature_query_vec<1><<<(unsigned)((warps + 7) / 8), 256, 0, (cudaStream_t)stream>>>(a);
+    k_feature_query_vec<1><<<(unsigned)((a.n_samples + kVecBlock - 1) / kVecBlock), kVecBlock, 0, (cudaStream_t)stream>>>(a);
   else if (vec)
-    k_feature_query_vec<0><<<(unsigned)((warps + 7) / 8), 256, 0, (cudaStream_t)stream>>>(a);
+    k_feature_query_vec<0><<<(unsigned)((a.n_samples + kVecBlock - 1) / kVecBlock), kVecBlock, 0, (cudaStream_t)stream>>>(a);
   else
     k_feature_query<<<(unsigned)((warps + 7) / 8), 256, 0, (cudaStream_t)stream>>>(a);
   return check_launch("k_feature_query");

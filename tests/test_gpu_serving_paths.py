@@ -137,3 +137,42 @@ def test_clamp_t_any_shape(rays, S, off):
     d = torch.cat([t[:, 1:] - t[:, :-1], torch.full_like(t[:, :1], 0.004)], 1)
     m = ((d < 1e-8) | (d > 2 * torch.tensor(0.004, device="cuda"))).float()
     assert torch.equal(ops.clamp_t(t, 0.004), d * (1 - m) + m * 0.004)
+
+
+# a tile is 4096 entries; 4096 tiles are the most whose counts each block adds up itself
+@pytest.mark.parametrize("n", [1, 3, 511, 4096, 4099, 300_001, 4096 * 4096, 4096 * 4096 + 5])
+@pytest.mark.parametrize("shift", [0, 1, 4])
+def test_mask_scan_any_size(n, shift):
+    """Byte-exact exclusive scan: aligned and unaligned masks, any nonzero byte set, either side of the tile limit."""
+    g = torch.Generator(device="cuda").manual_seed(n + shift)
+    m = torch.randint(0, 5, (n + shift,), device="cuda", generator=g, dtype=torch.uint8)[shift:]
+    offsets, count = ops.mask_scan(m)
+    incl = (m != 0).cumsum(0)
+    assert torch.equal(offsets.long(), incl - (m != 0).long()) and int(count) == int(incl[-1])
+
+
+@pytest.mark.parametrize("half", [False, True])
+@pytest.mark.parametrize("rays,S,P,F", [(1, 1, 1, 8), (43, 3, 3, 32), (127, 1, 8, 32), (129, 8, 8, 32), (60, 5, 11, 40),
+                                        (33, 4, 17, 64), (300, 2, 40, 8)])
+def test_feature_gather_paths_agree(rays, S, P, F, half):
+    """Rows a multiple of 16 bytes take the wide gather; the same rows from an unaligned base take the general one."""
+    rng = np.random.default_rng(rays * 100 + P)
+    n, dev = 500, "cuda"
+    T = lambda *s: torch.from_numpy(rng.standard_normal(s).astype(np.float32)).to(dev)
+    xyz, rgb, dir_, sp = T(n, 3), T(n, 3), T(n, 3), T(rays, S, 3)
+    feat = T(n, F).to(torch.float16 if half else torch.float32)
+    odd = torch.empty(n * F + 1, dtype=feat.dtype, device=dev)[1:].view(n, F)
+    odd.copy_(feat)
+    ids = torch.from_numpy(rng.integers(-1, n, (rays, S, P)).astype(np.int32)).to(dev)
+    mask = torch.from_numpy(rng.random((rays, S)) < 0.4).to(dev)
+    mask[-1, -1] = True
+    uv = torch.from_numpy(rng.integers(0, 90, (rays, 2)).astype(np.int32)).to(dev)
+    for ray_uv in (None, uv):
+        call = lambda f: ops.feature_query(xyz, rgb, dir_, f, sp, ids, mask, T_c2w, 80.0, 81.0, 20.0, 21.0, 37, ray_uv)
+        T_c2w = torch.eye(4, device=dev) + 0.1 * torch.arange(16, device=dev, dtype=torch.float32).view(4, 4)
+        wide, general = call(feat), call(odd)
+        assert all(torch.equal(a, b) for a, b in zip(wide, general))
+        assert torch.equal(wide[4], sp[mask])
+        sel = ids[mask].long()
+        want = torch.where((sel >= 0)[..., None], feat.float()[sel.clamp(min=0)], torch.zeros((), device=dev))
+        assert torch.equal(wide[3], want) and torch.equal(wide[5], sel >= 0)
