@@ -17,10 +17,11 @@
 //                     per entry; -1 into the off-image tail of the outputs
 //   k_order           one thread per bucket entry: its rank among its bucket's
 //                     entries gives its final position (buckets <= 2048)
-//   k_sort_huge_list  buckets above 2048 entries, which k_scan_hash lists as
-//                     it writes the table: one CTA each, bitonic sort in place
-//                     in global memory (k_sort_huge_scan finds them by
-//                     scanning the table where there is no workspace)
+//                     and, before that, buckets above 2048 entries, which
+//                     k_scan_hash lists as it writes the table: one CTA each,
+//                     bitonic sort in place in global memory
+//                     (k_sort_huge_scan finds them by scanning the table where
+//                     there is no workspace)
 //
 // The atomic slots make the order inside a bucket arbitrary; ranking restores
 // the reference's order: ascending point id (the stable sort's order) when
@@ -43,6 +44,7 @@ constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 4;                    // counts per thread in the scan
 constexpr int kScanTile = kScanThreads * kScanItems;
 constexpr int kHugeThreads = 512;
+constexpr int kOrderThreads = 512;
 // Look-back words of the scan: a status bit above the tile's total in the
 // low 32 bits (0 = not yet published).
 constexpr unsigned long long kAggregate = 1ull << 62;
@@ -156,7 +158,7 @@ __device__ __forceinline__ int block_reduce_sum(int v, int* sh) {
 // reports (the table is then wrong; this does not happen while the tiles it
 // waits on are running).  `withhold` >= 0 names a tile that never publishes
 // its total, so that a test can make the others give up.  Also lists the pixels whose
-// buckets exceed kRankMax (count in scalars[1]), for k_sort_huge_list.
+// buckets exceed kRankMax (count in scalars[1]), for k_order.
 // scalars[2]: the tile counter; scalars[0]: the points inside the image.
 __global__ void __launch_bounds__(kScanThreads) k_scan_hash(const int* __restrict__ counts, int hw, int chunks_per_tile,
                                                             unsigned long long* __restrict__ look,
@@ -338,44 +340,6 @@ struct SplitEntries {
   __device__ __forceinline__ int id_at(int j) const { return __ldg(id + j); }
 };
 
-// One thread per entry j < n_in of the scratch copy: rank among the entries of
-// its bucket -> final position.  Buckets of one entry are copied; buckets above
-// kRankMax are left to k_sort_huge_list / k_sort_huge_scan.  The order mode
-// is a template argument so that the rank loop -- the kernel's instructions
-// are mostly its iterations -- compares ids alone when ordering by id.
-template <class Entries, int kByDepth, int kByPosition>
-__global__ void __launch_bounds__(256) k_order(Entries in, const int2* __restrict__ hash, int hw,
-                                               const int* __restrict__ scalars, int n_fixed,
-                                               int* __restrict__ out_idx, float* __restrict__ out_depth) {
-  const BucketOrder bo{kByDepth, kByPosition};
-  const int n_in = n_fixed >= 0 ? n_fixed : scalars[0];
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n_in; j += gridDim.x * blockDim.x) {
-    int2 h, e;
-    if (!in.entry(j, hash, hw, h, e)) continue;
-    // a bucket inside [0, n_in) -- always, unless the scan gave up waiting (hp_pts2plane_status),
-    // when the scratch may hold records no point wrote: then outputs are wrong but stay in bounds
-    if (h.x < 0 || h.y < 1 || h.y > n_in - h.x) continue;
-    if (h.y > kRankMax) continue;
-    const float d = __int_as_float(e.y);
-    int pos = h.x;
-    if (h.y > 1) {
-      int rank = 0;
-      if constexpr (!kByDepth && !kByPosition) {
-        for (int q = h.x; q < h.x + h.y; q++) rank += in.id_at(q) < e.x;
-      } else {
-        const unsigned long long kj = entry_key(bo, e.x, d, j);
-        for (int q = h.x; q < h.x + h.y; q++) {
-          const int2 eq = in.id_depth(q);
-          rank += entry_key(bo, eq.x, __int_as_float(eq.y), q) < kj;
-        }
-      }
-      pos += rank;
-    }
-    out_idx[pos] = e.x;
-    out_depth[pos] = d;
-  }
-}
-
 // Compare-exchange of positions i < l (ascending) in a bucket of c entries;
 // positions >= c act as +inf and are never touched (the "flip" bitonic
 // variant compares only towards the larger index, ascending).  While sorting,
@@ -397,7 +361,7 @@ __device__ __forceinline__ void cx_global(const BucketOrder& bo, int* idx, float
 // place in global memory after copying it from the scratch entries (indexed by
 // position).
 template <class Entries>
-__device__ __forceinline__ void sort_bucket(int2 h, Entries in, int* __restrict__ out_idx, float* __restrict__ out_depth,
+__device__ __noinline__ void sort_bucket(int2 h, Entries in, int* __restrict__ out_idx, float* __restrict__ out_depth,
                                             const BucketOrder& bo) {
   const int c = h.y;
   int* idx = out_idx + h.x;
@@ -431,15 +395,49 @@ __device__ __forceinline__ void sort_bucket(int2 h, Entries in, int* __restrict_
   __syncthreads();
 }
 
-// hp_pts2plane: the buckets k_scan_hash listed, one CTA each in turn.
-template <class Entries>
-__global__ void __launch_bounds__(kHugeThreads) k_sort_huge_list(const int* __restrict__ huge,
-                                                                 const int* __restrict__ scalars, Entries in,
-                                                                 const int2* __restrict__ hash,
-                                                                 int* __restrict__ out_idx,
-                                                                 float* __restrict__ out_depth, BucketOrder bo) {
-  const int n = scalars[1];
-  for (int q = blockIdx.x; q < n; q += gridDim.x) sort_bucket(hash[huge[q]], in, out_idx, out_depth, bo);
+// One thread per entry j < n_in of the scratch copy: rank among the entries of
+// its bucket -> final position.  Buckets of one entry are copied; buckets above
+// kRankMax come from the list `huge` (hp_pts2plane), one CTA each, or are left
+// to k_sort_huge_scan.  A launch of its own for that list cost every view 3 us
+// to find it empty (a build of 100k points, 48.3 -> 42.7 us with one memset
+// less); blocks of kOrderThreads sort a huge bucket as fast as it did (256
+// threads: 1.9x slower), and rank as fast as blocks of 256.  The order mode
+// is a template argument so that the rank loop -- the kernel's instructions
+// are mostly its iterations -- compares ids alone when ordering by id.
+template <class Entries, int kByDepth, int kByPosition>
+__global__ void __launch_bounds__(kOrderThreads) k_order(Entries in, const int2* __restrict__ hash, int hw,
+                                               const int* __restrict__ scalars, int n_fixed,
+                                               const int* __restrict__ huge, int* __restrict__ out_idx,
+                                               float* __restrict__ out_depth) {
+  const BucketOrder bo{kByDepth, kByPosition};
+  const int n_in = n_fixed >= 0 ? n_fixed : scalars[0];
+  const int n_huge = huge ? scalars[1] : 0;
+  for (int q = blockIdx.x; q < n_huge; q += gridDim.x) sort_bucket(hash[huge[q]], in, out_idx, out_depth, bo);
+  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n_in; j += gridDim.x * blockDim.x) {
+    int2 h, e;
+    if (!in.entry(j, hash, hw, h, e)) continue;
+    // a bucket inside [0, n_in) -- always, unless the scan gave up waiting (hp_pts2plane_status),
+    // when the scratch may hold records no point wrote: then outputs are wrong but stay in bounds
+    if (h.x < 0 || h.y < 1 || h.y > n_in - h.x) continue;
+    if (h.y > kRankMax) continue;
+    const float d = __int_as_float(e.y);
+    int pos = h.x;
+    if (h.y > 1) {
+      int rank = 0;
+      if constexpr (!kByDepth && !kByPosition) {
+        for (int q = h.x; q < h.x + h.y; q++) rank += in.id_at(q) < e.x;
+      } else {
+        const unsigned long long kj = entry_key(bo, e.x, d, j);
+        for (int q = h.x; q < h.x + h.y; q++) {
+          const int2 eq = in.id_depth(q);
+          rank += entry_key(bo, eq.x, __int_as_float(eq.y), q) < kj;
+        }
+      }
+      pos += rank;
+    }
+    out_idx[pos] = e.x;
+    out_depth[pos] = d;
+  }
 }
 
 // hp_scatter_hashtable (no workspace for a list): each CTA scans a contiguous
@@ -493,8 +491,8 @@ __global__ void __launch_bounds__(256) k_runs(const int* __restrict__ point_idx,
 // ---------------------------------------------------------------------------
 static constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// Scratch of hp_pts2plane.  The look-back words and the scalars are adjacent,
-// so one memset clears both.
+// Scratch of hp_pts2plane.  The scalars, the look-back words and the counts are
+// adjacent, so one memset clears them.
 struct BuildLayout {
   size_t counts, pid_slot, depth, tmp, huge, look, scalars, total;
 };
@@ -504,6 +502,10 @@ static constexpr BuildLayout build_layout(int64_t n, int64_t hw) {
   const int64_t tiles = nchunks < kScanMaxTiles ? nchunks : kScanMaxTiles;
   BuildLayout L{};
   size_t o = 0;
+  L.scalars = o;
+  o += 256;
+  L.look = o;
+  o += align256(sizeof(unsigned long long) * (size_t)(tiles > 0 ? tiles : 1));
   L.counts = o;
   o += align256(sizeof(int) * (size_t)(hw > 0 ? hw : 1));
   L.pid_slot = o;
@@ -514,11 +516,6 @@ static constexpr BuildLayout build_layout(int64_t n, int64_t hw) {
   o += align256(sizeof(int4) * (size_t)(n > 0 ? n : 1));
   L.huge = o;  // pixels of buckets above kRankMax entries: at most n / (kRankMax + 1)
   o += align256(sizeof(int) * (size_t)(n / (kRankMax + 1) + 1));
-  L.look = o;
-  o += sizeof(unsigned long long) * (size_t)(tiles > 0 ? tiles : 1);
-  o = align256(o);
-  L.scalars = o;
-  o += 256;
   L.total = o;
   return L;
 }
@@ -538,19 +535,16 @@ template <class Entries>
 static int32_t launch_order(int hw, int n_fixed, int n_grid, Entries in, const int2* hash, const int* scalars,
                             const int* huge, int* out_idx, float* out_depth, BucketOrder bo, cudaStream_t st) {
   if (n_grid > 0) {
-    const int g = grid_for(n_grid, 256);
+    const int g = grid_for(n_grid, kOrderThreads);
     if (!bo.by_depth && !bo.by_position)
-      k_order<Entries, 0, 0><<<g, 256, 0, st>>>(in, hash, hw, scalars, n_fixed, out_idx, out_depth);
+      k_order<Entries, 0, 0><<<g, kOrderThreads, 0, st>>>(in, hash, hw, scalars, n_fixed, huge, out_idx, out_depth);
     else if (!bo.by_position)
-      k_order<Entries, 1, 0><<<g, 256, 0, st>>>(in, hash, hw, scalars, n_fixed, out_idx, out_depth);
+      k_order<Entries, 1, 0><<<g, kOrderThreads, 0, st>>>(in, hash, hw, scalars, n_fixed, huge, out_idx, out_depth);
     else
-      k_order<Entries, 1, 1><<<g, 256, 0, st>>>(in, hash, hw, scalars, n_fixed, out_idx, out_depth);
+      k_order<Entries, 1, 1><<<g, kOrderThreads, 0, st>>>(in, hash, hw, scalars, n_fixed, huge, out_idx, out_depth);
     if (int32_t rc = check_launch("k_order")) return rc;
   }
-  if (huge) {
-    k_sort_huge_list<<<148, kHugeThreads, 0, st>>>(huge, scalars, in, hash, out_idx, out_depth, bo);
-    return check_launch("k_sort_huge_list");
-  }
+  if (huge) return HP_OK;  // k_order sorted those listed
   const int blocks = (hw + kHugeThreads - 1) / kHugeThreads < 148 * 2 ? (hw + kHugeThreads - 1) / kHugeThreads : 148 * 2;
   k_sort_huge_scan<<<blocks, kHugeThreads, 0, st>>>(hw, in, hash, out_idx, out_depth, bo);
   return check_launch("k_sort_huge_scan");
@@ -607,8 +601,8 @@ static int32_t pts2plane(const float* xyz, int64_t n_points, const hp_camera* ca
   int32_t fw, fi;
   hp_projection_rounding(n_points, &fw, &fi);
 
-  if (cudaMemsetAsync(counts, 0, sizeof(int) * hw, st) != cudaSuccess ||
-      cudaMemsetAsync(look, 0, L.total - L.look, st) != cudaSuccess)
+  static_assert(build_layout(1, 1).scalars == 0, "cleared from the start of the workspace");
+  if (cudaMemsetAsync(ws, 0, L.counts + sizeof(int) * hw, st) != cudaSuccess)
     return set_error(HP_ERR_CUDA, "hp_pts2plane: cudaMemsetAsync failed: %s", cudaGetErrorString(cudaGetLastError()));
   if (n > 0) {
     k_project_count<<<grid_for((n + 3) / 4, 256), 256, 0, st>>>(xyz, n, cam->w2c, cam->K, H, W, fw, fi, counts,

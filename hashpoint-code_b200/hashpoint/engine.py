@@ -113,9 +113,8 @@ class ViewPipeline:
         return self.sp_xyz, self.pc_idx, self.sp_t, self.mask
 
     # kernels each render() launches (hp_pts2plane: project/count, scan,
-    # scatter, order, huge-bucket sort; hp_quick_sampling: ray list with the
-    # packing, sampling)
-    KERNELS_PER_VIEW = 7
+    # scatter, order; hp_quick_sampling: ray list with the packing, sampling)
+    KERNELS_PER_VIEW = 6
 
 
 class ViewRing:
