@@ -39,9 +39,13 @@
 //                 26 -> 34% active (143,000 x 8: 1141 -> ~800 us).  Of that the
 //                 second tile gave 6%, the MMA loop run by a whole warp 15%
 //                 (one lane took 590 cycles a chunk of two 128-cycle MMAs), the
-//                 biases and alpha weights from shared memory 9%.  What is left
-//                 is each team's chain: inputs 6 k cycles, three epilogues 2 k
-//                 each, the last one 7 k, four layers 2.1 k each.
+//                 biases and alpha weights from shared memory 9%.  Then
+//                 warps 16 and 17 issuing by elect.sync with uniform operands:
+//                 a layer's wait 5.8 -> 4.5 k cycles, the whole forward of
+//                 143,000 x 8, colour branch included, 898 -> 761 us.  What is
+//                 left is each team's chain: inputs 4 k cycles, four layers of
+//                 about 4 k with the other team's in between, three epilogues
+//                 2 k each, the last one 8 k, the alphas 2 k.
 //   k_agg_color   one CTA = 128 samples: the colour-branch input tile arrives
 //                 with one bulk copy, three layers on the tensor cores, the
 //                 final 128->3 layer and the sigmoid on the CUDA cores.
@@ -491,63 +495,56 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_agg_pairs(AggArgs g, long l
   // the CTA's tiles blockIdx.x + i * gridDim.x; team i % 2 serves tile i
   const long long my_tiles = blockIdx.x < n_tiles ? (n_tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
   bool fail = false;
+  // a converged warp's wait: the same answer in every lane, also when one of them gives up
+  auto wait_warp = [&](uint64_t* b, unsigned parity) -> bool {
+    if (__all_sync(0xffffffffu, tc::mbar_try_wait(b, parity))) return true;
+    return __all_sync(0xffffffffu, wait_or_abort(b, parity, abort, g.wait_ns));
+  };
 
   if (warp == kLoadWarp) {
-    // ---- weight loads: W3b once, then each layer's chunks for one team's tile and again for the other's
-    if (lane == 0) {
-      if (!g.withhold_w3b) {
-        tc::mbar_arrive_expect_tx(&bar.w3b, kW3bBytes);
-        tc::bulk_load(W3b, g.packed + kW3bOff, kW3bBytes, &bar.w3b);
+    // ---- weight loads: W3b once, then each layer's chunks for one team's tile and again for the other's.
+    // A whole warp like the MMA issue: a stage is free for one chunk's MMAs only, so the time from its
+    // commit to the copy counts.
+    if (!g.withhold_w3b) tc::warp_bulk_load(W3b, g.packed + kW3bOff, kW3bBytes, &bar.w3b);
+    uint32_t q = 0;
+    each_layer(my_tiles, [&](int, int L) -> bool {
+      const uint8_t* src = g.packed + (size_t)pair_chunk0(L) * kChunkBytes;
+#pragma unroll
+      for (int kc = 0; kc < pair_chunks(L); kc++, q++) {
+        const uint32_t st = q % kStages;
+        if (q >= kStages && !wait_warp(&bar.empty[st], ((q / kStages) - 1) & 1)) return false;
+        tc::warp_bulk_load(stages + (size_t)st * kChunkBytes, src + (size_t)kc * kChunkBytes, kChunkBytes,
+                           &bar.full[st]);
       }
-      long long q = 0;
-      each_layer(my_tiles, [&](int, int L) -> bool {
-        const uint8_t* src = g.packed + (size_t)pair_chunk0(L) * kChunkBytes;
-        for (int kc = 0; kc < pair_chunks(L); kc++, q++) {
-          const int st = (int)(q % kStages);
-          if (q >= kStages && !wait_or_abort(&bar.empty[st], (unsigned)(((q / kStages) - 1) & 1), abort, g.wait_ns))
-            return false;
-          tc::mbar_arrive_expect_tx(&bar.full[st], kChunkBytes);
-          tc::bulk_load(stages + (size_t)st * kChunkBytes, src + (size_t)kc * kChunkBytes, kChunkBytes, &bar.full[st]);
-        }
-        return true;
-      });
-      // the last copy into each stage has landed before the CTA ends
-      for (long long d = q - 1; d >= 0 && d >= q - kStages; d--)
-        if (!tc::mbar_wait(&bar.full[d % kStages], (unsigned)((d / kStages) & 1))) fail = true;
-      if (!g.withhold_w3b && !tc::mbar_wait(&bar.w3b, 0)) fail = true;
-    }
-    __syncwarp();  // the warp's other lanes wait for lane 0 here, not at the block barrier
+      return true;
+    });
+    // the last copy into each stage has landed before the CTA ends
+    for (uint32_t d = q > kStages ? q - kStages : 0; d < q; d++)
+      if (!tc::mbar_wait(&bar.full[d % kStages], (d / kStages) & 1)) fail = true;
+    if (!g.withhold_w3b && !tc::mbar_wait(&bar.w3b, 0)) fail = true;
+    __syncwarp();
   } else if (warp == kMmaWarp) {
     // ---- MMA issue: layer L of team 0's tile, of team 1's, then layer L + 1.  The whole warp runs the
-    // loop, so that descriptors and barrier phases are warp-uniform; lane 0 issues.  (One lane running it
-    // took 590 cycles a chunk of two 128-cycle MMAs.)
+    // loop, so that descriptors and barrier phases are warp-uniform, and issues by elect.sync.  (A chunk of
+    // two 128-cycle MMAs took 590 cycles with one lane running the loop, 410 with the warp running it and
+    // lane 0 issuing in a branch.)
     const uint32_t idesc = tc::idesc_bf16(kAggRows, kPairN);
     const uint64_t w3b_desc = tc::smem_desc_plain(tc::smem_addr(W3b), 128u, 256u);
     const uint64_t b_base = tc::smem_desc_sw64(tc::smem_addr(stages));
     unsigned a_ph = 0;  // bit team: phase of its operand
     uint32_t q = 0;     // weight chunks consumed
-    // the same answer in every lane, also when one of them gives up
-    auto wait = [&](uint64_t* b, unsigned parity) -> bool {
-      return __all_sync(0xffffffffu, wait_or_abort(b, parity, abort, g.wait_ns));
-    };
-    bool ok = wait(&bar.w3b, 0);
+    bool ok = wait_warp(&bar.w3b, 0);
     // a chunk of K: two K = 16 steps of the operand at `a`
     auto chunk = [&](uint32_t acc, uint64_t a, bool first) -> bool {
       const uint32_t st = q % kStages;
-      if (!wait(&bar.full[st], (q / kStages) & 1)) return false;
-      if (lane == 0) {
-        const uint64_t b = b_base + st * (kChunkBytes >> 4);
-        tc::mma_bf16(acc, a, b, idesc, first ? 0u : 1u);
-        tc::mma_bf16(acc, a + 2, b + 2, idesc, 1u);
-        tc::mma_commit(&bar.empty[st]);
-      }
-      __syncwarp();
+      if (!wait_warp(&bar.full[st], (q / kStages) & 1)) return false;
+      tc::warp_mma2_commit(acc, a, b_base + st * (kChunkBytes >> 4), idesc, first ? 0u : 1u, &bar.empty[st]);
       q++;
       return true;
     };
     if (ok) {
       each_layer(my_tiles, [&](int team, int L) -> bool {
-        if (!(ok = wait(&bar.a_ready[team], (a_ph >> team) & 1))) return false;
+        if (!(ok = wait_warp(&bar.a_ready[team], (a_ph >> team) & 1))) return false;
         a_ph ^= 1u << team;
         tc::tc_fence_after();
         const uint32_t acc = tmem + (uint32_t)team * 256u;
@@ -557,20 +554,15 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_agg_pairs(AggArgs g, long l
         for (int kc = 0; kc < 256 / kPairChunkK && ok; kc++)
           ok = chunk(acc, a_base + (uint32_t)((kc >> 1) * (kAggRows * 128 / 16) + (kc & 1) * 4), kc == 0);
         if (ok && L == 0) ok = chunk(acc, a_tail, false);
-        if (lane == 0) {
-          if (ok && L == 2)  // block3.0's extra inputs (columns 256..271) times W3b
-            tc::mma_bf16(acc, a_tail, w3b_desc, idesc, 1u);
-          tc::mma_commit(&bar.acc_full[team]);
-        }
-        __syncwarp();
+        if (ok && L == 2)  // block3.0's extra inputs (columns 256..271) times W3b
+          tc::warp_mma_bf16(acc, a_tail, w3b_desc, idesc, 1u);
+        tc::warp_commit(&bar.acc_full[team]);
         return ok;
       });
     }
     if (!ok) fail = true;
-    if (lane == 0) {
-      tc::mma_commit(&bar.idle);
-      if (!tc::mbar_wait(&bar.idle, 0)) fail = true;
-    }
+    tc::warp_commit(&bar.idle);
+    if (!tc::mbar_wait(&bar.idle, 0)) fail = true;
     __syncwarp();
   } else {
     // ---- a team: inputs, epilogues, reductions of its tiles

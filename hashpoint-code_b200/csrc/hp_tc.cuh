@@ -151,6 +151,59 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
                : "memory");
 }
 
+// --- the same, called by a converged warp: one lane (the same each time) issues --
+// In a branch of one lane the operands of each tcgen05 or bulk instruction are
+// per-thread values that the warp has to move to uniform registers first; called
+// by the whole warp with elect.sync's predicate they are uniform to begin with
+// (two MMAs and their commit: 230 cycles in a branch, about 100 so).
+__device__ __forceinline__ void warp_mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                              uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+__device__ __forceinline__ void warp_commit(uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_addr(bar))
+      : "memory");
+}
+
+// Two K = 16 steps, 32 bytes apart in both operands, then a commit on bar.
+__device__ __forceinline__ void warp_mma2_commit(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                                 uint32_t accumulate, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred p, e, t;\n\t.reg .b64 a2, b2;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.eq.b32 t, 0, 0;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "add.s64 a2, %1, 2;\n\t"
+      "add.s64 b2, %2, 2;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], a2, b2, %3, t;\n\t"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n\t}" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(smem_addr(bar))
+      : "memory");
+}
+
+// mbar_arrive_expect_tx and bulk_load.
+__device__ __forceinline__ void warp_bulk_load(void* dst_smem, const void* src, unsigned bytes, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%3], %2;\n\t"
+      "@e cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n\t}" ::"r"(
+          smem_addr(dst_smem)),
+      "l"(src), "r"(bytes), "r"(smem_addr(bar))
+      : "memory");
+}
+
 // 32 consecutive fp32 columns of this thread's TMEM lane (the warp reads lanes
 // 32 * (warp % 4) .. + 31); taddr = base + (lane0 << 16) + column.  The wait
 // for the load is in the same asm statement: as a statement of its own it
