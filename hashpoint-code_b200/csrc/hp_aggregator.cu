@@ -46,9 +46,16 @@
 //                 left is each team's chain: inputs 4 k cycles, four layers of
 //                 about 4 k with the other team's in between, three epilogues
 //                 2 k each, the last one 8 k, the alphas 2 k.
-//   k_agg_color   one CTA = 128 samples: the colour-branch input tile arrives
-//                 with one bulk copy, three layers on the tensor cores, the
-//                 final 128->3 layer and the sigmoid on the CUDA cores.
+//   k_agg_color   one CTA = 128 samples at a time: three layers on the tensor
+//                 cores, the final 128->3 layer and the sigmoid on the CUDA
+//                 cores.  Its weights (144 KB) are loaded once and stay in
+//                 shared memory; the next tile's input columns 128.. are
+//                 loaded while this tile's hidden layers, whose operand is
+//                 columns 0..127, run, and the rest at its end.  A tile's
+//                 steps are one chain (load, layer, epilogue, ...), which
+//                 bounds the kernel.  143,000 samples, the whole forward: 761
+//                 us with the weights streamed for every tile, the load of its
+//                 inputs waited for and 8 warps, 710 so.
 //   k_agg_scatter alpha and colour of sample m to the m-th set position of
 //                 mask_out, zeros elsewhere.
 //
@@ -74,7 +81,7 @@ constexpr int kTeams = 2;                          // tiles in flight per CTA
 constexpr int kTeamThreads = 256;                  // math warps of a team
 constexpr int kMathThreads = kTeams * kTeamThreads;  // warps 0..15
 constexpr int kPairThreads = kMathThreads + 64;    // + MMA warp + load warp
-constexpr int kColorThreads = 256;
+constexpr int kColorThreads = 512;
 constexpr int kMmaWarp = 16, kLoadWarp = 17;
 constexpr int kPairChunkK = 32;                    // pair weight chunk: 256 outputs x 32 K, 64-byte swizzled
 constexpr int kChunkK = 64;                        // colour weight chunk: 128 outputs x 64 K, 128-byte swizzled
@@ -129,9 +136,10 @@ constexpr unsigned kPBar = kPW3b + kW3bBytes;
 constexpr unsigned kPScratch = kPBar + 256;
 constexpr unsigned kPParams = kPScratch + 2 * 4 * kAggRows * 4;  // block1.2 bias, block3.2 bias, alpha weights
 // colour kernel shared memory
-constexpr unsigned kCStages = kATileBytes;
-constexpr unsigned kCBar = kCStages + kStages * kChunkBytes;
-constexpr unsigned kCScratch = kCBar + 256;
+constexpr unsigned kCWeights = kATileBytes;                    // all of the branch's chunks, loaded once
+constexpr unsigned kCBar = kCWeights + (unsigned)kColorBytes;
+constexpr unsigned kCParams = kCBar + 256;                     // the 128->3 layer's weights
+constexpr unsigned kAHead = kAggRows * 256;                    // columns 0..127 of the operand: two blocks
 
 struct PairBars {
   uint64_t full[kStages];
@@ -161,16 +169,11 @@ struct PairScratch {           // of one team
   float apart[4][kAggRows];    // alpha-branch partial dot products (column quarters)
 };
 
-struct Ring {  // colour kernel: barriers and bookkeeping of one CTA's weight stream (thread 0)
-  uint64_t full[kStages];
-  uint64_t empty[kStages];
-  uint64_t done;   // all MMAs of a layer completed
-  uint64_t aload;  // colour-input tile landed
+struct ColorBars {
+  uint64_t w[kColorChunks];  // weight chunk c landed
+  uint64_t a;                // both parts of the input tile landed
+  uint64_t done;             // all MMAs of a layer completed
   uint32_t tmem;
-};
-
-struct ColorScratch {
-  float opart[2][kAggRows][4];
 };
 
 // Wait for a phase; gives up (and raises the CTA's abort flag) after limit_ns,
@@ -187,52 +190,6 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, unsigned parity, vo
       return false;
     }
   }
-}
-
-// Weight chunk stream of the colour kernel: chunk g of this CTA is packed chunk g % n_chunks.
-struct ChunkStream {
-  const uint8_t* base;
-  int n_chunks;
-  unsigned bytes;
-  long long issued, consumed, total;
-};
-
-__device__ __forceinline__ bool refill(ChunkStream& s, uint8_t* stages, Ring& ring) {
-  while (s.issued < s.total && s.issued < s.consumed + kStages - 1) {
-    const int st = (int)(s.issued % kStages);
-    if (s.issued >= kStages && !tc::mbar_wait(&ring.empty[st], (unsigned)(((s.issued / kStages) - 1) & 1)))
-      return false;
-    tc::mbar_arrive_expect_tx(&ring.full[st], s.bytes);
-    tc::bulk_load(stages + (size_t)st * s.bytes, s.base + (size_t)(s.issued % s.n_chunks) * s.bytes, s.bytes,
-                  &ring.full[st]);
-    s.issued++;
-  }
-  return true;
-}
-
-// One colour layer: D[tmem] = A (K wide) * W^T over K / 64 streamed chunks, then a
-// commit on ring.done.  Thread 0 only.
-__device__ __forceinline__ bool issue_layer(ChunkStream& s, uint8_t* stages, Ring& ring, uint32_t a_addr, int K,
-                                            uint32_t d_tmem, uint32_t idesc) {
-  bool ok = true;
-  for (int c = 0; c < K / kChunkK && ok; c++) {
-    const int st = (int)(s.consumed % kStages);
-    if (!tc::mbar_wait(&ring.full[st], (unsigned)((s.consumed / kStages) & 1))) {
-      ok = false;
-      break;
-    }
-    tc::tc_fence_after();
-    const uint32_t b_addr = tc::smem_addr(stages + (size_t)st * s.bytes);
-#pragma unroll
-    for (int j = 0; j < kChunkK / 16; j++)
-      tc::mma_bf16(d_tmem, tc::smem_desc_sw128(a_addr + (uint32_t)c * (kAggRows * 128) + (uint32_t)j * 32u),
-                   tc::smem_desc_sw128(b_addr + (uint32_t)j * 32u), idesc, (c > 0 || j > 0) ? 1u : 0u);
-    tc::mma_commit(&ring.empty[st]);
-    s.consumed++;
-    ok = refill(s, stages, ring);
-  }
-  tc::mma_commit(&ring.done);  // also on failure, so the other threads' wait ends
-  return ok;
 }
 
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
@@ -734,93 +691,134 @@ __global__ void __launch_bounds__(kColorThreads, 1) k_agg_color(AggArgs g, long 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   uint8_t* A = smem;
-  uint8_t* stages = smem + kCStages;
-  Ring& ring = *reinterpret_cast<Ring*>(smem + kCBar);
-  ColorScratch& sc = *reinterpret_cast<ColorScratch*>(smem + kCScratch);
+  ColorBars& bar = *reinterpret_cast<ColorBars*>(smem + kCBar);
+  float* s_wc = reinterpret_cast<float*>(smem + kCParams);
   const float* prm = reinterpret_cast<const float*>(g.packed + kParamOff);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid < 3 * kColorN) s_wc[tid] = prm[kPWC4 + tid];
 
   if (tid == 0) {
-    for (int i = 0; i < kStages; i++) {
-      tc::mbar_init(&ring.full[i], 1);
-      tc::mbar_init(&ring.empty[i], 1);
-    }
-    tc::mbar_init(&ring.done, 1);
-    tc::mbar_init(&ring.aload, 1);
+    for (int c = 0; c < kColorChunks; c++) tc::mbar_init(&bar.w[c], 1);
+    tc::mbar_init(&bar.a, 2);  // the tile's two parts
+    tc::mbar_init(&bar.done, 1);
     tc::mbar_init_fence();
   }
-  if (warp == 0) tc::tmem_alloc(&ring.tmem, 128);
+  if (warp == 0) tc::tmem_alloc(&bar.tmem, 128);
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
-  const uint32_t tmem = ring.tmem;
-  const long long my_tiles = blockIdx.x < n_tiles ? (n_tiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-  ChunkStream cs{g.packed + kColorOff, kColorChunks, kChunkBytes, 0, 0, my_tiles * kColorChunks};
-  bool fail = false;
-  if (tid == 0) fail = !refill(cs, stages, ring);
-  int stop = __syncthreads_or(fail);
-  unsigned done_phase = 0, a_phase = 0;
-  bool a_pending = false;
+  const uint32_t tmem = bar.tmem;
+  // warp 0 loads and issues: a tile's columns 0..127 (the hidden layers' operand too) and the rest apart
+  long long a_parts = 0, a_done = 0;  // loads issued (two a tile), tiles waited for
+  auto load_head = [&](long long t) {
+    tc::warp_bulk_load(A, g.color_in + (size_t)t * kATileBytes, kAHead, &bar.a);
+    a_parts++;
+  };
+  auto load_rest = [&](long long t) {
+    tc::warp_bulk_load(A + kAHead, g.color_in + (size_t)t * kATileBytes + kAHead, kATileBytes - kAHead, &bar.a);
+    a_parts++;
+  };
+  if (warp == 0 && blockIdx.x < n_tiles) {
+    load_head(blockIdx.x);
+    load_rest(blockIdx.x);
+    for (int c = 0; c < kColorChunks; c++)
+      tc::warp_bulk_load(smem + kCWeights + c * kChunkBytes, g.packed + kColorOff + (size_t)c * kChunkBytes,
+                         kChunkBytes, &bar.w[c]);
+  }
+  auto wait_warp = [&](uint64_t* b, unsigned parity) -> bool {
+    return __all_sync(0xffffffffu, tc::mbar_wait(b, parity));
+  };
   const uint32_t idesc = tc::idesc_bf16(kAggRows, kColorN);
-  const int er = 32 * (warp & 3) + lane, eh = warp >> 2;
+  const uint64_t a_base = tc::smem_desc_sw128(tc::smem_addr(A));
+  const uint64_t w_base = tc::smem_desc_sw128(tc::smem_addr(smem + kCWeights));
+  const int er = 32 * (warp & 3) + lane, cq = warp >> 2;  // row, column quarter
   const uint32_t lane_addr = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+  // the last layer's partial sums, in the operand (its last reader, that layer, has completed)
+  float(*opart)[kAggRows][4] = reinterpret_cast<float(*)[kAggRows][4]>(A);
+  unsigned done_phase = 0;
+  bool fail = false;
+  int stop = 0;
 
   for (long long t = blockIdx.x; t < n_tiles && !stop; t += gridDim.x) {
-    for (int L = 0; L < 3 && !stop; L++) {
-      if (tid == 0) {
+    const bool more = t + gridDim.x < n_tiles;
+    int chunk0 = 0;
+#pragma unroll
+    for (int L = 0; L < 3; L++) {
+      const int chunks = color_k(L) / kChunkK;
+      if (warp == 0) {
         bool ok = true;
-        if (L == 0) {  // this tile's inputs (the previous tile's MMAs have completed)
-          tc::mbar_arrive_expect_tx(&ring.aload, kATileBytes);
-          tc::bulk_load(A, g.color_in + (size_t)t * kATileBytes, kATileBytes, &ring.aload);
-          a_pending = true;
-          ok = tc::mbar_wait(&ring.aload, a_phase & 1);
-          if (ok) a_pending = false;
-          a_phase++;
+        if (L == 0) {
+          ok = wait_warp(&bar.a, (unsigned)a_done & 1);
+          a_done += ok;
         }
         tc::tc_fence_after();
-        if (!ok) {
-          fail = true;
-          tc::mma_commit(&ring.done);
-        } else if (!issue_layer(cs, stages, ring, tc::smem_addr(A), color_k(L), tmem, idesc)) {
-          fail = true;
+        for (int c = 0; c < chunks && ok; c++) {
+          if (t == blockIdx.x) ok = wait_warp(&bar.w[chunk0 + c], 0);
+          if (!ok) break;
+          // of the last input chunk (columns 256..319) the upper half is zeros on both sides
+          const int steps = L == 0 && c == chunks - 1 ? kChunkK / 32 : kChunkK / 16;
+          for (int j = 0; j < steps; j++)
+            tc::warp_mma_bf16(tmem, a_base + (uint32_t)(c * (kAggRows * 128 / 16) + 2 * j),
+                              w_base + (uint32_t)((chunk0 + c) * (kChunkBytes / 16) + 2 * j), idesc,
+                              (c > 0 || j > 0) ? 1u : 0u);
         }
+        if (!ok) fail = true;
+        tc::warp_commit(&bar.done);  // also on failure, so the other warps' wait ends
       }
-      if (!tc::mbar_wait(&ring.done, done_phase & 1)) fail = true;
+      chunk0 += chunks;
+      // the biases on their way while the layer runs: of 32 columns, 64 in the last layer's warps
+      const float4* bias = reinterpret_cast<const float4*>(prm + (L == 0 ? kPCB1 : L == 1 ? kPCB2 : kPCB3));
+      constexpr int kLast = kColorN / 2 / 4;
+      float4 b[kLast];
+      if (L < 2) {
+#pragma unroll
+        for (int q = 0; q < 8; q++) b[q] = __ldg(bias + 8 * cq + q);
+      } else if (cq < 2) {
+#pragma unroll
+        for (int q = 0; q < kLast; q++) b[q] = __ldg(bias + kLast * cq + q);
+      }
+      if (!tc::mbar_wait(&bar.done, done_phase & 1)) fail = true;
       done_phase++;
       tc::tc_fence_after();
-      const float* bias = prm + (L == 0 ? kPCB1 : L == 1 ? kPCB2 : kPCB3);
+      if (L == 0 && more && warp == 0 && !__any_sync(0xffffffffu, fail)) load_rest(t + gridDim.x);
       if (L < 2) {
-#pragma unroll 1
-        for (int cc = 0; cc < 2; cc++) {
-          const int col0 = 64 * eh + 32 * cc;
-          float v[32];
-          tc::tmem_ld32(lane_addr + (uint32_t)col0, v);
+        const int col0 = 32 * cq;
+        float v[32];
+        tc::tmem_ld32(lane_addr + (uint32_t)col0, v);
 #pragma unroll
-          for (int i = 0; i < 32; i++) v[i] = leaky(__fadd_rn(v[i], __ldg(bias + col0 + i)));
-#pragma unroll
-          for (int q = 0; q < 4; q++) store_unit(A, er, col0 / 8 + q, v + 8 * q);
+        for (int q = 0; q < 8; q++) {
+          v[4 * q] = leaky(__fadd_rn(v[4 * q], b[q].x));
+          v[4 * q + 1] = leaky(__fadd_rn(v[4 * q + 1], b[q].y));
+          v[4 * q + 2] = leaky(__fadd_rn(v[4 * q + 2], b[q].z));
+          v[4 * q + 3] = leaky(__fadd_rn(v[4 * q + 3], b[q].w));
         }
-      } else {
+#pragma unroll
+        for (int q = 0; q < 4; q++) store_unit(A, er, col0 / 8 + q, v + 8 * q);
+      } else if (cq < 2) {
         float o[3] = {0.0f, 0.0f, 0.0f};
-        const float* wc = prm + kPWC4;
-#pragma unroll 1
+#pragma unroll
         for (int cc = 0; cc < 2; cc++) {
-          const int col0 = 64 * eh + 32 * cc;
+          const int col0 = 64 * cq + 32 * cc;
           float v[32];
           tc::tmem_ld32(lane_addr + (uint32_t)col0, v);
 #pragma unroll
-          for (int i = 0; i < 32; i++) {
-            const float f = leaky(__fadd_rn(v[i], __ldg(bias + col0 + i)));
+          for (int q = 0; q < 8; q++) {
+            const float4 bq = b[8 * cc + q];
+            const float f0 = leaky(__fadd_rn(v[4 * q], bq.x)), f1 = leaky(__fadd_rn(v[4 * q + 1], bq.y));
+            const float f2 = leaky(__fadd_rn(v[4 * q + 2], bq.z)), f3 = leaky(__fadd_rn(v[4 * q + 3], bq.w));
 #pragma unroll
-            for (int j = 0; j < 3; j++) o[j] = __fmaf_rn(f, __ldg(wc + j * 128 + col0 + i), o[j]);
+            for (int j = 0; j < 3; j++) {
+              const float4 w = *reinterpret_cast<const float4*>(s_wc + j * kColorN + col0 + 4 * q);
+              o[j] = __fmaf_rn(f3, w.w, __fmaf_rn(f2, w.z, __fmaf_rn(f1, w.y, __fmaf_rn(f0, w.x, o[j]))));
+            }
           }
         }
-#pragma unroll
-        for (int j = 0; j < 3; j++) sc.opart[eh][er][j] = o[j];
+        *reinterpret_cast<float4*>(opart[cq][er]) = make_float4(o[0], o[1], o[2], 0.0f);
       }
       tc::tc_fence_before();
       tc::fence_async_smem();
       stop = __syncthreads_or(fail);
+      if (stop) break;
     }
     if (stop) break;
     if (tid < kAggRows) {
@@ -828,21 +826,25 @@ __global__ void __launch_bounds__(kColorThreads, 1) k_agg_color(AggArgs g, long 
       if (m < g.M) {
 #pragma unroll
         for (int j = 0; j < 3; j++) {
-          const float z = __fadd_rn(__fadd_rn(sc.opart[0][tid][j], sc.opart[1][tid][j]), prm[kPCB4 + j]);
+          const float z = __fadd_rn(__fadd_rn(opart[0][tid][j], opart[1][tid][j]), prm[kPCB4 + j]);
           const float s = 1.0f / (1.0f + expf(-z));
           g.color[m * 3 + j] = __fsub_rn(__fmul_rn(s, 1.002f), 0.001f);
         }
       }
     }
-    __syncthreads();
+    __syncthreads();  // opart is read
+    if (warp == 0 && more) load_head(t + gridDim.x);
   }
 
-  if (tid == 0) {
-    if (a_pending && !tc::mbar_wait(&ring.aload, (a_phase - 1) & 1)) fail = true;
-    for (long long q = cs.consumed; q < cs.issued; q++)
-      if (!tc::mbar_wait(&ring.full[q % kStages], (unsigned)((q / kStages) & 1))) fail = true;
-    tc::mma_commit(&ring.done);
-    if (!tc::mbar_wait(&ring.done, done_phase & 1)) fail = true;
+  if (warp == 0) {  // what was issued has completed before the CTA ends
+    if (a_parts % 2 && lane == 0) tc::mbar_arrive(&bar.a);  // gave up between a tile's two loads
+    __syncwarp();
+    if (a_parts > 2 * a_done && !tc::mbar_wait(&bar.a, (unsigned)a_done & 1)) fail = true;
+    if (blockIdx.x < n_tiles)
+      for (int c = 0; c < kColorChunks; c++)
+        if (!tc::mbar_wait(&bar.w[c], 0)) fail = true;
+    tc::warp_commit(&bar.done);
+    if (!tc::mbar_wait(&bar.done, done_phase & 1)) fail = true;
   }
   if (fail) atomicExch(g.status, 1);
   tc::tc_fence_before();
@@ -976,8 +978,8 @@ AggLayout agg_layout(long long M) {
 
 constexpr unsigned kPairSmem = kPParams + 3 * kPairN * 4 + 1024;
 static_assert(kTeams * sizeof(PairScratch) == kPParams - kPScratch, "scratch");
-constexpr unsigned kColorSmem = kCScratch + sizeof(ColorScratch) + 1024;
-static_assert(sizeof(PairBars) <= 256 && sizeof(Ring) <= 256, "barrier block");
+constexpr unsigned kColorSmem = kCParams + 3 * kColorN * 4 + 1024;
+static_assert(sizeof(PairBars) <= 256 && sizeof(ColorBars) <= 256, "barrier block");
 static_assert(kPairSmem <= 227 * 1024 && kColorSmem <= 227 * 1024, "shared memory");
 static_assert(kTeamThreads / 32 * kRedBytes <= kABytes && kABytes % 1024 == 0, "transpose buffers fit in A");
 }  // namespace

@@ -42,11 +42,6 @@ __device__ __forceinline__ void mbar_init_fence() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
-               : "memory");
-}
-
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
   uint32_t ok;
   asm volatile(
@@ -71,15 +66,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
     if (mbar_try_wait(bar, parity)) return true;
     if (global_ns() - t0 > kWaitNs) return false;
   }
-}
-
-// --- bulk copy (no tensor map; the issuing CTA is the only destination) -------
-// bytes: a multiple of 16; both addresses 16-byte aligned.
-__device__ __forceinline__ void bulk_load(void* dst_smem, const void* src, unsigned bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_addr(dst_smem)),
-               "l"(src), "r"(bytes), "r"(smem_addr(bar))
-               : "memory");
 }
 
 // Generic-proxy shared-memory writes -> visible to the async proxy (tcgen05.mma).
@@ -192,7 +178,8 @@ __device__ __forceinline__ void warp_mma2_commit(uint32_t d_tmem, uint64_t a_des
       : "memory");
 }
 
-// mbar_arrive_expect_tx and bulk_load.
+// Bulk copy (no tensor map; the issuing CTA is the only destination), counted by
+// bar.  bytes: a multiple of 16; both addresses 16-byte aligned.
 __device__ __forceinline__ void warp_bulk_load(void* dst_smem, const void* src, unsigned bytes, uint64_t* bar) {
   asm volatile(
       "{\n\t.reg .pred e;\n\t"

@@ -176,3 +176,23 @@ def test_feature_gather_paths_agree(rays, S, P, F, half):
         sel = ids[mask].long()
         want = torch.where((sel >= 0)[..., None], feat.float()[sel.clamp(min=0)], torch.zeros((), device=dev))
         assert torch.equal(wide[3], want) and torch.equal(wide[5], sel >= 0)
+
+
+@pytest.mark.parametrize("M", [128 * 148, 128 * 148 + 1, 2 * 128 * 148 + 5])
+def test_aggregator_tiles_agree(M):
+    """CTAs that serve several tiles one after another give what they give for one tile each, bit for bit."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    R = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    layers = [(R(o, i) / i ** 0.5, 0.1 * R(o)) for _, o, i in ops.AGG_LAYERS]
+    packed = ops.aggregator_pack([w for w, _ in layers], [b for _, b in layers])
+    P = 2
+    sp, rays = R(M, 3), R(M, 3)
+    ins = [sp[:, None] + 0.01 * R(M, P, 3), R(M, P, 3), R(M, P, 3), R(M, P, 32), sp, R(M, P) > -0.5]
+    call = lambda a, b: ops.aggregator_forward(packed, *[x[a:b].contiguous() for x in ins],
+                                               torch.ones((b - a, 1), dtype=torch.bool, device="cuda"),
+                                               rays[a:b].contiguous(), check_status=True)
+    alpha, color = call(0, M)
+    step = 128 * 64
+    parts = [call(a, min(M, a + step)) for a in range(0, M, step)]
+    assert torch.equal(alpha, torch.cat([p[0] for p in parts])) and torch.equal(color, torch.cat([p[1] for p in parts]))
+    assert torch.isfinite(color).all() and color.std() > 0
