@@ -42,7 +42,7 @@
 //                 biases and alpha weights from shared memory 9%.  Then
 //                 warps 16 and 17 issuing by elect.sync with uniform operands:
 //                 a layer's wait 5.8 -> 4.5 k cycles, the whole forward of
-//                 143,000 x 8, colour branch included, 898 -> 761 us.  What is
+//                 143,000 x 8, colour branch included, 898 -> 761 us (685 with the steps below).  What is
 //                 left is each team's chain: inputs 4 k cycles, four layers of
 //                 about 4 k with the other team's in between, three epilogues
 //                 2 k each, the last one 8 k, the alphas 2 k.
@@ -304,8 +304,10 @@ __device__ __forceinline__ void input_units(uint8_t* A, int r, const float* feat
   }
 }
 
-// A team's view of one tile's inputs: builds A; returns the aggregation weight of the thread's row.
-__device__ __forceinline__ float build_inputs(const AggArgs& g, long long t, int spt, uint8_t* A, int tid) {
+// A team's view of one tile's inputs: builds A; returns the aggregation weight of the
+// thread's row, and whether its point is valid.
+__device__ __forceinline__ float build_inputs(const AggArgs& g, long long t, int spt, uint8_t* A, int tid,
+                                              bool& valid) {
   const int P = g.P;
   const int r = tid & (kAggRows - 1), h = tid >> 7;  // h: which 18 of the row's 36 units
   const long long m = t * spt + r / P;
@@ -314,6 +316,7 @@ __device__ __forceinline__ float build_inputs(const AggArgs& g, long long t, int
   const long long e = m * P + p;
   float feat[kFeatDim], df[6];
   float inv = 0.0f;
+  valid = false;
 #pragma unroll
   for (int i = 0; i < kFeatDim; i++) feat[i] = 0.0f;
 #pragma unroll
@@ -333,7 +336,8 @@ __device__ __forceinline__ float build_inputs(const AggArgs& g, long long t, int
       df[3 + i] = __fsub_rn(__fmul_rn(x, x), __fmul_rn(s, s));
       d2 = __fmaf_rn(df[i], df[i], d2);
     }
-    if (__ldg(g.valid + e)) inv = __fdiv_rn(1.0f, __fadd_rn(sqrtf(d2), 1e-6f));
+    valid = __ldg(g.valid + e) != 0;
+    if (valid) inv = __fdiv_rn(1.0f, __fadd_rn(sqrtf(d2), 1e-6f));
   }
   // aggregation weight: inv / (sum over the sample's P rows + 1e-6); the rows are adjacent lanes
   float sum = inv;
@@ -529,6 +533,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_agg_pairs(AggArgs g, long l
     PairScratch& sc = reinterpret_cast<PairScratch*>(smem + kPScratch)[team];
     const uint32_t acc = tmem + (uint32_t)team * 256u + ((uint32_t)(32 * (warp & 3)) << 16);
     unsigned acc_ph = 0;
+    const float ba = __ldg(prm + kPBA);
     int stop = 0;
     auto ready = [&] {  // the operand is written and the accumulator read
       tc::tc_fence_before();
@@ -541,7 +546,8 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_agg_pairs(AggArgs g, long l
     };
     for (long long i = team; i < my_tiles && !stop; i += kTeams) {
       const long long t = blockIdx.x + i * gridDim.x;
-      const float w = build_inputs(g, t, spt, A, ttid);  // of row er, which is the row the thread built
+      bool valid;
+      const float w = build_inputs(g, t, spt, A, ttid, valid);  // of row er, which is the row the thread built
       ready();
       // layer 1 (its bias: column 284 of the inputs)
       layer();
@@ -553,16 +559,40 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_agg_pairs(AggArgs g, long l
         const long long m = t * spt + er / P;
         const long long e = m * P + er % P;
         if (er < spt * P && m < g.M) {
-          float dot = 0.0f;
+          float dot = 0.0f, ray[3];
 #pragma unroll
           for (int c = 0; c < 3; c++) {
             const float dv = __ldg(g.pc_dir + e * 3 + c), rd = __ldg(g.rays_d + m * 3 + c);
+            ray[c] = rd;
             ex[c] = __ldg(g.pc_rgb + e * 3 + c);
             ex[3 + c] = __fsub_rn(dv, rd);
             dot = c == 0 ? __fmul_rn(dv, rd) : __fmaf_rn(dv, rd, dot);
           }
           ex[6] = dot;
           ex[7] = 1.0f;  // its W3b column holds block3.0's bias
+          // The colour row's ray columns, PE(ray_d, 4) -> 256..279 and zeros to 319: here, while layer 2 runs.
+          // At the tile's end they waited for the ray again, and the alphas below for the valid flags: 710 us
+          // a forward of 143,000 x 8, 685 so.
+          if (er % P == 0) {
+            uint8_t* crow = g.color_in + (size_t)(m / kAggRows) * kATileBytes;
+            const int cr = (int)(m % kAggRows);
+            float s4[3][4], c4[3][4];
+#pragma unroll
+            for (int c = 0; c < 3; c++) bands<4>(ray[c], s4[c], c4[c]);
+#pragma unroll
+            for (int u = 0; u < 3; u++) {
+              float v[8];
+#pragma unroll
+              for (int c = 0; c < 4; c++) {
+                const int a = 4 * u + c;
+                v[2 * c] = s4[a / 4][a % 4];
+                v[2 * c + 1] = c4[a / 4][a % 4];
+              }
+              store_unit(crow, cr, 32 + u, v);
+            }
+#pragma unroll
+            for (int u = 35; u < 40; u++) zero_unit(crow, cr, u);
+          }
         }
       }
       layer();
@@ -628,27 +658,6 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_agg_pairs(AggArgs g, long l
           }
           __syncwarp();
         }
-        const long long m = t * spt + er / P;
-        if (cq == 1 && er % P == 0 && er < spt * P && m < g.M) {  // PE(ray_d, 4) -> columns 256..279, zeros to 319
-          uint8_t* crow = g.color_in + (size_t)(m / kAggRows) * kATileBytes;
-          const int cr = (int)(m % kAggRows);
-          float s4[3][4], c4[3][4];
-#pragma unroll
-          for (int c = 0; c < 3; c++) bands<4>(__ldg(g.rays_d + m * 3 + c), s4[c], c4[c]);
-#pragma unroll
-          for (int u = 0; u < 3; u++) {
-            float v[8];
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-              const int a = 4 * u + c;
-              v[2 * c] = s4[a / 4][a % 4];
-              v[2 * c + 1] = c4[a / 4][a % 4];
-            }
-            store_unit(crow, cr, 32 + u, v);
-          }
-#pragma unroll
-          for (int u = 35; u < 40; u++) zero_unit(crow, cr, u);
-        }
       }
       tc::tc_fence_before();
       stop = tc::named_sync_or(fail || *abort, 1 + team, kTeamThreads);
@@ -660,9 +669,9 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_agg_pairs(AggArgs g, long l
         const int p = r % P;
         const bool in = r < spt * P && m < g.M;
         float a = 0.0f;
-        if (in && __ldg(g.valid + m * P + p)) {
+        if (valid) {
           const float z = __fadd_rn(__fadd_rn(__fadd_rn(sc.apart[0][r], sc.apart[1][r]),
-                                              __fadd_rn(sc.apart[2][r], sc.apart[3][r])), prm[kPBA]);
+                                              __fadd_rn(sc.apart[2][r], sc.apart[3][r])), ba);
           a = softplus(__fsub_rn(z, 1.0f));
         }
         float x = __fmul_rn(a, w);
