@@ -115,6 +115,7 @@ __device__ __forceinline__ float4 load_point(const float* __restrict__ xyz, int 
 // without the square root whenever e2 is outside a band of relative width
 // 2^-16 around radius^2 -- far wider than the few-ulp errors of e2 and
 // norm3df -- and norm3df decides inside the band, so the result is identical.
+// A radius of zero, below zero or NaN keeps nothing: norm3df decides all.
 struct RadiusTest {
   float r, lo2, hi2;
   bool fast;  // else the band is everything
@@ -124,7 +125,7 @@ __host__ __device__ inline RadiusTest make_radius_test(float r) {
   RadiusTest rt;
   rt.r = r;
   const double r2 = (double)r * (double)r;
-  rt.fast = r2 > 1e-30 && r2 < 1e30;
+  rt.fast = r > 0.0f && r2 > 1e-30 && r2 < 1e30;
   rt.lo2 = rt.fast ? (float)(r2 * (1.0 - 1.0 / 65536.0)) : -1.0f;
   rt.hi2 = rt.fast ? (float)(r2 * (1.0 + 1.0 / 65536.0)) : INFINITY;
   return rt;
