@@ -649,6 +649,9 @@ __device__ __forceinline__ unsigned serve_rays(const SampleArgs& a, const int L,
                                                int entries) {
   constexpr unsigned kAll = 0xffffffffu;
   constexpr unsigned kCloseKeys = 512;  // of a float's bits: at least 2^-15 of its value
+  // The reference's "farthest" starts at 1e3: eight entries no nearer than that leave it there, and slot 0 the
+  // one to replace.  1e6 (a squared distance) less kCloseKeys, as bits:
+  constexpr unsigned kFarKey = 0x49742400u - kCloseKeys;
   constexpr int kSumBits = 21, kQuant = 10;  // histogram word: sum of distances in radius / 2^kQuant, count above;
                                              // 2^kQuant entries fit
   const int lane = threadIdx.x & 31;
@@ -939,6 +942,7 @@ __device__ __forceinline__ unsigned serve_rays(const SampleArgs& a, const int L,
               if (first && todo > kBallBuf) {
                 if (sl < kBallBuf) key = sk;
                 if (sl > 0 && sl < kBallBuf && sk - prev < kCloseKeys + kBallBuf) close = true;
+                if (least >= kFarKey) close = true;
                 limit = least;
               }
             }
