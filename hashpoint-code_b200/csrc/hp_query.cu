@@ -22,6 +22,11 @@ DevCamera dev_camera(const hp_camera* cam);
 DevOptions dev_options(const hp_options* o);
 
 constexpr int kQueryWarps = 4;
+#ifdef HP_TESTING
+constexpr unsigned kWindowMax = 64;  // so that small tables take several rounds a window
+#else
+constexpr unsigned kWindowMax = 0x7fffffffu;
+#endif
 constexpr int kQueryRays = 8;  // rays a warp serves in turn, their directions computed side by side
 
 // Bound by the latency of the dependent loads (bucket, id, point) and the
@@ -73,27 +78,31 @@ __global__ void __launch_bounds__(kQueryWarps * 32) k_quick_query(const float* _
     if (q + 1 < rays) ahead = bucket(__shfl_sync(kAll, my_ray, q + 1), 0);
     int* row = out + (r0 + q) * cap;
     int base = 0;
-    for (int c0 = 0; c0 < k2 && base < cap && ray >= 0; c0 += 32) {
+    for (int c0 = 0, cells = 32; c0 < k2 && base < cap && ray >= 0; c0 += cells) {
       if (c0 > 0) rg = bucket(ray, c0);
-      const int cnt = rg.y - rg.x;
-      int pre = cnt;
+      // Candidates are numbered in 32 bits.  Clamped windows repeat buckets and tables may overlap, so 32 cells can
+      // hold more than 2^31: then the round takes the cells before the one that reaches kWindowMax (at least one).
+      unsigned cnt = (unsigned)(rg.y - rg.x), pre = cnt;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(kAll, pre, o);
-        if (lane >= o) pre += t;
+        const unsigned t = __shfl_up_sync(kAll, pre, o);
+        if (lane >= o) pre = min(pre + t, kWindowMax);  // both below 2^31
       }
-      const int total = __shfl_sync(kAll, pre, 31);
+      const unsigned beyond = __ballot_sync(kAll, pre >= kWindowMax);
+      cells = beyond ? max(__ffs(beyond) - 1, 1) : 32;
+      const unsigned total = __shfl_sync(kAll, pre, cells - 1);
+      if (lane >= cells) cnt = 0, pre = total;
       pre -= cnt;
       const bool deep = __any_sync(kAll, cnt > kQueryPerCell);
       int carry = 0;  // lane c's copy: cell c's ids of earlier chunks
-      for (int j0 = 0; j0 < total && base < cap; j0 += 32) {
-        const int j = j0 + lane;
+      for (unsigned j0 = 0; j0 < total && base < cap; j0 += 32) {
+        const unsigned j = j0 + lane;
         int c = 0;
 #pragma unroll
         for (int s = 16; s > 0; s >>= 1)
           if (__shfl_sync(kAll, pre, c + s) <= j) c += s;
-        const int first = __shfl_sync(kAll, pre, c);
-        const int at = __shfl_sync(kAll, rg.x, c) + (j - first);
+        const unsigned first = __shfl_sync(kAll, pre, c);
+        const int at = __shfl_sync(kAll, rg.x, c) + (int)(j - first);
         int id = -1;
         float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
         if (j < total) {
@@ -108,8 +117,8 @@ __global__ void __launch_bounds__(kQueryWarps * 32) k_quick_query(const float* _
         bool in = within_radius(rt, id >= 0, squared(e0, e1, e2), e0, e1, e2);
         unsigned m = __ballot_sync(kAll, in);
         if (deep) {  // only a cell's first kQueryPerCell
-          const int before = __shfl_sync(kAll, carry, c) + __popc(m & below & ~lane_span(0, max(first - j0, 0)));
-          carry += __popc(m & lane_span(min(max(pre - j0, 0), 32), min(max(pre + cnt - j0, 0), 32)));
+          const int before = __shfl_sync(kAll, carry, c) + __popc(m & below & ~lane_span(0, max((int)(first - j0), 0)));
+          carry += __popc(m & lane_span(min(max((int)(pre - j0), 0), 32), min(max((int)(pre + cnt - j0), 0), 32)));
           in = in && before < kQueryPerCell;
           m = __ballot_sync(kAll, in);
         }

@@ -28,11 +28,12 @@ LIB_PATH = os.path.join(LIB_DIR, LIB_NAME)
 CUDA_HOME = os.environ.get("CUDA_HOME", "/usr/local/cuda")
 NVCC = os.path.join(CUDA_HOME, "bin", "nvcc")
 SOURCES = ["hp_api.cu", "hp_build.cu", "hp_sample.cu", "hp_query.cu", "hp_feature.cu", "hp_aggregator.cu"]
-# The test-only library (include/hashpoint_b200_testing.h): the tensor-core operand-form self-check and a
-# wait-expiry test of the Aggregator, compiled with the sources they exercise; never loaded by the product.
+# The test-only library (include/hashpoint_b200_testing.h): the tensor-core operand-form self-check, wait-expiry
+# tests of the Aggregator and the scan, and the search with windows of few candidates treated as those beyond 2^31
+# are, compiled with the sources they exercise; never loaded by the product.
 TESTING_LIB_NAME = "libhashpoint_b200_testing.so"
 TESTING_LIB_PATH = os.path.join(LIB_DIR, TESTING_LIB_NAME)
-TESTING_SOURCES = ["hp_api.cu", "hp_build.cu", "hp_aggregator.cu", "hp_tc_check.cu"]
+TESTING_SOURCES = ["hp_api.cu", "hp_build.cu", "hp_sample.cu", "hp_query.cu", "hp_aggregator.cu", "hp_tc_check.cu"]
 TESTING_FLAGS = ["-DHP_TESTING"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
@@ -317,6 +318,9 @@ def testing_lib():
         T.hp_pts2plane_withheld.restype = i32
         T.hp_pts2plane_status.argtypes = [vp, i64, i32, i32, vp]
         T.hp_pts2plane_status.restype = i32
+        opt_p = ctypes.POINTER(HpOptions)
+        T.hp_quick_query_for_nearby_point.argtypes = [vp, i64, cam_p, opt_p, vp, i64, vp, vp, i64, vp, vp]
+        T.hp_quick_query_for_nearby_point.restype = i32
         _testing = T
         return _testing
 

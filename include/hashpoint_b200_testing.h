@@ -6,6 +6,11 @@
  * sources they exercise, into a separate shared library,
  * libhashpoint_b200_testing.so, which also exports the product entry points of
  * those sources.  None has a counterpart in the reference.
+ *
+ * In that library hp_quick_query_for_nearby_point numbers at most 64 candidates
+ * of a window at once, where the product numbers up to 2^31, so that small
+ * tables take the rounds that windows of more candidates take; outputs are the
+ * same.
  */
 #ifndef HASHPOINT_B200_TESTING_H
 #define HASHPOINT_B200_TESTING_H

@@ -22,6 +22,19 @@ def _sample(X, c2w, cam, o, sidx, table, **tuning):
                               tuning=ops.make_tuning(**tuning) if tuning else None)
 
 
+def _query(X, c2w, cam, o, sidx, table, rays, L=None):
+    """quick_query by the product library, or by L."""
+    if L is None:
+        return ops.quick_query(X, c2w, cam.fx, cam.fy, cam.cx, cam.cy, cam.width, cam.height, o, sidx, table, rays)
+    out = torch.empty((len(rays), o.num_point_per_ray), dtype=torch.int32, device="cuda")
+    spec = ops.make_camera(c2w=c2w, fx=cam.fx, fy=cam.fy, cx=cam.cx, cy=cam.cy, width=cam.width, height=cam.height)
+    rc = L.hp_quick_query_for_nearby_point(X.data_ptr(), len(X), spec, ops.make_options(o), sidx.data_ptr(), len(sidx),
+                                           table.data_ptr(), rays.data_ptr(), len(rays), out.data_ptr(),
+                                           torch.cuda.current_stream().cuda_stream)
+    native.check(rc, "hp_quick_query_for_nearby_point", L)
+    return out
+
+
 @pytest.mark.parametrize("radius", [-0.05, -1e-20, 0.0, float("nan")])
 def test_radius_that_keeps_nothing(radius):
     """A candidate is kept when its distance is below the radius: never for one of zero or less."""
@@ -30,8 +43,7 @@ def test_radius_that_keeps_nothing(radius):
     assert (table[:, 1] > 0).any()
     o = synth.Options(kernel_size=3, radius_threshold=radius, num_point_per_ray=16)
     rays = torch.arange(1200, dtype=torch.int32, device="cuda")
-    rows = ops.quick_query(X, c2w, cam.fx, cam.fy, cam.cx, cam.cy, 40, 30, o, sidx, table, rays)
-    assert (rows == -1).all()
+    assert (_query(X, c2w, cam, o, sidx, table, rays) == -1).all()
     sp_xyz, pc_idx, sp_t, mask = _sample(X, c2w, cam, o, sidx, table)
     assert not mask.any() and (pc_idx == -1).all() and (sp_t == 0).all() and (sp_xyz == 0).all()
 
@@ -53,3 +65,33 @@ def test_points_a_thousand_away_from_a_sample():
     # that close
     bad = ~((out[3].cpu().numpy() == ref[3]).all(-1) & (out[1].cpu().numpy() == ref[1]).all((-1, -2)))
     assert (ref[4].reshape(24, 32)[bad] < 1e-6).all() and bad.sum() <= 7
+
+
+# (points, image, kernel, radius, row length): cells of 0 to 100 candidates
+WINDOWS = [(20_000, (60, 45), 5, 0.03, 256), (30_000, (30, 20), 7, 0.05, 99), (4_000, (9, 7), 31, 0.1, 300),
+           (500, (3, 2), 5, 0.5, 64), (2_000, (1, 1), 5, 5.0, 40)]
+
+
+@pytest.mark.parametrize("n,size,k,radius,cap", WINDOWS)
+def test_query_windows_taken_in_rounds(n, size, k, radius, cap):
+    """The test library numbers at most 64 candidates at once, as the product does 2^31: the rows are the same."""
+    native.build_testing()
+    cam = synth.look_at_camera((0.3, 0.2, 4.0), (0, 0, 0), *size, 0.5 * size[0])
+    X, c2w, sidx, table = _view(synth.shapes_cloud(np.random.default_rng(n), n), cam)
+    o = synth.Options(kernel_size=k, radius_threshold=radius, num_point_per_ray=cap)
+    rays = torch.arange(-1, size[0] * size[1] + 1, dtype=torch.int32, device="cuda")
+    want = _query(X, c2w, cam, o, sidx, table, rays)
+    assert (want >= 0).any()
+    assert torch.equal(_query(X, c2w, cam, o, sidx, table, rays, native.testing_lib()), want)
+
+
+def test_query_window_beyond_two_to_the_31():
+    """961 window cells, all the one bucket of 70 million ids."""
+    native.build()
+    cam = synth.look_at_camera((0, 0, 4.0), (0, 0, 0), 1, 1, 1.0)
+    X = torch.zeros((1, 3), device="cuda")
+    sidx = torch.zeros(70_000_000, dtype=torch.int32, device="cuda")
+    table = torch.tensor([[0, len(sidx)]], dtype=torch.int32, device="cuda")
+    o = synth.Options(kernel_size=31, radius_threshold=1.0, num_point_per_ray=20)
+    rows = _query(X, torch.from_numpy(cam.c2w).cuda(), cam, o, sidx, table, torch.zeros(3, dtype=torch.int32, device="cuda"))
+    assert (rows == 0).all()
