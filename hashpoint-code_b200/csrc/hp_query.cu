@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(kQueryWarps * 32) k_quick_query(const float* _
       pre -= cnt;
       const bool deep = __any_sync(kAll, cnt > kQueryPerCell);
       int carry = 0;  // lane c's copy: cell c's ids of earlier chunks
-      for (unsigned j0 = 0; j0 < total && base < cap; j0 += 32) {
+      for (unsigned j0 = 0; j0 < total && base < cap;) {
         const unsigned j = j0 + lane;
         int c = 0;
 #pragma unroll
@@ -125,6 +125,11 @@ __global__ void __launch_bounds__(kQueryWarps * 32) k_quick_query(const float* _
         const int pos = base + __popc(m & below);
         if (in && pos < cap) row[pos] = id;
         base += __popc(m);
+        j0 += 32;
+        if (deep) {  // the cell the chunk ended in has given its ids: on to the next one
+          const int last = __shfl_sync(kAll, c, 31);
+          if (__shfl_sync(kAll, carry, last) >= kQueryPerCell) j0 = max(j0, __shfl_sync(kAll, pre + cnt, last));
+        }
       }
     }
     const int written = min(base, cap);

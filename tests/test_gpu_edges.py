@@ -95,3 +95,34 @@ def test_query_window_beyond_two_to_the_31():
     o = synth.Options(kernel_size=31, radius_threshold=1.0, num_point_per_ray=20)
     rows = _query(X, torch.from_numpy(cam.c2w).cuda(), cam, o, sidx, table, torch.zeros(3, dtype=torch.int32, device="cuda"))
     assert (rows == 0).all()
+
+
+def _time(f, runs=9):
+    """Median microseconds of a call on the device."""
+    f()
+    t = []
+    for _ in range(runs):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        f()
+        b.record()
+        b.synchronize()
+        t.append(1e3 * a.elapsed_time(b))
+    return sorted(t)[runs // 2]
+
+
+def test_query_stops_at_a_cells_last_id():
+    """A cell gives at most 32 ids: buckets a hundred times as deep cost no more (they did cost that much more)."""
+    native.build()
+    cam = synth.look_at_camera((0, 0, 4.0), (0, 0, 0), 4, 4, 4.0)
+    X, c2w = torch.zeros((1, 3), device="cuda"), torch.from_numpy(cam.c2w).cuda()
+    o = synth.Options(kernel_size=5, radius_threshold=5.0, num_point_per_ray=1024)
+    rays = torch.arange(16, dtype=torch.int32, device="cuda").repeat(4)
+
+    def call(n):
+        sidx = torch.zeros(16 * n, dtype=torch.int32, device="cuda")
+        table = torch.stack([torch.arange(16, device="cuda") * n, torch.full((16,), n, device="cuda")], 1).int()
+        assert ((_query(X, c2w, cam, o, sidx, table, rays) == 0).sum(1) == 25 * 32).all()
+        return _time(lambda: _query(X, c2w, cam, o, sidx, table, rays))
+
+    assert call(100_000) < 4 * call(1_000)
