@@ -27,14 +27,19 @@ constexpr unsigned kWindowMax = 64;  // so that small tables take several rounds
 #else
 constexpr unsigned kWindowMax = 0x7fffffffu;
 #endif
-constexpr int kQueryRays = 8;  // rays a warp serves in turn, their directions computed side by side
+constexpr int kQueryRays = 8;  // rays a warp serves in turn in a long list, their directions computed side by side
+constexpr int64_t kLongList = 1 << 17;  // rays from which it does
 
 // Bound by the latency of the dependent loads (bucket, id, point) and the
 // instructions of each ray's set-up; the rows themselves are 67 MB for 65,536
-// rays of 256 (10 us).  65,536 rays of a 1M-point view at 800 x 800, 5 x 5
-// window: 72 us (ncu, cold; the call 126 -> 68 us); a lane per cell left a warp
-// waiting for its longest bucket, twice, with a division and a norm a
-// candidate: 179 us.  2, 4 or 8 rays a warp are level.
+// rays of 256 (10 us).  A lane per cell left a warp waiting for its longest
+// bucket, twice, with a division and a norm a candidate: 132 us for 65,536 rays
+// of a 1M-point view at 800 x 800, 5 x 5 window (launch and flushed caches
+// included), 60 us so.  A warp a ray fills the SMs from the shortest lists on
+// (kRays = 1: 500 rays 29 us, with eight a warp 55; 5,000 rays 30 and 59; 65,536
+// rays 60 and 65); from some 100,000 rays the shared set-up is worth more
+// (300,000 rays: 203 us with one, 188 with eight).
+template <int kRays>
 __global__ void __launch_bounds__(kQueryWarps * 32) k_quick_query(const float* __restrict__ xyz, int n_points,
                                                                   const int* __restrict__ sidx, int n_sorted,
                                                                   const int2* __restrict__ hash, DevCamera cam,
@@ -44,12 +49,12 @@ __global__ void __launch_bounds__(kQueryWarps * 32) k_quick_query(const float* _
   constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
-  const int64_t r0 = ((int64_t)blockIdx.x * kQueryWarps + (threadIdx.x >> 5)) * kQueryRays;
+  const int64_t r0 = ((int64_t)blockIdx.x * kQueryWarps + (threadIdx.x >> 5)) * kRays;
   if (r0 >= n_rays) return;
   const int cap = opt.num_point_per_ray, k = opt.k, k2 = k * k, W = cam.width, H = cam.height;
   int my_ray = -1;
   Ray mine{};
-  if (lane < kQueryRays && r0 + lane < n_rays) {
+  if (lane < kRays && r0 + lane < n_rays) {
     my_ray = __ldg(ray_ids + r0 + lane);
     if (my_ray < 0 || my_ray >= W * H) my_ray = -1;
     if (my_ray >= 0) make_ray(cam.c2w, cam.fx, cam.fy, cam.cx, cam.cy, my_ray % W, my_ray / W, mine);
@@ -62,7 +67,7 @@ __global__ void __launch_bounds__(kQueryWarps * 32) k_quick_query(const float* _
     window_cell(ray / W, ray % W, k, H, W, l, vv, uu);
     return bucket_range(__ldg(hash + (size_t)vv * W + uu), n_sorted);
   };
-  const int rays = (int)(n_rays - r0 < kQueryRays ? n_rays - r0 : kQueryRays);
+  const int rays = (int)(n_rays - r0 < kRays ? n_rays - r0 : kRays);
   int2 ahead = bucket(__shfl_sync(kAll, my_ray, 0), 0);
   for (int q = 0; q < rays; q++) {
     const int ray = __shfl_sync(kAll, my_ray, q);
@@ -227,8 +232,10 @@ extern "C" int32_t hp_quick_query_for_nearby_point(const float* xyz, int64_t n_p
     return set_error(HP_ERR_INVALID_ARGUMENT, "hp_quick_query_for_nearby_point: null pointer");
   if (((uintptr_t)hash_table & 7) != 0)
     return set_error(HP_ERR_INVALID_ARGUMENT, "hp_quick_query_for_nearby_point: hash_table must be 8-byte aligned");
-  const int64_t per = kQueryWarps * kQueryRays;
-  k_quick_query<<<(unsigned)((n_rays + per - 1) / per), kQueryWarps * 32, 0, (cudaStream_t)stream>>>(
+  const bool one = n_rays < kLongList;
+  const int64_t block = kQueryWarps * (one ? 1 : kQueryRays);
+  (one ? k_quick_query<1> : k_quick_query<kQueryRays>)<<<(unsigned)((n_rays + block - 1) / block), kQueryWarps * 32, 0,
+                                                        (cudaStream_t)stream>>>(
       xyz, (int)n_points, sorted_point_idx, (int)n_sorted, (const int2*)hash_table, dev_camera(cam), dev_options(opt),
       make_radius_test(opt->radius_threshold), ray_ids, (int)n_rays, out);
   return check_launch("k_quick_query");

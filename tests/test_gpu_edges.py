@@ -126,3 +126,33 @@ def test_query_stops_at_a_cells_last_id():
         return _time(lambda: _query(X, c2w, cam, o, sidx, table, rays))
 
     assert call(100_000) < 4 * call(1_000)
+
+
+def test_query_short_lists_fill_the_chip():
+    """592 rays of 25 buckets of 1,000 ids, none near: on 148 SMs they take little longer than one (with eight rays a warp
+    one after another they took eight times as long)."""
+    native.build()
+    cam = synth.look_at_camera((0, 0, 4.0), (0, 0, 0), 4, 4, 4.0)
+    X, c2w = torch.tensor([[50.0, 50.0, 0.0]], device="cuda"), torch.from_numpy(cam.c2w).cuda()
+    o = synth.Options(kernel_size=5, radius_threshold=0.1, num_point_per_ray=8)
+    sidx = torch.zeros(16_000, dtype=torch.int32, device="cuda")
+    table = torch.stack([torch.arange(16, device="cuda") * 1000, torch.full((16,), 1000, device="cuda")], 1).int()
+
+    def call(n):
+        rays = torch.full((n,), 5, dtype=torch.int32, device="cuda")
+        assert (_query(X, c2w, cam, o, sidx, table, rays) == -1).all()
+        return _time(lambda: _query(X, c2w, cam, o, sidx, table, rays))
+
+    assert call(592) < 3 * call(1)
+
+
+def test_query_long_and_short_lists_agree():
+    """Either side of the list length from which a warp serves eight rays: the same rows."""
+    cam = synth.look_at_camera((0.3, 0.2, 4.0), (0, 0, 0), 400, 330, 360.0)
+    X, c2w, sidx, table = _view(synth.shapes_cloud(np.random.default_rng(3), 60_000), cam)
+    o = synth.Options(kernel_size=3, radius_threshold=0.02, num_point_per_ray=12)
+    rays = torch.randperm(400 * 330, device="cuda")[:(1 << 17) + 3].int()
+    long = _query(X, c2w, cam, o, sidx, table, rays)
+    assert (long >= 0).any()
+    for a, b in ((0, (1 << 17) - 1), (4, 5), (1 << 17, (1 << 17) + 3)):
+        assert torch.equal(_query(X, c2w, cam, o, sidx, table, rays[a:b].contiguous()), long[a:b])
