@@ -129,8 +129,9 @@ struct RayList {
 // a warp: with 640, 4M-point views at 512 x 512 lose 22% to rays whose list
 // overflows; shapes and sphere views are level, the 3M-point clustered view
 // gains 5% (less shared memory leaves more L1).
-template <int kStage_, int kBlocks_, int kTileH_, int kTileW_>
+template <int kStage_, int kBlocks_, int kTileH_, int kTileW_, class Index_ = int>
 struct StageCfg {
+  using Index = Index_;  // numbers the candidates of a window in the general walk
   static constexpr int kStage = kStage_;
   static constexpr int kBlocks = kBlocks_;
   static constexpr int kTileH = kTileH_;
@@ -147,6 +148,17 @@ using Cfg4 = StageCfg<3840, 8, 16, 16>;
 using Cfg5 = StageCfg<3968, 6, 16, 16>;
 constexpr int kStageConfigs = 5;  // hp_tuning.stage_config 1..5 (0 = the default)
 constexpr int kDefaultStageConfig = 4;
+// Clamped window cells repeat a bucket (and tables may overlap), so a window's
+// 25 cells can hold 25 times the id list: up to 2^26 ids an int numbers them,
+// beyond that the default configuration with a walk in 64-bit indices serves
+// the view.  (Called from the same kernel, that walk cost the other rays 3%.)
+#ifdef HP_TESTING
+constexpr int64_t kIntIds = 40;
+#else
+constexpr int64_t kIntIds = 1 << 26;
+#endif
+using CfgWide = StageCfg<Cfg4::kStage, Cfg4::kBlocks, Cfg4::kTileH, Cfg4::kTileW, long long>;
+constexpr int kWideConfig = kStageConfigs + 1;
 
 __device__ __forceinline__ int2 cell_range(const SampleArgs& a, int vv, int uu) {
   return bucket_range(__ldg(a.hash + (size_t)vv * a.cam.width + uu), a.n_sorted);
@@ -201,6 +213,9 @@ __host__ __device__ inline void derive_args(SampleArgs& a) {
   a.near0 = a.opt.radius * 1.001f;
   a.quanta = 1.0f / a.opt.radius;
   a.eps = fabsf(a.opt.radius / a.opt.alpha_g);
+  // The reference's "farthest" buffer entry starts at 1e3, so eight entries beyond that leave slot 0 the one to
+  // replace; the lanes' buffer does not know this: such radii are left to the general walk.
+  if (a.opt.radius > 1e3f) a.eps = INFINITY;
 }
 
 __device__ __forceinline__ int bin_index(const BinDiv& bd, float x) {
@@ -225,31 +240,23 @@ __device__ __forceinline__ int bin_index(const BinDiv& bd, bool in, float x) {
   return b;
 }
 
-// Warp-cooperative sample_ray.  The ray's k*k window cells (reference order:
-// rows, then columns, clamped) are concatenated into one candidate sequence:
-// lane c < k*k holds cell c's range and its exclusive prefix, and each chunk
-// of 32 consecutive candidates is spread over the lanes, every lane finding its
-// cell by a binary search over the prefixes (shuffles).  Everything
-// order-dependent reproduces sample_ray exactly: the 48-per-cell cap from
-// ballot ranks plus a per-cell carry, bin sums added one candidate at a time
-// in sequence order, and the 8-entry ball buffers fed hits in sequence order.
-// A ray costs about ceil(candidates / 32) chunks per pass, so heavy rays finish
-// in a fraction of the time one thread would need for them.
+// The general walk: a ray by a whole warp, with the reference's own arithmetic.
+// The ray's k*k window cells (reference order: rows, then columns, clamped) are
+// concatenated into one candidate sequence: lane c < k*k holds cell c's range
+// (cbase, ccnt) and its exclusive prefix, and each chunk of 32 consecutive
+// candidates is spread over the lanes, every lane finding its cell by a binary
+// search over the prefixes (shuffles).  What depends on the order: the
+// 48-per-cell cap from ballot ranks plus a per-cell carry, bin sums added one
+// candidate at a time in sequence order, and the 8-entry ball buffers fed hits
+// in sequence order.  J numbers the candidates (see kIntIds).
+template <class J>
 __device__ __noinline__ void sample_ray_warp(const SampleArgs& a, int v, int u, unsigned* wbuf) {
   const unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
   const int W = a.cam.width, H = a.cam.height, k = a.opt.k;
   const int lo = ((k + 1) >> 1) - 1;
-  const int ray = v * W + u;
-  const int S = a.opt.S, P = a.opt.P;
-  const float radius = a.opt.radius;
-  Ray r;
-  make_ray(a.cam.c2w, a.cam.fx, a.cam.fy, a.cam.cx, a.cam.cy, u, v, r);
-  const float inv_dd = __frcp_rn(r.dd);
-  const RadiusTest& rt = a.rt;
-
-  // lane c < k*k: cell c's first index and count; exclusive prefix over cells
+  // lane c < k*k: cell c's first index and count
   int cbase = 0, ccnt = 0;
   if (lane < k * k) {
     const int q = lane / k;
@@ -258,27 +265,36 @@ __device__ __noinline__ void sample_ray_warp(const SampleArgs& a, int v, int u, 
     cbase = rg.x;
     ccnt = rg.y - rg.x;
   }
-  int cpre = ccnt;
+  const int ray = v * W + u;
+  const int S = a.opt.S, P = a.opt.P;
+  const float radius = a.opt.radius;
+  Ray r;
+  make_ray(a.cam.c2w, a.cam.fx, a.cam.fy, a.cam.cx, a.cam.cy, u, v, r);
+  const float inv_dd = __frcp_rn(r.dd);
+  const RadiusTest& rt = a.rt;
+
+  J cpre = ccnt;  // exclusive prefix over cells
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(kAll, cpre, o);
+    const J t = __shfl_up_sync(kAll, cpre, o);
     if (lane >= o) cpre += t;
   }
-  const int total = __shfl_sync(kAll, cpre, 31);
+  const J total = __shfl_sync(kAll, cpre, 31);
   cpre -= ccnt;
+  auto span = [](J x) { return (int)min(max(x, J(0)), J(32)); };
   const bool capped = __any_sync(kAll, ccnt > kKeptPerCell);
 
   // body(j0, valid, idx, cell, pc) per lane and chunk: candidate j0 + lane of
   // the sequence, its index for src.fetch, its cell and the cell's first j
   auto chunks = [&](auto&& body) {
-    for (int j0 = 0; j0 < total; j0 += 32) {
-      const int j = j0 + lane;
+    for (J j0 = 0; j0 < total; j0 += 32) {
+      const J j = j0 + lane;
       int c = 0;
 #pragma unroll
       for (int s = 16; s > 0; s >>= 1)
         if (__shfl_sync(kAll, cpre, c + s) <= j) c += s;
-      const int pc = __shfl_sync(kAll, cpre, c);
-      const int idx = __shfl_sync(kAll, cbase, c) + (j - pc);
+      const J pc = __shfl_sync(kAll, cpre, c);
+      const int idx = __shfl_sync(kAll, cbase, c) + (int)(j - pc);
       body(j0, j < total, idx, c, pc);
     }
   };
@@ -287,19 +303,19 @@ __device__ __noinline__ void sample_ray_warp(const SampleArgs& a, int v, int u, 
   // has its 48 kept candidates, the rest of it is skipped -- none of them can
   // be kept.
   auto capped_chunks = [&](const int& carry, auto&& body) {
-    for (int j0 = 0; j0 < total;) {
-      const int j = j0 + lane;
+    for (J j0 = 0; j0 < total;) {
+      const J j = j0 + lane;
       int c = 0;
 #pragma unroll
       for (int s = 16; s > 0; s >>= 1)
         if (__shfl_sync(kAll, cpre, c + s) <= j) c += s;
-      const int pc = __shfl_sync(kAll, cpre, c);
-      const int idx = __shfl_sync(kAll, cbase, c) + (j - pc);
+      const J pc = __shfl_sync(kAll, cpre, c);
+      const int idx = __shfl_sync(kAll, cbase, c) + (int)(j - pc);
       body(j0, j < total, idx, c, pc);
       j0 += 32;
       if (capped) {
         const int last = __shfl_sync(kAll, c, 31);
-        if (__shfl_sync(kAll, carry, last) >= kKeptPerCell) j0 = max(j0, __shfl_sync(kAll, cpre + ccnt, last));
+        if (__shfl_sync(kAll, carry, last) >= kKeptPerCell) j0 = max(j0, __shfl_sync(kAll, J(cpre + ccnt), last));
       }
     }
   };
@@ -317,11 +333,11 @@ __device__ __noinline__ void sample_ray_warp(const SampleArgs& a, int v, int u, 
   };
   // kept candidates that are among the first 48 kept of their cell; `carry`
   // (lane c's copy is cell c's) counts a cell's kept candidates of earlier chunks
-  auto accept = [&](bool kept, int j0, int cell, int pc, int& carry) -> bool {
+  auto accept = [&](bool kept, J j0, int cell, J pc, int& carry) -> bool {
     if (!capped) return kept;
     const unsigned m = __ballot_sync(kAll, kept);
-    const int before = __shfl_sync(kAll, carry, cell) + __popc(m & below & ~lane_span(0, max(pc - j0, 0)));
-    carry += __popc(m & lane_span(min(max(cpre - j0, 0), 32), min(max(cpre + ccnt - j0, 0), 32)));
+    const int before = __shfl_sync(kAll, carry, cell) + __popc(m & below & ~lane_span(0, span(pc - j0)));
+    carry += __popc(m & lane_span(span(cpre - j0), span(cpre + ccnt - j0)));
     return kept && before < kKeptPerCell;
   };
   const BinDiv& bdiv = a.bins;
@@ -333,7 +349,7 @@ __device__ __noinline__ void sample_ray_warp(const SampleArgs& a, int v, int u, 
   float tmin = 1e3f, tmax = -1e3f;
   {
     int carry = 0;
-    capped_chunks(carry, [&](int j0, bool valid, int idx, int cell, int pc) {
+    capped_chunks(carry, [&](J j0, bool valid, int idx, int cell, J pc) {
       float t = 0.f, e0, e1, e2;
       if (accept(eval(valid, idx, t, e0, e1, e2), j0, cell, pc, carry)) {
         if (tmin > t) tmin = t;
@@ -364,7 +380,7 @@ __device__ __noinline__ void sample_ray_warp(const SampleArgs& a, int v, int u, 
     for (int q = 0; q < kBins / 32; q++) s1[q] = 0u, s2[q] = 0u;
     {
       int carry = 0;
-      capped_chunks(carry, [&](int j0, bool valid, int idx, int cell, int pc) {
+      capped_chunks(carry, [&](J j0, bool valid, int idx, int cell, J pc) {
         float t = 0.f, e0, e1, e2;
         if (accept(eval(valid, idx, t, e0, e1, e2), j0, cell, pc, carry)) {
           const int b = bin_of(t, tmin);
@@ -421,7 +437,7 @@ __device__ __noinline__ void sample_ray_warp(const SampleArgs& a, int v, int u, 
 #pragma unroll
       for (int q = 0; q < kWalkBatch; q++) bsum[q] = 0.0f, bcnt[q] = 0;
       int carry = 0;
-      capped_chunks(carry, [&](int j0, bool valid, int idx, int cell, int pc) {
+      capped_chunks(carry, [&](J j0, bool valid, int idx, int cell, J pc) {
         float t = 0.f, e0 = 0.f, e1 = 0.f, e2 = 0.f;
         int mine = -1;
         float dist = 0.0f;
@@ -508,7 +524,7 @@ __device__ __noinline__ void sample_ray_warp(const SampleArgs& a, int v, int u, 
       maxd[q] = 1e3f;
       settled[q] = false;
     }
-    chunks([&](int, bool valid, int idx, int, int) {
+    chunks([&](J, bool valid, int idx, int, J) {
       float dq[kBallPass];
       bool hq[kBallPass];
       int id = -1;
@@ -649,9 +665,6 @@ __device__ __forceinline__ unsigned serve_rays(const SampleArgs& a, const int L,
                                                int entries) {
   constexpr unsigned kAll = 0xffffffffu;
   constexpr unsigned kCloseKeys = 512;  // of a float's bits: at least 2^-15 of its value
-  // The reference's "farthest" starts at 1e3: eight entries no nearer than that leave it there, and slot 0 the
-  // one to replace.  1e6 (a squared distance) less kCloseKeys, as bits:
-  constexpr unsigned kFarKey = 0x49742400u - kCloseKeys;
   constexpr int kSumBits = 21, kQuant = 10;  // histogram word: sum of distances in radius / 2^kQuant, count above;
                                              // 2^kQuant entries fit
   const int lane = threadIdx.x & 31;
@@ -705,7 +718,9 @@ __device__ __forceinline__ unsigned serve_rays(const SampleArgs& a, const int L,
     }
     const int c0 = __shfl_sync(kAll, cnt, gb), c1 = __shfl_sync(kAll, cnt, gb + 1), c2 = __shfl_sync(kAll, cnt, gb + 2),
               c3 = __shfl_sync(kAll, cnt, gb + 3), c4 = __shfl_sync(kAll, cnt, gb + 4);
-    p1 = c0, p2 = p1 + c1, p3 = p2 + c2, p4 = p3 + c3, T = p4 + c4;
+    p1 = c0, p2 = (int)((unsigned)p1 + c1), p3 = (int)((unsigned)p2 + c2), p4 = (int)((unsigned)p3 + c3);
+    T = (int)((unsigned)p4 + c4);
+    good = good && (p2 | p3 | p4 | T) >= 0;  // (clamped rows repeat: their sum may pass 2^31)
     base = __shfl_sync(kAll, first, gb);
     const int f1 = __shfl_sync(kAll, first, gb + 1), f2 = __shfl_sync(kAll, first, gb + 2),
               f3 = __shfl_sync(kAll, first, gb + 3), f4 = __shfl_sync(kAll, first, gb + 4);
@@ -942,7 +957,6 @@ __device__ __forceinline__ unsigned serve_rays(const SampleArgs& a, const int L,
               if (first && todo > kBallBuf) {
                 if (sl < kBallBuf) key = sk;
                 if (sl > 0 && sl < kBallBuf && sk - prev < kCloseKeys + kBallBuf) close = true;
-                if (least >= kFarKey) close = true;
                 limit = least;
               }
             }
@@ -1181,7 +1195,7 @@ __device__ __forceinline__ void serve_list(const SampleArgs& a0, const SampleArg
       odd &= ~((0xffffffffu >> (32 - L)) << l);
       const int ray = __shfl_sync(0xffffffffu, e.x, l);
       __syncwarp();
-      sample_ray_warp(a, ray / a.cam.width, ray % a.cam.width, reinterpret_cast<unsigned*>(pool));
+      sample_ray_warp<typename Cfg::Index>(a, ray / a.cam.width, ray % a.cam.width, reinterpret_cast<unsigned*>(pool));
     }
     __syncwarp();
     i++;
@@ -1348,10 +1362,10 @@ static SamplingKernels sampling_kernels() {
           Cfg::kTileW,
           Cfg::kEntries};
 }
-static const SamplingKernels& stage_kernels(int config) {  // config 1..kStageConfigs
-  static const SamplingKernels table[kStageConfigs] = {sampling_kernels<Cfg1>(), sampling_kernels<Cfg2>(),
-                                                       sampling_kernels<Cfg3>(), sampling_kernels<Cfg4>(),
-                                                       sampling_kernels<Cfg5>()};
+static const SamplingKernels& stage_kernels(int config) {  // config 1..kWideConfig
+  static const SamplingKernels table[kWideConfig] = {sampling_kernels<Cfg1>(), sampling_kernels<Cfg2>(),
+                                                     sampling_kernels<Cfg3>(), sampling_kernels<Cfg4>(),
+                                                     sampling_kernels<Cfg5>(), sampling_kernels<CfgWide>()};
   return table[config - 1];
 }
 
@@ -1371,7 +1385,7 @@ static int64_t max_view_entries(int64_t H, int64_t W) {
 // device and size the persistent grid from their occupancy.
 int32_t sampling_grid(int config, int* blocks, int* sm_count = nullptr) {
   static std::mutex mu;
-  static int grid[128][kStageConfigs] = {{0}}, sm_counts[128] = {0};
+  static int grid[128][kWideConfig] = {{0}}, sm_counts[128] = {0};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return set_error(HP_ERR_CUDA, "hp_quick_sampling: cudaGetDevice failed");
   if (dev < 0 || dev >= 128)
@@ -1546,6 +1560,7 @@ extern "C" int32_t hp_quick_sampling_tuned(const float* xyz, int64_t n_points, c
     return rc;
   Tune tn;
   if (int32_t rc = read_tuning("hp_quick_sampling", tuning, tn)) return rc;
+  if (n_sorted > kIntIds) tn.config = kWideConfig;
   const ListLayout L = list_layout(cam->height, cam->width, n_sorted);
   if (!workspace || workspace_bytes < L.total || ((uintptr_t)workspace & 255) != 0)
     return set_error(HP_ERR_WORKSPACE, "hp_quick_sampling: workspace needs %zu bytes, 256-byte aligned (got %zu)",
@@ -1639,6 +1654,7 @@ extern "C" int32_t hp_quick_sampling_batch(const hp_view* views, const hp_view* 
       snprintf(msg, sizeof(msg), "%s", hp_last_error());
       return set_error(rc, "%s (view %d)", msg, v);
     }
+    if (hv.n_sorted > kIntIds) tn.config = kWideConfig;
   }
   const int64_t entries = batch_entries(views, n_views);
   const int64_t total_slots = batch_slots(views, n_views);

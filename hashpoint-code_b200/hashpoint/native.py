@@ -321,6 +321,10 @@ def testing_lib():
         opt_p = ctypes.POINTER(HpOptions)
         T.hp_quick_query_for_nearby_point.argtypes = [vp, i64, cam_p, opt_p, vp, i64, vp, vp, i64, vp, vp]
         T.hp_quick_query_for_nearby_point.restype = i32
+        T.hp_quick_sampling_workspace_size.argtypes = [i64, i32, i32]
+        T.hp_quick_sampling_workspace_size.restype = sz
+        T.hp_quick_sampling.argtypes = [vp, i64, cam_p, opt_p, vp, i64, vp, vp, vp, vp, vp, vp, sz, vp]
+        T.hp_quick_sampling.restype = i32
         _testing = T
         return _testing
 

@@ -7,10 +7,10 @@
  * libhashpoint_b200_testing.so, which also exports the product entry points of
  * those sources.  None has a counterpart in the reference.
  *
- * In that library hp_quick_query_for_nearby_point numbers at most 64 candidates
- * of a window at once, where the product numbers up to 2^31, so that small
- * tables take the rounds that windows of more candidates take; outputs are the
- * same.
+ * In that library small tables take the paths of windows whose candidates pass
+ * 2^31, with the same outputs: hp_quick_query_for_nearby_point numbers at most
+ * 64 candidates of a window at once, and hp_quick_sampling's general walk counts
+ * in 64 bits for views of more than 40 ids (the product: 2^26).
  */
 #ifndef HASHPOINT_B200_TESTING_H
 #define HASHPOINT_B200_TESTING_H

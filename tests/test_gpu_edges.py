@@ -85,6 +85,39 @@ def test_query_windows_taken_in_rounds(n, size, k, radius, cap):
     assert torch.equal(_query(X, c2w, cam, o, sidx, table, rays, native.testing_lib()), want)
 
 
+def _reversed_buckets(sidx, table):
+    """The same buckets, stored last pixel first: rays with two non-empty cells in a window row take the general walk."""
+    sidx, h = sidx.cpu().numpy(), table.cpu().numpy().copy()
+    out, at = np.full_like(sidx, -1), 0
+    for p in np.nonzero(h[:, 1] > 0)[0][::-1]:
+        s, c = h[p]
+        out[at:at + c] = sidx[s:s + c]
+        h[p, 0] = at
+        at += c
+    return torch.from_numpy(out).cuda(), torch.from_numpy(h).cuda()
+
+
+@pytest.mark.parametrize("n,size,k,radius", [w[:4] for w in WINDOWS if w[2] <= 5] + [(60_000, (40, 31), 5, 0.03),
+                                                                                    (60_000, (33, 16), 2, 0.5)])
+def test_sampling_walk_in_64_bit_indices(n, size, k, radius):
+    """The test library's general walk numbers a window's candidates in 64 bits: the same bytes."""
+    native.build_testing()
+    T = native.testing_lib()
+    cam = synth.look_at_camera((0.3, 0.2, 4.0), (0, 0, 0), *size, 0.5 * size[0])
+    X, c2w, sidx, table = _view(synth.shapes_cloud(np.random.default_rng(n), n), cam)
+    o = synth.Options(kernel_size=k, radius_threshold=radius, num_point_cloud_per_sp=8)
+    want = _sample(X, c2w, cam, o, sidx, table)
+    sidx, table = _reversed_buckets(sidx, table)
+    got = [torch.empty_like(t) for t in want]
+    spec = ops.make_camera(c2w=c2w, fx=cam.fx, fy=cam.fy, cx=cam.cx, cy=cam.cy, width=cam.width, height=cam.height)
+    ws = torch.empty(T.hp_quick_sampling_workspace_size(len(sidx), size[1], size[0]), dtype=torch.uint8, device="cuda")
+    rc = T.hp_quick_sampling(X.data_ptr(), len(X), spec, ops.make_options(o), sidx.data_ptr(), len(sidx), table.data_ptr(),
+                             *[t.data_ptr() for t in got], ws.data_ptr(), len(ws),
+                             torch.cuda.current_stream().cuda_stream)
+    native.check(rc, "hp_quick_sampling", T)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
 def test_query_window_beyond_two_to_the_31():
     """961 window cells, all the one bucket of 70 million ids."""
     native.build()
