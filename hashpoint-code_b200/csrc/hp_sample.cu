@@ -214,7 +214,7 @@ __host__ __device__ inline void derive_args(SampleArgs& a) {
   a.quanta = 1.0f / a.opt.radius;
   a.eps = fabsf(a.opt.radius / a.opt.alpha_g);
   // The reference's "farthest" buffer entry starts at 1e3, so eight entries beyond that leave slot 0 the one to
-  // replace; the lanes' buffer does not know this: such radii are left to the general walk.
+  // replace; the lanes' buffer does not know this: such radii are left to serve_exact.
   if (a.opt.radius > 1e3f) a.eps = INFINITY;
 }
 
@@ -650,19 +650,28 @@ __device__ __forceinline__ float sqrt_fast(float x) {
   return y;
 }
 
+// What serve_rays leaves to serve_exact, by its lanes' groups.
+struct Unsettled {
+  int n;        // listed candidates; -1: none are listed yet
+  int emitted;  // samples emitted; -1: the walk is to be done again
+  bool balls;   // their points are to be selected again
+};
+
 // Serve 32 / L rays, L lanes each: `entry` is the group's list entry (ray < 0:
 // none); pool: the warp's kHistWords words and `entries` listed candidates.
-// Returns the lanes of groups left unserved, for sample_ray_warp.
+// Returns the lanes of groups left unserved, for sample_ray_warp (their list
+// overflows), and in `left` what else is left, for serve_exact.
 //
 // The walk uses mean distances from the histogram's quantised sums, and the ball
 // buffers order their hits by squared distance.  Both know their error; where a
-// comparison is closer than that (about one ray in a thousand, and the rays
-// whose window repeats rows at the image's edge), the ray is left to
-// sample_ray_warp, which has the reference's own arithmetic (sums of norm3df in
-// window order, buffers ordered by norm3df), so every decision is the
+// comparison is closer than that (about one ray in a thousand of a cloud
+// without equal distances), the ray's walk or point selection is left to
+// serve_exact, and so are rays whose window's rows are no runs (at the image's
+// edge, where they repeat cells); it has the reference's own arithmetic (sums of
+// norm3df in window order, buffers ordered by norm3df), so every decision is the
 // reference's.
 __device__ __forceinline__ unsigned serve_rays(const SampleArgs& a, const int L, int4 entry, unsigned char* pool,
-                                               int entries) {
+                                               int entries, Unsettled& left) {
   constexpr unsigned kAll = 0xffffffffu;
   constexpr unsigned kCloseKeys = 512;  // of a float's bits: at least 2^-15 of its value
   constexpr int kSumBits = 21, kQuant = 10;  // histogram word: sum of distances in radius / 2^kQuant, count above;
@@ -745,18 +754,16 @@ __device__ __forceinline__ unsigned serve_rays(const SampleArgs& a, const int L,
     cpre -= ccnt;
     good = good && L == 32;
   }
-  // a table whose buckets do not follow one another: left to the general walk
-  const bool general = live && !good;
-  unsigned odd = __ballot_sync(kAll, general);
-  live = live && !general;
-  if (!__any_sync(kAll, live)) return odd;
+  int n = live && !good ? -1 : 0;  // no runs: nothing is listed here
+  left = {n, 0, false};
+  live = live && good;
+  if (!__any_sync(kAll, live)) return 0u;
   if (!live) T = 0;
 
   // pass A: tmin over the kept candidates (epcq_render_topk.cu:132-161) and the list
   const float omax = fmaxf(fabsf(r.o[0]), fmaxf(fabsf(r.o[1]), fabsf(r.o[2])));
   const float c0 = __fmaf_rn(1e-5f, 1.0f + omax, a.near0);
   float tmin = 1e3f;
-  int n = 0;
   {
     const int Tmax = __reduce_max_sync(kAll, T);
     auto index = [&](int j) {
@@ -804,11 +811,8 @@ __device__ __forceinline__ unsigned serve_rays(const SampleArgs& a, const int L,
       p = pn;
     }
   }
-  {
-    const unsigned over = __ballot_sync(kAll, n > cap);  // more listed candidates than the group holds
-    odd |= over;
-    if (n > cap) live = false, n = 0;
-  }
+  const unsigned over = __ballot_sync(kAll, n > cap);  // more listed candidates than the group holds
+  if (n > cap) live = false, n = 0;
   for (int o = L >> 1; o > 0; o >>= 1) tmin = fminf(tmin, __shfl_xor_sync(kAll, tmin, o));
   __syncwarp();
 
@@ -845,7 +849,7 @@ __device__ __forceinline__ unsigned serve_rays(const SampleArgs& a, const int L,
   int emitted = 0;
   // how far the walk's alpha can be off by the quantised sums (relative); the mean lies within half a quantum
   const float eps = __fmaf_rn(a.eps, 1.0f / (1 << kQuant) + 1e-5f, 1e-5f);
-  bool close = !(eps < 0.05f) || !rt.fast;  // a comparison was closer than its error: left to the general walk
+  bool close = rows != 0u && (!(eps < 0.05f) || !rt.fast);  // a comparison was closer than its error
   {
     // primary-surface walk (epcq_render_topk.cu:181-204): L bins at a time, their alphas side by side
     float transmit = 1.0f, off = 0.0f, t0 = 0.0f, t1 = 0.0f;
@@ -892,8 +896,8 @@ __device__ __forceinline__ unsigned serve_rays(const SampleArgs& a, const int L,
         a.mask[at] = 1;
       }
     }
-    close = (__ballot_sync(kAll, close) & gmask) != 0u;
-    if (close) emitted = 0;
+    if ((__ballot_sync(kAll, close) & gmask) != 0u) emitted = -1;
+    close = false;
 
     // per-sample point selection (epcq_render_topk.cu:10-81), a sample at a time
     const int most = __reduce_max_sync(kAll, emitted);
@@ -999,9 +1003,249 @@ __device__ __forceinline__ unsigned serve_rays(const SampleArgs& a, const int L,
       }
     }
   }
-  close = (__ballot_sync(kAll, close && live) & gmask) != 0u;
-  if (live && !close) default_slots(a, (size_t)ray, emitted, sl, L);
-  return odd | __ballot_sync(kAll, close);
+  if (live && emitted >= 0) default_slots(a, (size_t)ray, emitted, sl, L);
+  left = {n, emitted, (__ballot_sync(kAll, close) & gmask) != 0u};
+  return over;
+}
+
+// The rays that serve_rays left, as it serves them: their list (made here cell
+// by cell where there is none), the walk over sums of norm3df added in window
+// order, a ray at a time by the whole warp, and the point selection with buffers
+// of norm3df in slot order, the warp's rays side by side.  Returns the lanes of
+// groups whose list overflows.
+//
+// A ray by sample_ray_warp walks its window three times and more; where many
+// rays come here (repeated or lattice points, whose distances tie) the whole
+// view waited for that.  1M points at 800 x 800, sampling alone: each place
+// three times 2910 us with it, 640 so (980 with one thread a ray); rounded to a
+// lattice 2360 and 590 (880); buckets out of pixel order 1980 and 950 (860).
+__device__ __forceinline__ unsigned serve_exact(const SampleArgs& a, int L, int4 entry, unsigned char* pool, int entries,
+                                             Unsettled left) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int gb = lane & ~(L - 1), sl = lane & (L - 1);
+  const unsigned group = kAll >> (32 - L), gmask = group << gb;
+  const unsigned before = (1u << lane) - 1u, below = gmask & before;
+  const int cap = entries * L / 32;
+  int* lists = reinterpret_cast<int*>(pool + kHistWords * 4);
+  int* list = lists + gb * (entries / 32);
+  const int S = a.opt.S, P = a.opt.P;
+  const RadiusTest& rt = a.rt;
+  const int ray = entry.x;
+  Ray r;
+#pragma unroll
+  for (int i = 0; i < 3; i++) r.o[i] = __ldg(a.cam.c2w + 4 * i + 3);
+  r.d[0] = __int_as_float(entry.y), r.d[1] = __int_as_float(entry.z), r.d[2] = __int_as_float(entry.w);
+  r.dd = dot3(r.d[0], r.d[1], r.d[2], r.d[0], r.d[1], r.d[2]);
+  int n = left.n, emitted = left.emitted;
+  bool balls = left.balls;
+
+  // the list of a window whose rows are no runs
+  if (__any_sync(kAll, n < 0)) {
+    const bool make = n < 0;
+    n = make ? 0 : n;
+    const int W = a.cam.width, H = a.cam.height, k = a.opt.k, lo = ((k + 1) >> 1) - 1;
+    const float inv_dd = __frcp_rn(r.dd);
+    const float omax = fmaxf(fabsf(r.o[0]), fmaxf(fabsf(r.o[1]), fabsf(r.o[2])));
+    const float c0 = __fmaf_rn(1e-5f, 1.0f + omax, a.near0);
+    const int v = make ? ray / W : 0, u = make ? ray - v * W : 0;
+    for (int c = 0; c < k * k; c++) {
+      int2 rg = make_int2(0, 0);
+      if (make) rg = cell_range(a, min(max(v + c / k - lo, 0), H - 1), min(max(u + c % k - lo, 0), W - 1));
+      const unsigned count = (unsigned)(rg.y - rg.x);
+      int had = 0;  // kept of this cell
+      for (unsigned j0 = 0; __any_sync(kAll, j0 < count); j0 += (unsigned)L) {
+        const int idx = rg.x + (int)(j0 + sl);
+        float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+        bool in = j0 + sl < count;
+        if (in) p = __ldg(a.pts + idx);
+        in = in && __float_as_int(p.w) >= 0;
+        const float t = ray_t(r, inv_dd, p);
+        const float e0 = __fsub_rn(p.x, __fmaf_rn(t, r.d[0], r.o[0]));
+        const float e1 = __fsub_rn(p.y, __fmaf_rn(t, r.d[1], r.o[1]));
+        const float e2 = __fsub_rn(p.z, __fmaf_rn(t, r.d[2], r.o[2]));
+        const float q = squared(e0, e1, e2);
+        bool kept = within_radius(rt, in, q, e0, e1, e2);
+        const bool near = kept || (in && q <= near_limit(c0, t));
+        const unsigned km = __ballot_sync(kAll, kept), nm = __ballot_sync(kAll, near);
+        kept = kept && had + __popc(km & below) < kKeptPerCell;
+        had = min(had + __popc(km & gmask), kKeptPerCell);
+        const int pos = n + __popc(nm & below);
+        if (near && pos < cap) list[pos] = kept ? idx : idx | (int)0x80000000u;
+        n = min(n + __popc(nm & gmask), cap + 1);
+      }
+    }
+    if (make) emitted = n > cap ? 0 : -1;
+    __syncwarp();
+  }
+  const unsigned over = __ballot_sync(kAll, n > cap);
+
+  // the walk (epcq_render_topk.cu:181-204)
+  float* sums = reinterpret_cast<float*>(pool);
+  int* counts = reinterpret_cast<int*>(pool) + kBins;
+  static_assert(2 * kBins <= kHistWords, "sums and counts");
+  const unsigned walks = __ballot_sync(kAll, emitted < 0);
+  for (unsigned todo = walks; todo;) {
+    const int g = __ffs(todo) - 1;
+    todo &= ~(group << g);
+    const int* from = lists + g * (entries / 32);
+    const int m = __shfl_sync(kAll, n, g);
+    Ray w;
+#pragma unroll
+    for (int i = 0; i < 3; i++) w.o[i] = r.o[i], w.d[i] = __shfl_sync(kAll, r.d[i], g);
+    w.dd = __shfl_sync(kAll, r.dd, g);
+    const float inv_dd = __frcp_rn(w.dd);
+    for (int b = lane; b < 2 * kBins; b += 32) reinterpret_cast<int*>(pool)[b] = 0;
+    auto entry_at = [&](int i, float4& p) {
+      const int idx = i < m ? from[i] : -1;  // listed but not kept: below 0, too
+      p = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (idx >= 0) p = __ldg(a.pts + idx);
+      return idx >= 0;
+    };
+    float tmin = 1e3f;
+    for (int i0 = 0; i0 < m; i0 += 32) {
+      float4 p;
+      if (entry_at(i0 + lane, p)) tmin = fminf(tmin, ray_t(w, inv_dd, p));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) tmin = fminf(tmin, __shfl_xor_sync(kAll, tmin, o));
+    __syncwarp();
+    for (int i0 = 0; i0 < m; i0 += 32) {
+      float4 p;
+      bool in = entry_at(i0 + lane, p);
+      const float t = ray_t(w, inv_dd, p);
+      const int b = bin_index(a.bins, in, __fsub_rn(t, tmin));
+      const float dist = norm3df(__fsub_rn(p.x, __fmaf_rn(t, w.d[0], w.o[0])), __fsub_rn(p.y, __fmaf_rn(t, w.d[1], w.o[1])),
+                                 __fsub_rn(p.z, __fmaf_rn(t, w.d[2], w.o[2])));
+      in = in && b < kBins;
+      // a bin's first lane adds those of the bin in order
+      const unsigned peers = __match_any_sync(kAll, in ? b : kBins + lane);
+      const bool first = in && (peers & before) == 0u;
+      unsigned rest = first ? peers : 0u;
+      float sum = first ? sums[b] : 0.0f;
+      while (__any_sync(kAll, rest != 0u)) {
+        const float x = __shfl_sync(kAll, dist, rest ? __ffs(rest) - 1 : lane);
+        if (rest) sum = __fadd_rn(sum, x);
+        rest &= rest - 1;
+      }
+      if (first) sums[b] = sum, counts[b] += __popc(peers);
+      __syncwarp();
+    }
+    const size_t slot0 = (size_t)__shfl_sync(kAll, ray, g) * S;
+    float transmit = 1.0f;
+    int out = 0;
+    bool more = true;
+    for (int b0 = 0; b0 < kBins && more; b0 += 32) {
+      const int cnt = counts[b0 + lane];
+      unsigned used = __ballot_sync(kAll, cnt > 1);
+      if (!used) continue;
+      const float sdf = __fdiv_rn(sums[b0 + lane], __fadd_rn((float)cnt, 1e-6f));
+      const float alpha = __fmul_rn(a.opt.gamma, __expf(__fdiv_rn(-sdf, a.opt.alpha_g)));
+      const float t = __fmaf_rn((float)(b0 + lane), a.opt.t_intvl, tmin);
+      int slot = -1;
+      while (used && more) {
+        const int src = __ffs(used) - 1;
+        used &= used - 1;
+        const float al = __shfl_sync(kAll, alpha, src);
+        more = !(transmit < 1e-3f || out >= S);
+        if (more) {
+          if (__fmul_rn(al, transmit) > 1e-3f) {
+            if (lane == src) slot = out;
+            out++;
+          }
+          transmit = __fsub_rn(transmit, al);
+        }
+      }
+      if (slot >= 0) {
+        const size_t at = slot0 + slot;
+#pragma unroll
+        for (int i = 0; i < 3; i++) a.sp_xyz[at * 3 + i] = __fmaf_rn(t, w.d[i], w.o[i]);
+        a.sp_t[at] = t;
+        a.mask[at] = 1;
+      }
+    }
+    if (gb == g) emitted = out, balls = out > 0;
+    __syncwarp();
+  }
+
+  // point selection (epcq_render_topk.cu:10-81): lanes 0..7 of a group hold its buffer's slots
+  const size_t slot0 = (size_t)(ray < 0 ? 0 : ray) * S;
+  const int most = __reduce_max_sync(kAll, balls ? emitted : 0), nball = __reduce_max_sync(kAll, balls ? n : 0);
+  for (int s = 0; s < most; s++) {
+    const bool on = balls && s < emitted;
+    const float ts = on ? *(volatile const float*)(a.sp_t + slot0 + s) : 0.0f;
+    const float sx = __fmaf_rn(ts, r.d[0], r.o[0]), sy = __fmaf_rn(ts, r.d[1], r.o[1]), sz = __fmaf_rn(ts, r.d[2], r.o[2]);
+    float held = 0.0f, farthest = 1e3f;  // this lane's slot; the group's "farthest" entry and its slot
+    int held_id = -1, size = 0, at = 0;
+    bool settled = false;  // one was replaced: `farthest` is the maximum (before: the minimum of what came)
+    for (int i0 = 0; i0 < nball; i0 += L) {
+      float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+      const bool in = on && i0 + sl < n;
+      if (in) p = __ldg(a.pts + (list[i0 + sl] & 0x7fffffff));
+      const float e0 = __fsub_rn(sx, p.x), e1 = __fsub_rn(sy, p.y), e2 = __fsub_rn(sz, p.z);
+      const bool look = in && !(squared(e0, e1, e2) > rt.hi2);
+      if (!__any_sync(kAll, look)) continue;
+      const float dist = norm3df(e0, e1, e2);
+      const bool hit = look && dist < rt.r;
+      // those that can change the buffer: all while it fills; then those below `farthest`, and, before the first of
+      // these has replaced an entry, any after it
+      const unsigned hits = __ballot_sync(kAll, hit) & gmask, nearer = __ballot_sync(kAll, hit && dist < farthest) & gmask;
+      unsigned todo = size < kBallBuf ? hits : settled ? nearer : nearer ? hits & ~((nearer & -nearer) - 1u) : 0u;
+      while (__any_sync(kAll, todo != 0u)) {
+        const int src = todo ? __ffs(todo) - 1 : lane;
+        const float x = __shfl_sync(kAll, dist, src);
+        const int id = __shfl_sync(kAll, __float_as_int(p.w), src);
+        const bool fill = todo && size < kBallBuf, swap = todo && !fill && x < farthest;
+        if (fill || swap) {
+          const int slot = fill ? size : at;
+          if (sl == slot) held = x, held_id = id;
+        }
+        if (fill) {
+          if (farthest > x) farthest = x, at = size;
+          size++;
+        }
+        if (__any_sync(kAll, swap)) {  // the new maximum: the slot just filled if it holds it, else the first that does
+          float top = sl < kBallBuf ? held : -1.0f;
+#pragma unroll
+          for (int o = kBallBuf / 2; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(kAll, top, o));
+          top = __shfl_sync(kAll, top, gb);
+          const unsigned tops = __ballot_sync(kAll, sl < kBallBuf && held == top) & gmask;
+          if (swap) {
+            if (top != x) at = __ffs(tops) - 1 - gb;
+            farthest = top;
+            settled = true;
+          }
+        }
+        todo &= todo - 1;
+      }
+    }
+    if (on) {
+      int* row = a.pc_idx + (slot0 + s) * P;
+      if (sl < kBallBuf && sl < P) row[sl] = sl < size ? held_id : -1;
+      for (int e = kBallBuf + sl; e < P; e += L) row[e] = -1;
+    }
+  }
+  if ((walks >> lane) & 1u) default_slots(a, (size_t)ray, emitted, sl, L);
+  return over;
+}
+
+// All that serve_rays leaves; one call, out of line: called one by one, the two
+// took registers from the rays that never come here (shapes view 446 us, so 425).
+template <class J>
+__device__ __noinline__ void serve_left(const SampleArgs& a, int L, int4 entry, unsigned char* pool, int entries,
+                                        Unsettled left, unsigned over) {
+#ifdef HP_TESTING  // by the general walk, to hold serve_exact against it
+  over |= __ballot_sync(0xffffffffu, left.n < 0 || left.emitted < 0 || left.balls);
+#else
+  over |= serve_exact(a, L, entry, pool, entries, left);
+#endif
+  while (over) {  // the general walk, ray by ray
+    const int l = __ffs(over) - 1;
+    over &= ~((0xffffffffu >> (32 - L)) << l);
+    const int ray = __shfl_sync(0xffffffffu, entry.x, l);
+    __syncwarp();
+    sample_ray_warp<J>(a, ray / a.cam.width, ray % a.cam.width, reinterpret_cast<unsigned*>(pool));
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1190,13 +1434,10 @@ __device__ __forceinline__ void serve_list(const SampleArgs& a0, const SampleArg
     const int L = back ? 32 : 8;
     const int4 e = __ldg(back ? rl.rays + (rl.cap - 1 - (long long)i) : rl.rays + (size_t)i * 4 + (lane >> 3));
     if constexpr (kBatch) view_args(back ? rl.back_view[i] : rl.front_view[i]);
-    for (unsigned odd = serve_rays(a, L, e, pool, Cfg::kEntries); odd;) {  // the general walk, ray by ray
-      const int l = __ffs(odd) - 1;
-      odd &= ~((0xffffffffu >> (32 - L)) << l);
-      const int ray = __shfl_sync(0xffffffffu, e.x, l);
-      __syncwarp();
-      sample_ray_warp<typename Cfg::Index>(a, ray / a.cam.width, ray % a.cam.width, reinterpret_cast<unsigned*>(pool));
-    }
+    Unsettled left;
+    const unsigned over = serve_rays(a, L, e, pool, Cfg::kEntries, left);
+    if (__any_sync(0xffffffffu, left.n < 0 || left.emitted < 0 || left.balls) || over)
+      serve_left<typename Cfg::Index>(a, L, e, pool, Cfg::kEntries, left, over);
     __syncwarp();
     i++;
   }

@@ -9,8 +9,9 @@
  *
  * In that library small tables take the paths of windows whose candidates pass
  * 2^31, with the same outputs: hp_quick_query_for_nearby_point numbers at most
- * 64 candidates of a window at once, and hp_quick_sampling's general walk counts
- * in 64 bits for views of more than 40 ids (the product: 2^26).
+ * 64 candidates of a window at once, and hp_quick_sampling's general walk, which
+ * serves every ray that its fast arithmetic leaves, counts in 64 bits for views
+ * of more than 40 ids (the product: 2^26).
  */
 #ifndef HASHPOINT_B200_TESTING_H
 #define HASHPOINT_B200_TESTING_H

@@ -97,25 +97,55 @@ def _reversed_buckets(sidx, table):
     return torch.from_numpy(out).cuda(), torch.from_numpy(h).cuda()
 
 
-@pytest.mark.parametrize("n,size,k,radius", [w[:4] for w in WINDOWS if w[2] <= 5] + [(60_000, (40, 31), 5, 0.03),
-                                                                                    (60_000, (33, 16), 2, 0.5)])
-def test_sampling_walk_in_64_bit_indices(n, size, k, radius):
-    """The test library's general walk numbers a window's candidates in 64 bits: the same bytes."""
+def _cloud(kind, n, rng):
+    xyz = synth.shapes_cloud(rng, n)
+    if kind == "twins":  # every point three times
+        xyz = np.repeat(xyz[:n // 3], 3, 0)[rng.permutation(n // 3 * 3)]
+    if kind == "lattice":
+        xyz = np.round(xyz / 0.004) * 0.004
+    return xyz.astype(np.float32)
+
+
+SHAPED = dict(radius_threshold=0.03)
+SLOW = dict(radius_threshold=0.05, sdf2weight_gaussian_gamma=0.05, num_sample_points_per_ray=40, num_point_cloud_per_sp=11)
+
+
+@pytest.mark.parametrize("kind,n,size,opt", [
+    ("shapes", 20_000, (60, 45), SHAPED), ("shapes", 60_000, (40, 31), SHAPED),
+    ("shapes", 60_000, (33, 16), dict(kernel_size=2, radius_threshold=0.5)),
+    ("shapes", 2_000, (1, 1), dict(radius_threshold=5.0)),
+    ("shapes", 3_000, (3, 200), SHAPED), ("shapes", 3_000, (200, 2), dict(kernel_size=4, radius_threshold=0.06)),  # repeated cells
+    ("twins", 20_000, (60, 45), SHAPED), ("twins", 60_000, (40, 31), SHAPED), ("twins", 20_000, (61, 40), SLOW),
+    ("lattice", 30_000, (97, 61), SHAPED), ("lattice", 90_000, (40, 31), SLOW),
+    # mean distances that the quantised sums cannot tell apart, for all rays or for some
+    ("shapes", 20_000, (60, 45), dict(SLOW, sdf2weight_gaussian_alpha=0.0005)),
+    ("shapes", 20_000, (60, 45), dict(SLOW, sdf2weight_gaussian_alpha=0.005)),
+    ("shapes", 9_000, (40, 33), dict(kernel_size=3, radius_threshold=1e-16)),
+    ("shapes", 9_000, (40, 33), dict(kernel_size=3, radius_threshold=1e16)),
+    ("shapes", 20_000, (60, 45), dict(SHAPED, sdf2weight_gaussian_alpha=0.0)),
+    ("shapes", 20_000, (60, 45), dict(SHAPED, sdf2weight_gaussian_alpha=-0.2, sdf2weight_gaussian_gamma=-0.1)),
+])
+def test_left_rays_by_lists_and_by_the_general_walk(kind, n, size, opt):
+    """The test library serves every ray that the fast arithmetic leaves by the general walk, in 64-bit indices, and a table
+    in reversed pixel order leaves every ray with two filled cells in a window row: the same bytes three times."""
     native.build_testing()
     T = native.testing_lib()
-    cam = synth.look_at_camera((0.3, 0.2, 4.0), (0, 0, 0), *size, 0.5 * size[0])
-    X, c2w, sidx, table = _view(synth.shapes_cloud(np.random.default_rng(n), n), cam)
-    o = synth.Options(kernel_size=k, radius_threshold=radius, num_point_cloud_per_sp=8)
+    cam = synth.look_at_camera((0.3, 0.2, 4.0), (0, 0, 0), *size, 0.5 * max(size))
+    X, c2w, sidx, table = _view(_cloud(kind, n, np.random.default_rng(n)), cam)
+    sidx[::50] = n + 7  # ids beyond the cloud are skipped
+    o = synth.Options(**{"num_point_cloud_per_sp": 8, **opt})
     want = _sample(X, c2w, cam, o, sidx, table)
-    sidx, table = _reversed_buckets(sidx, table)
+    turned = _reversed_buckets(sidx, table)
+    assert all(torch.equal(a, b) for a, b in zip(_sample(X, c2w, cam, o, *turned), want))
     got = [torch.empty_like(t) for t in want]
     spec = ops.make_camera(c2w=c2w, fx=cam.fx, fy=cam.fy, cx=cam.cx, cy=cam.cy, width=cam.width, height=cam.height)
     ws = torch.empty(T.hp_quick_sampling_workspace_size(len(sidx), size[1], size[0]), dtype=torch.uint8, device="cuda")
-    rc = T.hp_quick_sampling(X.data_ptr(), len(X), spec, ops.make_options(o), sidx.data_ptr(), len(sidx), table.data_ptr(),
-                             *[t.data_ptr() for t in got], ws.data_ptr(), len(ws),
-                             torch.cuda.current_stream().cuda_stream)
-    native.check(rc, "hp_quick_sampling", T)
-    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    for s, h in ((sidx, table), turned):
+        rc = T.hp_quick_sampling(X.data_ptr(), len(X), spec, ops.make_options(o), s.data_ptr(), len(s), h.data_ptr(),
+                                 *[t.data_ptr() for t in got], ws.data_ptr(), len(ws),
+                                 torch.cuda.current_stream().cuda_stream)
+        native.check(rc, "hp_quick_sampling", T)
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
 
 
 def test_query_window_beyond_two_to_the_31():
@@ -189,3 +219,17 @@ def test_query_long_and_short_lists_agree():
     assert (long >= 0).any()
     for a, b in ((0, (1 << 17) - 1), (4, 5), (1 << 17, (1 << 17) + 3)):
         assert torch.equal(_query(X, c2w, cam, o, sidx, table, rays[a:b].contiguous()), long[a:b])
+
+
+@pytest.mark.parametrize("kind,opt", [("twins", {}), ("lattice", {}), ("shapes", dict(sdf2weight_gaussian_alpha=0.0001))])
+def test_ties_cost_little(kind, opt):
+    """Equal distances (repeated or lattice points) and close mean distances leave most rays to exact arithmetic: at most
+    three times the time of a cloud without them (a walk of its own for each such ray: six times)."""
+    cam = synth.look_at_camera((0.3, 0.2, 4.0), (0, 0, 0), 400, 400, 555.0)
+
+    def call(kind, **opt):
+        X, c2w, sidx, table = _view(_cloud(kind, 300_000, np.random.default_rng(5)), cam)
+        o = synth.Options(radius_threshold=0.016, num_sample_points_per_ray=8, num_point_cloud_per_sp=8, **opt)
+        return _time(lambda: _sample(X, c2w, cam, o, sidx, table))
+
+    assert call(kind, **opt) < 3 * call("shapes")
