@@ -66,7 +66,7 @@ namespace hp {
 
 constexpr int kTeReg = 4;        // emitted sample depths kept in registers (sample_ray_warp)
 constexpr int kBallPass = 2;     // samples served by one ball-query walk
-constexpr int kHeavyWindow = 320;  // default: rays with more window candidates get a whole warp
+constexpr int kHeavyWindow = 240;  // default: rays with more window candidates get a whole warp (8 lanes hold 240 to 256)
 constexpr int kMaxHeavyWindow = 4096;  // largest tunable threshold
 constexpr int kWalkBatch = 4;    // bins whose sums one walk pass of sample_ray_warp gathers
 constexpr int kClasses = 64;     // window-size classes a tile's rays are ordered by

@@ -185,7 +185,7 @@ class Autotuner:
     Candidates are timed with CUDA events on the renderer's own batch; the
     cache is filled once per class and then only read."""
 
-    HEAVY = (224, 320)
+    HEAVY = (96, 240)  # 8 lanes hold at least 240 candidates of a ray in every configuration
     STAGES = native.STAGE_CONFIGS
 
     def __init__(self, reps=3):

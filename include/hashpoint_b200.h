@@ -251,8 +251,9 @@ HP_API size_t hp_quick_sampling_workspace_size(int64_t n_sorted, int32_t height,
 /* Launch tuning of hp_quick_sampling_tuned and hp_quick_sampling_batch (NULL
  * or 0 fields = defaults).  Outputs never depend on it.
  *   heavy_window   rays whose window holds more candidates are served by a
- *                  whole warp instead of 8 lanes (0..4096; default 320, and at
- *                  most what 8 lanes hold on chip: stage_points / 16).
+ *                  whole warp instead of 8 lanes (0..4096; default 240; values
+ *                  above what 8 lanes hold on chip, stage_points / 16, act as
+ *                  that).
  *   blocks_per_sm  resident blocks of the persistent sampling kernel per SM
  *                  (default: as many as fit).
  *   stage_config   candidates a block holds on chip, resident blocks, and the
