@@ -120,30 +120,15 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int m, int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, M x N x 16; issued by one thread.
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                         uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// Arrive on bar when every tcgen05 operation this thread issued so far has completed.
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar))
-               : "memory");
-}
-
-// --- the same, called by a converged warp: one lane (the same each time) issues --
+// --- MMA, commit, copy: called by a converged warp, one lane (the same each time) issues --
 // In a branch of one lane the operands of each tcgen05 or bulk instruction are
 // per-thread values that the warp has to move to uniform registers first; called
 // by the whole warp with elect.sync's predicate they are uniform to begin with
 // (two MMAs and their commit took 230 cycles in a branch; a forward of 143,000
 // samples x 8 went from 897 to 832 us with the MMAs issued so, to 762 with the
 // copies too).
+//
+// D[tmem] (+)= A[smem] * B[smem]^T, M x N x 16.
 __device__ __forceinline__ void warp_mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                               uint32_t accumulate) {
   asm volatile(
@@ -155,6 +140,7 @@ __device__ __forceinline__ void warp_mma_bf16(uint32_t d_tmem, uint64_t a_desc, 
       : "memory");
 }
 
+// Arrive on bar when every tcgen05 operation the lane issued so far has completed.
 __device__ __forceinline__ void warp_commit(uint64_t* bar) {
   asm volatile(
       "{\n\t.reg .pred e;\n\t"

@@ -47,8 +47,8 @@ EXPORTS = ["hp_version", "hp_last_error", "hp_projection_rounding", "hp_pts2plan
            "hp_clamp_t", "hp_render", "hp_aggregator_packed_size", "hp_aggregator_pack",
            "hp_aggregator_workspace_size", "hp_aggregator_forward", "hp_aggregator_status"]
 # declared in include/hashpoint_b200_testing.h, exported by the test-only library
-TESTING_EXPORTS = ["hp_tc_check_image_bytes", "hp_tc_check_mma", "hp_aggregator_forward_withheld",
-                   "hp_pts2plane_withheld"]
+TESTING_EXPORTS = ["hp_tc_check_image_bytes", "hp_tc_check_mma", "hp_tc_check_mma2",
+                   "hp_aggregator_forward_withheld", "hp_pts2plane_withheld"]
 
 HP_OK = 0
 
@@ -304,6 +304,8 @@ def testing_lib():
         T.hp_tc_check_image_bytes.restype = sz
         T.hp_tc_check_mma.argtypes = [vp, vp, i32, ctypes.c_uint32, i32, ctypes.c_uint32, vp, vp]
         T.hp_tc_check_mma.restype = i32
+        T.hp_tc_check_mma2.argtypes = [vp, vp, i32, ctypes.c_uint32, i32, ctypes.c_uint32, i32, vp, vp]
+        T.hp_tc_check_mma2.restype = i32
         T.hp_aggregator_workspace_size.argtypes = [i64]
         T.hp_aggregator_workspace_size.restype = sz
         T.hp_aggregator_status.argtypes = [vp, i64, vp]

@@ -40,6 +40,12 @@ enum { HP_TC_PLAIN = 0, HP_TC_SW128 = 1, HP_TC_SW64 = 2 };
 HP_API size_t hp_tc_check_image_bytes(int32_t operand);
 HP_API int32_t hp_tc_check_mma(const void* a_image, const void* b_image, int32_t a_form, uint32_t a_offset,
                                int32_t b_form, uint32_t b_offset, float* d, hp_stream_t stream);
+/* The same for the pair of K = 16 steps and its commit that the Aggregator's
+ * pair kernel issues a weight chunk with: K = 32 columns from the offsets on, a
+ * swizzled row of them (HP_TC_SW128 or HP_TC_SW64).  accumulate != 0: added to
+ * the product of the first 16 columns, which hp_tc_check_mma computes. */
+HP_API int32_t hp_tc_check_mma2(const void* a_image, const void* b_image, int32_t a_form, uint32_t a_offset,
+                                int32_t b_form, uint32_t b_offset, int32_t accumulate, float* d, hp_stream_t stream);
 
 /* A test of the Aggregator's bounded waits: hp_aggregator_forward with one
  * weight block (block3.0's extra-input columns) never loaded into the pair
