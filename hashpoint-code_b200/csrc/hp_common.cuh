@@ -30,13 +30,11 @@
 
 namespace hp {
 
-constexpr int kWarp = 32;
-constexpr int kLaneCells = 32;     // window cells one sampling warp of the reference covers (k*k <= 32)
 constexpr int kKeptPerCell = 48;   // kept points per window cell (POINT_BUFFER_SIZE48)
 constexpr int kBins = 128;         // t-histogram bins (MAX_SAMPLE_POINTS_NUM)
 constexpr int kBallBuf = 8;        // ids gathered per sample (POINT_BUFFER_SIZE8)
 constexpr int kQueryPerCell = 32;  // ids gathered per window cell by the ray query (POINT_BUFFER_SIZE)
-constexpr int kMaxKernel = 5;      // largest window side of the sampling path (k*k <= 32)
+constexpr int kMaxKernel = 5;      // largest window side of the sampling path (the reference's warps cover 32 cells)
 
 // Camera as the kernels see it: c2w stays a device pointer (rows 0..2 read).
 struct DevCamera {
@@ -82,17 +80,6 @@ __device__ __forceinline__ void make_ray(const float* __restrict__ c2w, float fx
 #pragma unroll
   for (int i = 0; i < 3; i++) r.d[i] = __fmul_rn(d[i], rn);
   r.dd = dot3(r.d[0], r.d[1], r.d[2], r.d[0], r.d[1], r.d[2]);
-}
-
-// PointRayInterset (cuda_util.cuh:215-236): t = (p-o).d / d.d, proj = fma(t, d, o),
-// dist = norm3df(p - proj).
-__device__ __forceinline__ void intersect(const Ray& r, float px, float py, float pz, float& t, float& dist) {
-  const float s0 = __fsub_rn(px, r.o[0]), s1 = __fsub_rn(py, r.o[1]), s2 = __fsub_rn(pz, r.o[2]);
-  t = __fdiv_rn(dot3(s0, s1, s2, r.d[0], r.d[1], r.d[2]), r.dd);
-  const float e0 = __fsub_rn(px, __fmaf_rn(t, r.d[0], r.o[0]));
-  const float e1 = __fsub_rn(py, __fmaf_rn(t, r.d[1], r.o[1]));
-  const float e2 = __fsub_rn(pz, __fmaf_rn(t, r.d[2], r.o[2]));
-  dist = norm3df(e0, e1, e2);
 }
 
 // calculate_neighbor_uv (cuda_util.cuh:382-388) in exact integer form:
@@ -147,11 +134,14 @@ __device__ __forceinline__ bool within_radius(const RadiusTest& rt, bool in, flo
   return kept;
 }
 
-// PointRayInterset's t (cuda_util.cuh:227): the correctly rounded quotient of
-// (p - o).d and d.d, with inv_dd = RN(1 / d.d): a first quotient, its exact
-// residual and one fused step (Markstein 1990).  d is normalised, so d.d is a
-// few ulp from 1; for every d.d within 64 ulp of 1 and every numerator mantissa
-// this equals the division, at 3 instructions for 10 and without its branch.
+// PointRayInterset (cuda_util.cuh:215-236): t = (p - o).d / d.d, the point's
+// projection on the ray fma(t, d, o), its distance norm3df(p - projection).
+// ray_t is t, the correctly rounded quotient, with inv_dd = RN(1 / d.d): a first
+// quotient, its exact residual and one fused step (Markstein 1990).  d is
+// normalised, so d.d is a few ulp from 1; for every d.d within 64 ulp of 1 and
+// every numerator mantissa this equals the division, at 3 instructions for 10
+// and without its branch.  (Numerators below 2^-100 and from 2^127 on, whose
+// residual or quotient leaves the normal range, are not covered.)
 __device__ __forceinline__ float ray_t(const Ray& r, float inv_dd, const float4& p) {
   const float num = dot3(__fsub_rn(p.x, r.o[0]), __fsub_rn(p.y, r.o[1]), __fsub_rn(p.z, r.o[2]), r.d[0], r.d[1], r.d[2]);
   const float q = __fmul_rn(num, inv_dd);
