@@ -44,7 +44,6 @@ constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 4;                    // counts per thread in the scan
 constexpr int kScanTile = kScanThreads * kScanItems;
 constexpr int kHugeThreads = 512;
-constexpr int kOrderThreads = 512;
 // Look-back words of the scan: a status bit above the tile's total in the
 // low 32 bits (0 = not yet published).
 constexpr unsigned long long kAggregate = 1ull << 62;
@@ -309,6 +308,8 @@ __device__ __forceinline__ unsigned long long entry_key(const BucketOrder& bo, i
 // Bucket entries in position order: hp_pts2plane's packed scratch records,
 // which carry their bucket ...
 struct PackedEntries {
+  static constexpr int kOrderThreads = 512;
+  static constexpr bool kListed = true;  // k_scan_hash lists the buckets above kRankMax
   const int4* rec;  // (id, depth bits, bucket start, bucket count)
   // entry j: its bucket (start, count) and (id, depth bits); false if none
   __device__ __forceinline__ bool entry(int j, const int2*, int, int2& bucket, int2& e) const {
@@ -324,6 +325,8 @@ struct PackedEntries {
 // ... or the caller's sorted arrays (hp_scatter_hashtable), whose buckets come
 // from the hash table.
 struct SplitEntries {
+  static constexpr int kOrderThreads = 256;
+  static constexpr bool kListed = false;
   const int* id;
   const float* depth;
   const int* pid;
@@ -361,7 +364,7 @@ __device__ __forceinline__ void cx_global(const BucketOrder& bo, int* idx, float
 // place in global memory after copying it from the scratch entries (indexed by
 // position).
 template <class Entries>
-__device__ __noinline__ void sort_bucket(int2 h, Entries in, int* __restrict__ out_idx, float* __restrict__ out_depth,
+__device__ __forceinline__ void sort_bucket(int2 h, Entries in, int* __restrict__ out_idx, float* __restrict__ out_depth,
                                             const BucketOrder& bo) {
   const int c = h.y;
   int* idx = out_idx + h.x;
@@ -395,24 +398,34 @@ __device__ __noinline__ void sort_bucket(int2 h, Entries in, int* __restrict__ o
   __syncthreads();
 }
 
+template <class Entries, int kByDepth, int kByPosition>
+__device__ __noinline__ void sort_listed(int2 h, Entries in, int* __restrict__ out_idx, float* __restrict__ out_depth) {
+  sort_bucket(h, in, out_idx, out_depth, BucketOrder{kByDepth, kByPosition});
+}
+
 // One thread per entry j < n_in of the scratch copy: rank among the entries of
 // its bucket -> final position.  Buckets of one entry are copied; buckets above
 // kRankMax come from the list `huge` (hp_pts2plane), one CTA each, or are left
 // to k_sort_huge_scan.  A launch of its own for that list cost every view 3 us
 // to find it empty (a build of 100k points, 48.3 -> 42.7 us with one memset
-// less); blocks of kOrderThreads sort a huge bucket as fast as it did (256
-// threads: 1.9x slower), and rank as fast as blocks of 256.  The order mode
+// less); blocks of 512 sort a huge bucket as fast as it did (256 threads: 1.9x
+// slower), out of line so that the ranking keeps its registers.  Where there is
+// no list, blocks of 256 rank faster and the scan sorts in line (1M points in 400
+// buckets by depth: 40.4 -> 34.9 ms; in 640,000: 35.8 -> 33.8 us).  The order mode
 // is a template argument so that the rank loop -- the kernel's instructions
 // are mostly its iterations -- compares ids alone when ordering by id.
 template <class Entries, int kByDepth, int kByPosition>
-__global__ void __launch_bounds__(kOrderThreads) k_order(Entries in, const int2* __restrict__ hash, int hw,
+__global__ void __launch_bounds__(Entries::kOrderThreads) k_order(Entries in, const int2* __restrict__ hash, int hw,
                                                const int* __restrict__ scalars, int n_fixed,
                                                const int* __restrict__ huge, int* __restrict__ out_idx,
                                                float* __restrict__ out_depth) {
   const BucketOrder bo{kByDepth, kByPosition};
   const int n_in = n_fixed >= 0 ? n_fixed : scalars[0];
-  const int n_huge = huge ? scalars[1] : 0;
-  for (int q = blockIdx.x; q < n_huge; q += gridDim.x) sort_bucket(hash[huge[q]], in, out_idx, out_depth, bo);
+  if constexpr (Entries::kListed) {
+    const int n_huge = scalars[1];
+    for (int q = blockIdx.x; q < n_huge; q += gridDim.x)
+      sort_listed<Entries, kByDepth, kByPosition>(hash[huge[q]], in, out_idx, out_depth);
+  }
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n_in; j += gridDim.x * blockDim.x) {
     int2 h, e;
     if (!in.entry(j, hash, hw, h, e)) continue;
@@ -529,22 +542,23 @@ static int grid_for(int64_t n, int threads) {
 
 // Bucket order shared by hp_pts2plane (packed scratch records, count on the
 // device) and hp_scatter_hashtable (entries in the caller's sorted input).
-// huge: the list of buckets above kRankMax (count in scalars[1]), or null to
-// find them by scanning the hash table.
+// huge: the list of buckets above kRankMax (count in scalars[1]) of entries
+// that have one; others' are found by scanning the hash table.
 template <class Entries>
 static int32_t launch_order(int hw, int n_fixed, int n_grid, Entries in, const int2* hash, const int* scalars,
                             const int* huge, int* out_idx, float* out_depth, BucketOrder bo, cudaStream_t st) {
   if (n_grid > 0) {
-    const int g = grid_for(n_grid, kOrderThreads);
+    constexpr int kThreads = Entries::kOrderThreads;
+    const int g = grid_for(n_grid, kThreads);
     if (!bo.by_depth && !bo.by_position)
-      k_order<Entries, 0, 0><<<g, kOrderThreads, 0, st>>>(in, hash, hw, scalars, n_fixed, huge, out_idx, out_depth);
+      k_order<Entries, 0, 0><<<g, kThreads, 0, st>>>(in, hash, hw, scalars, n_fixed, huge, out_idx, out_depth);
     else if (!bo.by_position)
-      k_order<Entries, 1, 0><<<g, kOrderThreads, 0, st>>>(in, hash, hw, scalars, n_fixed, huge, out_idx, out_depth);
+      k_order<Entries, 1, 0><<<g, kThreads, 0, st>>>(in, hash, hw, scalars, n_fixed, huge, out_idx, out_depth);
     else
-      k_order<Entries, 1, 1><<<g, kOrderThreads, 0, st>>>(in, hash, hw, scalars, n_fixed, huge, out_idx, out_depth);
+      k_order<Entries, 1, 1><<<g, kThreads, 0, st>>>(in, hash, hw, scalars, n_fixed, huge, out_idx, out_depth);
     if (int32_t rc = check_launch("k_order")) return rc;
   }
-  if (huge) return HP_OK;  // k_order sorted those listed
+  if constexpr (Entries::kListed) return HP_OK;  // k_order sorted those
   const int blocks = (hw + kHugeThreads - 1) / kHugeThreads < 148 * 2 ? (hw + kHugeThreads - 1) / kHugeThreads : 148 * 2;
   k_sort_huge_scan<<<blocks, kHugeThreads, 0, st>>>(hw, in, hash, out_idx, out_depth, bo);
   return check_launch("k_sort_huge_scan");
