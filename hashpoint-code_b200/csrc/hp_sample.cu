@@ -729,7 +729,8 @@ __device__ __forceinline__ unsigned serve_rays(const SampleArgs& a, const int L,
               c3 = __shfl_sync(kAll, cnt, gb + 3), c4 = __shfl_sync(kAll, cnt, gb + 4);
     p1 = c0, p2 = (int)((unsigned)p1 + c1), p3 = (int)((unsigned)p2 + c2), p4 = (int)((unsigned)p3 + c3);
     T = (int)((unsigned)p4 + c4);
-    good = good && (p2 | p3 | p4 | T) >= 0;  // (clamped rows repeat: their sum may pass 2^31)
+    // clamped rows repeat: their sum may pass 2^31 (less what the passes number beyond it)
+    good = good && (p2 | p3 | p4 | T | (int)((unsigned)T + 64u)) >= 0;
     base = __shfl_sync(kAll, first, gb);
     const int f1 = __shfl_sync(kAll, first, gb + 1), f2 = __shfl_sync(kAll, first, gb + 2),
               f3 = __shfl_sync(kAll, first, gb + 3), f4 = __shfl_sync(kAll, first, gb + 4);
@@ -807,6 +808,7 @@ __device__ __forceinline__ unsigned serve_rays(const SampleArgs& a, const int L,
       const int pos = n + __popc(nm & below);
       if (near && pos < cap) list[pos] = kept ? idx : idx | (int)0x80000000u;
       n += __popc(nm & gmask);
+      if (L == 32 && n > cap) break;  // the general walk's (8 lanes hold every window they get)
       idx = idx_n;
       p = pn;
     }
@@ -1008,8 +1010,8 @@ __device__ __forceinline__ unsigned serve_rays(const SampleArgs& a, const int L,
   return over;
 }
 
-// The rays that serve_rays left, as it serves them: their list (made here cell
-// by cell where there is none), the walk over sums of norm3df added in window
+// The rays that serve_rays left, as it serves them: their list (made here from
+// the cells where there is none), the walk over sums of norm3df added in window
 // order, a ray at a time by the whole warp, and the point selection with buffers
 // of norm3df in slot order, the warp's rays side by side.  Returns the lanes of
 // groups whose list overflows.
@@ -1018,7 +1020,8 @@ __device__ __forceinline__ unsigned serve_rays(const SampleArgs& a, const int L,
 // rays come here (repeated or lattice points, whose distances tie) the whole
 // view waited for that.  1M points at 800 x 800, sampling alone: each place
 // three times 2910 us with it, 640 so (980 with one thread a ray); rounded to a
-// lattice 2360 and 590 (880); buckets out of pixel order 1980 and 950 (860).
+// lattice 2360 and 580 (880); buckets out of pixel order 1980 and 834 (865; 950
+// with a cell at a time).
 __device__ __forceinline__ unsigned serve_exact(const SampleArgs& a, int L, int4 entry, unsigned char* pool, int entries,
                                              Unsettled left) {
   constexpr unsigned kAll = 0xffffffffu;
@@ -1040,7 +1043,7 @@ __device__ __forceinline__ unsigned serve_exact(const SampleArgs& a, int L, int4
   int n = left.n, emitted = left.emitted;
   bool balls = left.balls;
 
-  // the list of a window whose rows are no runs
+  // the list of a window whose rows are no runs: L cells at a time, their candidates numbered through
   if (__any_sync(kAll, n < 0)) {
     const bool make = n < 0;
     n = make ? 0 : n;
@@ -1049,15 +1052,29 @@ __device__ __forceinline__ unsigned serve_exact(const SampleArgs& a, int L, int4
     const float omax = fmaxf(fabsf(r.o[0]), fmaxf(fabsf(r.o[1]), fabsf(r.o[2])));
     const float c0 = __fmaf_rn(1e-5f, 1.0f + omax, a.near0);
     const int v = make ? ray / W : 0, u = make ? ray - v * W : 0;
-    for (int c = 0; c < k * k; c++) {
+    for (int cell0 = 0; cell0 < k * k; cell0 += L) {
+      const int l = cell0 + sl;
       int2 rg = make_int2(0, 0);
-      if (make) rg = cell_range(a, min(max(v + c / k - lo, 0), H - 1), min(max(u + c % k - lo, 0), W - 1));
-      const unsigned count = (unsigned)(rg.y - rg.x);
-      int had = 0;  // kept of this cell
-      for (unsigned j0 = 0; __any_sync(kAll, j0 < count); j0 += (unsigned)L) {
-        const int idx = rg.x + (int)(j0 + sl);
+      if (make && l < k * k) rg = cell_range(a, min(max(v + l / k - lo, 0), H - 1), min(max(u + l % k - lo, 0), W - 1));
+      const unsigned cnt = (unsigned)(rg.y - rg.x);
+      unsigned pre = cnt;
+      for (int o = 1; o < L; o <<= 1) {
+        const unsigned t = __shfl_up_sync(kAll, pre, o);
+        if (sl >= o) pre = min(pre + t, 0x7fffffffu);  // both below 2^31
+      }
+      unsigned total = __shfl_sync(kAll, pre, gb + L - 1);
+      if (total == 0x7fffffffu) n = cap + 1;  // too many to number: the general walk's
+      pre -= cnt;
+      int carry = 0;  // this lane's cell: kept so far
+      for (unsigned j0 = 0; __any_sync(kAll, j0 < total && n <= cap); j0 += (unsigned)L) {
+        const unsigned j = j0 + sl;
+        int c = gb;
+        for (int s = L >> 1; s > 0; s >>= 1)
+          if (__shfl_sync(kAll, pre, c + s) <= j) c += s;
+        const unsigned first = __shfl_sync(kAll, pre, c);
+        const int idx = __shfl_sync(kAll, rg.x, c) + (int)(j - first);
         float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-        bool in = j0 + sl < count;
+        bool in = j < total && n <= cap;
         if (in) p = __ldg(a.pts + idx);
         in = in && __float_as_int(p.w) >= 0;
         const float t = ray_t(r, inv_dd, p);
@@ -1068,8 +1085,10 @@ __device__ __forceinline__ unsigned serve_exact(const SampleArgs& a, int L, int4
         bool kept = within_radius(rt, in, q, e0, e1, e2);
         const bool near = kept || (in && q <= near_limit(c0, t));
         const unsigned km = __ballot_sync(kAll, kept), nm = __ballot_sync(kAll, near);
-        kept = kept && had + __popc(km & below) < kKeptPerCell;
-        had = min(had + __popc(km & gmask), kKeptPerCell);
+        auto lane_of = [&](unsigned x) { return gb + min(max((int)(x - j0), 0), L); };  // of candidate x
+        const int had = __shfl_sync(kAll, carry, c) + __popc(km & below & ~lane_span(0, lane_of(first)));
+        kept = kept && had < kKeptPerCell;
+        carry = min(carry + __popc(km & lane_span(lane_of(pre), lane_of(pre + cnt))), kKeptPerCell);
         const int pos = n + __popc(nm & below);
         if (near && pos < cap) list[pos] = kept ? idx : idx | (int)0x80000000u;
         n = min(n + __popc(nm & gmask), cap + 1);

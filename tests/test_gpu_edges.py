@@ -85,6 +85,17 @@ def test_query_windows_taken_in_rounds(n, size, k, radius, cap):
     assert torch.equal(_query(X, c2w, cam, o, sidx, table, rays, native.testing_lib()), want)
 
 
+def _sample_by(L, X, c2w, cam, o, sidx, table):
+    """quick_sampling by the library L."""
+    out = ops.sampling_outputs(cam.height, cam.width, o, "cuda")
+    spec = ops.make_camera(c2w=c2w, fx=cam.fx, fy=cam.fy, cx=cam.cx, cy=cam.cy, width=cam.width, height=cam.height)
+    ws = torch.empty(L.hp_quick_sampling_workspace_size(len(sidx), cam.height, cam.width), dtype=torch.uint8, device="cuda")
+    rc = L.hp_quick_sampling(X.data_ptr(), len(X), spec, ops.make_options(o), sidx.data_ptr(), len(sidx), table.data_ptr(),
+                             *[t.data_ptr() for t in out], ws.data_ptr(), len(ws), torch.cuda.current_stream().cuda_stream)
+    native.check(rc, "hp_quick_sampling", L)
+    return out
+
+
 def _reversed_buckets(sidx, table):
     """The same buckets, stored last pixel first: rays with two non-empty cells in a window row take the general walk."""
     sidx, h = sidx.cpu().numpy(), table.cpu().numpy().copy()
@@ -137,15 +148,8 @@ def test_left_rays_by_lists_and_by_the_general_walk(kind, n, size, opt):
     want = _sample(X, c2w, cam, o, sidx, table)
     turned = _reversed_buckets(sidx, table)
     assert all(torch.equal(a, b) for a, b in zip(_sample(X, c2w, cam, o, *turned), want))
-    got = [torch.empty_like(t) for t in want]
-    spec = ops.make_camera(c2w=c2w, fx=cam.fx, fy=cam.fy, cx=cam.cx, cy=cam.cy, width=cam.width, height=cam.height)
-    ws = torch.empty(T.hp_quick_sampling_workspace_size(len(sidx), size[1], size[0]), dtype=torch.uint8, device="cuda")
     for s, h in ((sidx, table), turned):
-        rc = T.hp_quick_sampling(X.data_ptr(), len(X), spec, ops.make_options(o), s.data_ptr(), len(s), h.data_ptr(),
-                                 *[t.data_ptr() for t in got], ws.data_ptr(), len(ws),
-                                 torch.cuda.current_stream().cuda_stream)
-        native.check(rc, "hp_quick_sampling", T)
-        assert all(torch.equal(a, b) for a, b in zip(got, want))
+        assert all(torch.equal(a, b) for a, b in zip(_sample_by(T, X, c2w, cam, o, s, h), want))
 
 
 def test_query_window_beyond_two_to_the_31():
@@ -233,3 +237,17 @@ def test_ties_cost_little(kind, opt):
         return _time(lambda: _sample(X, c2w, cam, o, sidx, table))
 
     assert call(kind, **opt) < 3 * call("shapes")
+
+
+def test_a_window_that_cannot_be_listed_is_not_walked_twice():
+    """One pixel of 50,000 points, its bucket in every window cell: the list made from the cells ends once it is full, so the
+    ray takes no longer than its general walk, which for one sample passes over all of it once."""
+    native.build_testing()
+    T = native.testing_lib()
+    cam = synth.look_at_camera((0.3, 0.2, 4.0), (0, 0, 0), 1, 1, 0.5)
+    X, c2w, sidx, table = _view(synth.shapes_cloud(np.random.default_rng(2), 50_000), cam)
+    o = synth.Options(radius_threshold=5.0, num_sample_points_per_ray=1, num_point_cloud_per_sp=8)
+    walk = lambda: _sample_by(T, X, c2w, cam, o, sidx, table)
+    here = lambda: _sample(X, c2w, cam, o, sidx, table)
+    assert all(torch.equal(a, b) for a, b in zip(here(), walk()))
+    assert _time(here, 5) < 1.3 * _time(walk, 5)
