@@ -325,7 +325,7 @@ def run_gpu(args):
     traffic = None
     try:
         tr = json.load(open(os.path.join(ROOT, "profiles", "traffic.json")))
-        traffic = tr.get("k_quick_sampling", {}).get(WORKLOAD)
+        traffic = tr.get("k_quick_sampling", {}).get(WORKLOAD, {}).get("stage_config %d" % stage)
     except (OSError, ValueError):
         pass
 
