@@ -111,6 +111,7 @@ constexpr size_t kW3bOff = kPairBytes;
 constexpr size_t kColorOff = kW3bOff + kW3bBytes;
 constexpr size_t kColorBytes = (size_t)kColorChunks * kChunkBytes;
 constexpr size_t kParamOff = kColorOff + kColorBytes;
+// (the slots kPB1 and kPB3 are written and not read: these biases come in through the weight blocks)
 enum : int {
   kPB1 = 0, kPB2 = 256, kPB3 = 512, kPB4 = 768, kPWA = 1024, kPBA = 1280,
   kPCB1 = 1284, kPCB2 = 1412, kPCB3 = 1540, kPWC4 = 1668, kPCB4 = 2052, kParams = 2056
@@ -617,9 +618,9 @@ __global__ void __launch_bounds__(kPairThreads, 1) k_agg_pairs(AggArgs g, long l
         }
       }
       // layer 4: alpha-branch dot product per row, and the weighted sum over each sample's
-      // rows: the warp's 32 rows x 32 columns go through a transpose buffer (in A, whose
-      // last reader, layer 4, has completed), lane l sums column l of each sample in place,
-      // and the sums are written to the colour-input rows 8 columns at a time.
+      // rows: the warp's 32 rows x 64 columns go through a transpose buffer (in A, whose
+      // last reader, layer 4, has completed), and lane l sums columns 2 l and 2 l + 1 of
+      // each sample and writes them to its colour-input row (sample_sums).
       layer();
       {
         const float2 w2 = make_float2(w, w);

@@ -14,7 +14,9 @@
 //                their directions, a tile's rays ordered by count
 //   k_quick_sampling  persistent warps take rays from the list.  A ray with few
 //                candidates is served by 8 lanes (four rays a warp), a heavy
-//                one by the whole warp; lanes stand for candidates:
+//                one by the whole warp; lanes stand for candidates (what the
+//                fast arithmetic cannot decide is done again by serve_exact, a
+//                ray whose list overflows by sample_ray_warp):
 //
 //   pass A  every candidate of the window (rows of cells are runs of the
 //           sorted ids) is tested against the ray once; those within the
@@ -42,10 +44,10 @@
 // first touch.  One thread per ray (tiles staged in shared memory, 32 rays of a
 // window-size class a warp) left half the lanes idle -- every window row and
 // buffer replacement waited for the longest lane -- and its blocks idle at
-// each tile's end; with lanes as candidates 27 of 32 lanes are active and there
-// is no barrier.  1M points, 800 x 800, radius 0.008: 1000 us -> 449 us (446 M
-// -> 336 M warp instructions, 54% -> 72% of the issue slots); 4M points at
-// 512 x 512: 4470 -> 1225 us; 100k points, 3 x 3 window: 193 -> 59 us.  Measured
+// each tile's end; with lanes as candidates 30 of 32 lanes are active and there
+// is no barrier.  1M points, 800 x 800, radius 0.008: 1000 us -> 418 us (446 M
+// -> 337 M warp instructions, 54% -> 73% of the issue slots); 4M points at
+// 512 x 512: 4470 -> 1103 us; 100k points, 3 x 3 window: 193 -> 57 us.  Measured
 // and not kept: the listed candidates themselves in shared memory (20 bytes an
 // entry leave too little L1: 780-1010 us on the first view), re-walking the
 // window in every pass instead of a list (760-850 us), copies of the code per
@@ -166,7 +168,7 @@ __device__ __forceinline__ int2 cell_range(const SampleArgs& a, int vv, int uu) 
 
 // Pack the candidates once per launch: pts[j] = (xyz of sorted_point_idx[j],
 // its id), or id -1 when the id is outside [0, n_points).  Every later fetch
-// of candidate j -- staging or global -- is then one 16-byte load instead of
+// of candidate j is then one 16-byte load instead of
 // an id load and a dependent point gather.
 __device__ __forceinline__ float4 packed_point(const int* __restrict__ sidx, int j, const float* __restrict__ xyz,
                                                int n_points) {
@@ -285,7 +287,7 @@ __device__ __noinline__ void sample_ray_warp(const SampleArgs& a, int v, int u, 
   const bool capped = __any_sync(kAll, ccnt > kKeptPerCell);
 
   // body(j0, valid, idx, cell, pc) per lane and chunk: candidate j0 + lane of
-  // the sequence, its index for src.fetch, its cell and the cell's first j
+  // the sequence, its index in a.pts, its cell and the cell's first j
   auto chunks = [&](auto&& body) {
     for (J j0 = 0; j0 < total; j0 += 32) {
       const J j = j0 + lane;
@@ -1409,8 +1411,8 @@ __global__ void __launch_bounds__(kThreads, 8) k_ray_list(const __grid_constant_
     list_tile<kTileH, kTileW>(a, (t / tiles_x) * kTileH, (t % tiles_x) * kTileW, 0, rl);
 }
 
-// The persistent warps: the units of two first (they run longest), then the
-// units of four.  Each takes its next position before it serves the current one.
+// The persistent warps: the rays of a whole warp first (they run longest), then
+// the units of four.  Each takes its next position before it serves the current one.
 template <class Cfg, bool kBatch>
 __device__ __forceinline__ void serve_list(const SampleArgs& a0, const SampleArgs* __restrict__ args, const RayList& rl,
                                            unsigned char* smem) {

@@ -4,8 +4,8 @@ The reference renders a view at a time: `pts2plane` then `quick_sampling`
 (epcq/epcq.py:279-325), one kernel launch each.  `BatchRenderer` takes many
 views at once -- different clouds, cameras, image sizes -- builds every view's
 hash table (hp_pts2plane, spread over a few streams so small builds overlap)
-and then runs hp_quick_sampling_batch: the tiles of all views in one queue,
-heaviest first, served by one persistent kernel, so the tail of one view
+and then runs hp_quick_sampling_batch: the rays of all views in one list,
+heavy ones first, served by one persistent kernel, so the tail of one view
 overlaps the work of the others.  Each view's outputs are bit-identical to the
 per-view launch.
 
@@ -14,11 +14,10 @@ The whole batch can be captured once as a CUDA graph and replayed (`capture`,
 move, and no call in the batch synchronises with the host.
 
 `Autotuner` picks the launch tuning of hp_quick_sampling_batch -- the stage
-configuration of the sampling pipeline (items in flight per block, staged
-points per item, blocks per SM; which items get split into row bands follows
-from the staged capacity) and which rays a whole warp serves -- by timing the
-candidates on the first batch of a shape class and caching the winner;
-outputs never depend on the choice.
+configuration of the sampling kernel (candidates listed on chip, blocks per
+SM, the tile whose rays are ordered together) and which rays a whole warp
+serves -- by timing the candidates on the first batch of a shape class and
+caching the winner; outputs never depend on the choice.
 """
 import ctypes
 import math

@@ -121,8 +121,8 @@ class ViewRing:
     """Many views of one shape through per-view launches, pipelined over `depth` streams.
 
     View i runs on pipeline i % depth (its own buffers) and that pipeline's stream, so view i+1's
-    hash-table build and tile scheduling run while view i's persistent sampling kernel drains its
-    last work items, and its sampling kernel's blocks start as view i's retire.  Every view is
+    hash-table build and ray list run while view i's persistent sampling kernel drains its
+    last rays, and its sampling kernel's blocks start as view i's retire.  Every view is
     still hp_pts2plane + hp_quick_sampling, each with the outputs the plain launch gives.  A
     view's outputs stay in its pipeline's buffers until view i + depth reuses them on the same
     stream: `on_view(i, pipe, stream)` is called right after view i is enqueued, so work it

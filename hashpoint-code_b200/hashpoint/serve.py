@@ -249,7 +249,7 @@ class Server:
         return output_bytes(req, self.store.options) + self.store.entry_bytes(req)
 
     def _launch(self, reqs, slot, t0_event):
-        # heavy views first: the batch takes its views' tiles in table order
+        # heavy views first: the batch takes its views' rays about in table order
         reqs = sorted(reqs, key=lambda r: -self.store.clouds[r.scene].shape[0])
         s = self.streams[slot]
         hold = []  # cached tables the batch reads

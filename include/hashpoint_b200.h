@@ -302,9 +302,10 @@ typedef struct hp_view {
 } hp_view;
 
 /* hp_quick_sampling for many views -- different clouds, cameras, image sizes
- * and options -- in one persistent launch over the tiles of all views, so one
- * view's tail overlaps the next views' work.  Tiles are taken view by view in
- * table order (heaviest first within a view), so put heavy views first.  Each
+ * and options -- in one persistent launch over the rays of all views, so one
+ * view's tail overlaps the other views' work.  The rays that a whole warp serves
+ * come first, then the others four at a time; either part about in table order,
+ * so put heavy views first.  Each
  * view's outputs are bit-identical to hp_quick_sampling's for that view.  No
  * counterpart call in the reference, which launches quick_sampling once per
  * view (epcq/csrc/epcq_render_topk.cu:341-417).  `views` (host) is checked and
