@@ -19,6 +19,8 @@ def _ptr(t):
 
 def _stream(device):
     """torch's current stream of `device` as an int (without the Stream object current_stream builds)."""
+    if device.type != "cuda":
+        raise ValueError("expected a CUDA device, got %s" % device)
     i = device.index
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if i is None else i)
 
